@@ -78,7 +78,7 @@ __device__ void block_gradient(const Noise &nz, const double *__restrict__ h, in
     for (int i = threadIdx.x; i < n; i += BS) {
         const int ip = (i + 1 == n) ? 0 : i + 1;
         const int im = (i == 0) ? n - 1 : i - 1;
-        g[i] = site_gradient(h[im], h[i], h[ip], ev[im], ev[i], es[im], es[i], dx, lt, f, arc);
+        g[i] = site_gradient<Noise>(h[im], h[i], h[ip], ev[im], ev[i], es[im], es[i], dx, lt, f, arc);
     }
     __syncthreads();
 }

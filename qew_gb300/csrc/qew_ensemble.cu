@@ -26,9 +26,7 @@ namespace {
 constexpr int kEnsBS = 512;
 
 struct EnsJob {
-    const double *coef64;
-    const double *poly64;  // FP64 cell-polynomial store, or null
-    int ky;                // y * 2^ky == y / dy, or kPolyNotPow2
+    NoiseBSpline64 nz64;
 #ifdef QEW_BOUNDS_CHECK
     unsigned long long *oob;
 #endif
@@ -41,30 +39,6 @@ struct EnsJob {
     qew_params p;
     PrecondCoef pc;
 };
-
-__device__ __forceinline__ NoiseBSpline64 job_noise64(const EnsJob &j) {
-    NoiseBSpline64 nz;
-    nz.coef = j.coef64;
-    nz.nx = j.nx;
-    nz.ny = j.ny;
-    nz.dx = j.fdx;
-    nz.dy = j.fdy;
-    nz.inv_dx = 1.0 / j.fdx;
-    nz.inv_dy = 1.0 / j.fdy;
-    nz.dx_pow2 = dbl_is_pow2(j.fdx);
-    nz.dy_pow2 = dbl_is_pow2(j.fdy);
-    nz.xconst = (j.n == j.nx && j.p.physical_size == j.Lx && nz.dx_pow2);
-    nz.wxc[0] = 0.125 * (1.0 / 6.0);  // bsw_value(1/2), as NoiseBSpline64::wxc
-    nz.wxc[1] = 2.875 * (1.0 / 6.0);
-    nz.wxc[2] = 2.875 * (1.0 / 6.0);
-    nz.wxc[3] = 0.125 * (1.0 / 6.0);
-    nz.poly = (j.n == j.nx && j.p.physical_size == j.Lx) ? j.poly64 : nullptr;
-    nz.ky = j.ky;
-#ifdef QEW_BOUNDS_CHECK
-    nz.oob = j.oob;
-#endif
-    return nz;
-}
 
 __device__ __forceinline__ NoiseSplit32 job_noise32(const EnsJob &j) {
     NoiseSplit32 nz;
@@ -104,7 +78,7 @@ k_ensemble(const EnsJob *__restrict__ jobs, const int *__restrict__ order, int c
         (void)npad_max;
         qew_lbfgs_result r32{};
         if (use32) r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(job_noise32(j), j.h, j.n, j.p, cfg32, j.pc, ws, npad);
-        qew_lbfgs_result r = lbfgs_block<NoiseBSpline64, kEnsBS>(job_noise64(j), j.h, j.n, j.p, cfg64, j.pc, ws, npad);
+        qew_lbfgs_result r = lbfgs_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws, npad);
         if (threadIdx.x == 0) {
             r.iterations += r32.iterations;
             r.n_func_evals += r32.n_func_evals;
@@ -140,9 +114,7 @@ extern "C" qew_status qew_ensemble_minimize(qew_ctx *ctx, int count, const qew_e
                             "ensemble_minimize: line %d needs a B-spline field with FP64%s "
                             "coefficients", k, use32 ? " and FP32" : "");
         EnsJob &j = jobs[k];
-        j.coef64 = f->coef64;
-        j.poly64 = f->poly64;
-        j.ky = make_bspline64(f).ky;
+        j.nz64 = make_bspline64(f, L.n, L.p.physical_size);
 #ifdef QEW_BOUNDS_CHECK
         j.oob = qew_bounds_words();
 #endif
@@ -270,7 +242,7 @@ k_serve_static(LaneRing *ring, unsigned int *head, LbfgsCfg cfg32, LbfgsCfg cfg6
             r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(job_noise32(j), j.h, j.n, j.p, cfg32,
                                                            j.pc, ws, npad);
         qew_lbfgs_result r =
-            lbfgs_block<NoiseBSpline64, kEnsBS>(job_noise64(j), j.h, j.n, j.p, cfg64, j.pc, ws, npad);
+            lbfgs_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws, npad);
         if (threadIdx.x == 0) {
             r.iterations += r32.iterations;
             r.n_func_evals += r32.n_func_evals;
@@ -352,9 +324,7 @@ qew_status qew_lane_publish(StaticLane *L, const qew_field *f, double *d_h, int 
         !f->coef64 || (L->use32 && !f->coef32))
         return QEW_ERR_INVALID;
     EnsJob j{};
-    j.coef64 = f->coef64;
-    j.poly64 = f->poly64;
-    j.ky = make_bspline64(f).ky;
+    j.nz64 = make_bspline64(f, n, p->physical_size);
 #ifdef QEW_BOUNDS_CHECK
     j.oob = qew_bounds_words();
 #endif

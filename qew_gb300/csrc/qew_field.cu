@@ -126,6 +126,25 @@ __global__ void k_edge_fp32(const double *__restrict__ c, float *__restrict__ ou
     }
 }
 
+// Largest |c| as its bit pattern (ordered like the number; infinities and NaNs
+// above every finite one) into *out, which the caller clears.
+__global__ void __launch_bounds__(256) k_max_abs_bits(const double *__restrict__ c, size_t n,
+                                                      unsigned long long *out) {
+    unsigned long long m = 0;
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
+         k += (size_t)gridDim.x * blockDim.x) {
+        const unsigned long long b =
+            (unsigned long long)__double_as_longlong(c[k]) & 0x7FFFFFFFFFFFFFFFull;
+        m = b > m ? b : m;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
+        m = q > m ? q : m;
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
 template <class Noise>
 __global__ void k_sample(Noise nz, const double *__restrict__ x, const double *__restrict__ y,
                          int m, double *v, double *dvdx, double *dvdy) {
@@ -304,8 +323,22 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
         st = qew_poly_store_build(ctx, c64, nx, ny, f->dy, f->poly64);
         if (st != QEW_OK) return cleanup(st);
     }
+    // the bound of the fixed-point gather (qew_fix.cuh)
+    unsigned long long max_bits = 0, *d_max = (unsigned long long *)tmp;
+    if (store & QEW_STORE_FP64) {
+        e = cudaMemsetAsync(d_max, 0, sizeof(*d_max), ctx->stream);
+        if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
+        const int blocks = (int)std::min<size_t>((N + 2047) / 2048, (size_t)ctx->num_sms * 8);
+        k_max_abs_bits<<<blocks, 256, 0, ctx->stream>>>(c64, N, d_max);
+        st = qew_launch_check(ctx, "max_abs");
+        if (st != QEW_OK) return cleanup(st);
+        e = cudaMemcpyAsync(&max_bits, d_max, sizeof(max_bits), cudaMemcpyDeviceToHost, ctx->stream);
+        if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
+    }
     e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "field build: %s", cudaGetErrorString(e)));
+    const int max_exp = (int)(max_bits >> 52);
+    f->fixb = max_bits == 0 ? 1023 : (max_exp >= 256 && max_exp <= 1792) ? max_exp : -1;
     qew_free_async(tmp, ctx->stream);
     tmp = nullptr;
     if (store & QEW_STORE_FP64) {

@@ -23,7 +23,7 @@ k_fire(Noise nz, double *__restrict__ h, int n, qew_params P, FireCfg c, double 
        qew_fire_result *out) {
     __shared__ double s_w[96];
     double *g = ws, *v = ws + npad, *ev = ws + 2 * npad, *es = ws + 3 * npad;
-    const LineDx dx = make_line_dx(P.physical_size, n);
+    const LineDx dx = make_line_dx(P.physical_size, n, P.line_tension, P.driving_force);
     const bool arc = (P.model == QEW_MODEL_ARCLENGTH);
     const double lt = P.line_tension, fd = P.driving_force;
     for (int i = threadIdx.x; i < n; i += BS) v[i] = 0.0;

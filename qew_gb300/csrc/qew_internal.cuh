@@ -19,6 +19,7 @@
 #include <string>
 
 #include "../../include/qew_gpu.h"
+#include "qew_fix.cuh"
 #include "qew_nvtx.cuh"
 
 // ---------------------------------------------------------------- handles
@@ -65,6 +66,7 @@ struct qew_field {
     float *coef32 = nullptr;   // [ny][nx], x fastest
     float *edge32 = nullptr;   // [ny][nx]: coefficients filtered along x at e + 1/2
     double *poly64 = nullptr;  // [ny][nx][4]: FP64 cell polynomials of the x-filtered field
+    int fixb = -1;  // biased exponent of the largest |coefficient| (qew_fix.cuh), -1: none usable
     cudaStream_t stream = nullptr;  // stream the coefficients were allocated on
 };
 
@@ -126,12 +128,14 @@ __device__ __forceinline__ T qew_ldg_checked(const T *base, size_t off, size_t s
 #define QEW_LDGP(ptr, base, size, w) \
     qew_ldg_checked((base), (size_t)((ptr) - (base)), (size), (w), __LINE__)
 #define QEW_OOB_PARAMS , size_t oob_n, unsigned long long *oob
+#define QEW_OOB_WORDS , unsigned long long *oob
 #define QEW_OOB_ARGS(n, w) , (n), (w)
 #else
 #define QEW_OOB_MEMBER
 #define QEW_IDX(i, n, w) (i)
 #define QEW_LDGP(ptr, base, size, w) __ldg(ptr)
 #define QEW_OOB_PARAMS
+#define QEW_OOB_WORDS
 #define QEW_OOB_ARGS(n, w)
 #endif
 
@@ -197,9 +201,12 @@ __host__ __device__ __forceinline__ bool dbl_is_pow2(double d) {
 }
 
 // Line spacing dx = physical_size / n with exact shortcuts for its divisions.
+// With the line's tension and force, the folded factors of the per-site
+// combine as well (site_gradient, qew_model_kernels.cuh).
 struct LineDx {
     double dx, inv_dx, inv_dx2;
     bool pow2;
+    double half_dx, c_el, fdx;  // dx / 2, -Gamma / dx, dx f
     __host__ __device__ __forceinline__ double div(double v) const {
         return pow2 ? v * inv_dx : v / dx;
     }
@@ -207,12 +214,16 @@ struct LineDx {
         return pow2 ? v * inv_dx2 : v / (dx * dx);
     }
 };
-__host__ __device__ __forceinline__ LineDx make_line_dx(double physical_size, int n) {
+__host__ __device__ __forceinline__ LineDx make_line_dx(double physical_size, int n,
+                                                        double lt = 0.0, double f = 0.0) {
     LineDx L;
     L.dx = physical_size / (double)n;
     L.inv_dx = 1.0 / L.dx;
     L.inv_dx2 = 1.0 / (L.dx * L.dx);
     L.pow2 = dbl_is_pow2(L.dx);
+    L.half_dx = 0.5 * L.dx;
+    L.c_el = -lt / L.dx;
+    L.fdx = L.dx * f;
     return L;
 }
 
@@ -283,6 +294,15 @@ __device__ __forceinline__ double poly_value(double q0, double q1, double q2, do
     return fma(dy * t, fma(fma(q2 * third, t, 0.5 * q1), t, q0), v0);
 }
 
+struct NoiseBSpline64;
+// NoiseBSpline64::dvdy (deriv) / value out of line: the FP64 16-tap sum, for
+// the few edges that the fixed-point gather declines.
+static __device__ __noinline__ double bspline_slow_call(const double *coef, int nx, int ny, double dx,
+                                                        double dy, double x, double y,
+                                                        bool deriv QEW_OOB_WORDS);
+__device__ __forceinline__ double bspline_slow(const NoiseBSpline64 &nz, bool deriv, double x,
+                                               double y);
+
 // DeviceNoise on x-fastest FP64 coefficients.
 struct NoiseBSpline64 {
     const double *__restrict__ coef;  // [ny][nx]
@@ -294,13 +314,83 @@ struct NoiseBSpline64 {
     // grid x = e + 1/2 exactly, so its cell is e and its x weights are those
     // of t = 1/2 (bit-identical to locating it).
     bool xconst;
-    double wxc[4];
     // The field's FP64 cell-polynomial store when it serves this line (one
     // point per field column), else null; ky: y * 2^ky == y / dy exactly
-    // (kPolyNotPow2 when dy is not a power of two).
+    // (kPolyNotPow2 when dy is not a power of two); kx the same for x.
     const double *__restrict__ poly;
-    int ky;
+    int ky, kx;
+    // The 16-tap sums in 64-bit fixed point (qew_fix.cuh): the field's bound
+    // kb (-1: FP64 sums) and the units of 2 dV/dt / dy and of 6 V, for the
+    // constant x weights (xconst) and for general ones.
+    int kb;
+    double fx_dv_c, fx_v_c, fx_dv_g, fx_v_g;
     QEW_OOB_MEMBER
+
+    // y / dy correctly rounded, from the correctly rounded 1 / dy (P.
+    // Markstein, IBM J. Res. Dev. 34 (1990); C. Brisebarre, J.-M. Muller,
+    // S. Raina, IEEE Trans. Comput. 53 (2004)): three FP64 instructions
+    // where the division takes nine. d's exponent and y's are checked so
+    // that nothing over- or underflows (fixed_div_ok, fx_locate).
+    static __device__ __forceinline__ double div_by(double y, double d, double inv_d) {
+        const double q = y * inv_d;
+        return fma(fma(-q, d, y), inv_d, q);
+    }
+    // Cell and fraction of a physical coordinate, as grid_locate gives them;
+    // false where the reference's fold has to decide (fx_cell).
+    static __device__ __forceinline__ bool fx_locate(double x, double d, double inv_d, int kexp,
+                                                     int n, int &ix, FxFrac &t) {
+        if (kexp != kPolyNotPow2) return fx_cell(x, kexp, n, ix, t);
+        const unsigned ef = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
+        if (ef - 523u > 1000u && x != 0.0) return false;  // |x| outside [2^-500, 2^500]
+        return fx_cell(div_by(x, d, inv_d), 0, n, ix, t);
+    }
+    // The stencil's row sums at cell (ix, iy): x weights w(1/2) times 48 in
+    // exact integers, E in units of 2^(K-52) / 48 ...
+    __device__ __forceinline__ void fx_rows_const(int e, int iy, long long E[4]) const {
+        const bool inner = e >= 1 && e + 2 < nx && iy >= 1 && iy + 2 < ny;
+        const double *p = coef + ((size_t)iy * (size_t)nx + (size_t)e);
+        int xs[4], ys[4];
+        if (!inner) {
+            wrap4(e, nx, xs);
+            wrap4(iy, ny, ys);
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            long long X[4];
+            const double *row = p + (ptrdiff_t)(b - 1) * (ptrdiff_t)nx;
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                X[a] = fx_tap<4>(inner ? QEW_LDGP(row + (a - 1), coef, (size_t)nx * (size_t)ny, oob)
+                                       : c(xs[a], ys[b]),
+                                 kb);
+            E[b] = ((X[0] + X[3]) + 23 * (X[1] + X[2])) >> 5;
+        }
+    }
+    // ... or general x weights, E in units of 2^(K-57).
+    __device__ __forceinline__ void fx_rows(int ix, FxFrac fx, int iy, long long E[4]) const {
+        const bool inner = ix >= 1 && ix + 2 < nx && iy >= 1 && iy + 2 < ny;
+        const double *p = coef + ((size_t)iy * (size_t)nx + (size_t)ix);
+        int xs[4], ys[4];
+        if (!inner) {
+            wrap4(ix, nx, xs);
+            wrap4(iy, ny, ys);
+        }
+        FxFrac wx[4];
+        fx_weights(fx, wx);
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const double *row = p + (ptrdiff_t)(b - 1) * (ptrdiff_t)nx;
+            long long s = 0;
+#pragma unroll
+            for (int a = 0; a < 4; ++a)
+                s += fx_mul(fx_tap<8>(inner ? QEW_LDGP(row + (a - 1), coef,
+                                                       (size_t)nx * (size_t)ny, oob)
+                                            : c(xs[a], ys[b]),
+                                      kb),
+                            wx[a]);
+            E[b] = s >> 4;
+        }
+    }
 
     // Row cell and fraction of height y: from y's bits when dy is a power of
     // two and y / dy lies in [0, ny), else the reference's locate.
@@ -361,6 +451,9 @@ struct NoiseBSpline64 {
     // dV/dy / V at the midpoint of edge e (xc its physical x). With the
     // cell-polynomial store: one 32-byte cell and two FMAs (the wrap edge,
     // e = nx - 1, is not at a half-integer column and keeps the 16 taps).
+    // Without it, the 16 taps in fixed point; what its locate declines
+    // (negative or huge heights, non-finite ones) is summed in FP64. The last
+    // product is never contracted, so every kernel gets the same bits.
     __device__ __forceinline__ double dvdy_edge(int e, double xc, double y) const {
         if (poly && e + 1 < nx) {
             int iy;
@@ -371,22 +464,22 @@ struct NoiseBSpline64 {
             poly_load3(poly + ((size_t)iy * (size_t)nx + (size_t)e) * 4, q0, q1, q2);
             return poly_dvdy(q0, q1, q2, t);
         }
-        if (!xconst || e + 1 >= nx) return dvdy(xc, y);
-        int iy, xs[4], iyn[4];
-        double fy, dwy[4];
-        grid_locate(y, dy, inv_dy, dy_pow2, ny, iy, fy);
-        wrap4(e, nx, xs);
-        wrap4(iy, ny, iyn);
-        bsw_deriv(fy, dwy);
-        double dg = 0;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            double row = 0;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) row += c(xs[a], iyn[b]) * dwy[b];
-            dg += wxc[a] * row;
+        if (kb >= 0) {
+            int ix, iy;
+            FxFrac fx, fy;
+            if (fx_locate(y, dy, inv_dy, ky, ny, iy, fy)) {
+                long long E[4];
+                if (xconst && e + 1 < nx) {
+                    fx_rows_const(e, iy, E);
+                    return __dmul_rn(fx_to_double(fx_cubic_dt2(E, fy)), fx_dv_c);
+                }
+                if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
+                    fx_rows(ix, fx, iy, E);
+                    return __dmul_rn(fx_to_double(fx_cubic_dt2(E, fy)), fx_dv_g);
+                }
+            }
         }
-        return dy_pow2 ? dg * inv_dy : dg / dy;
+        return bspline_slow(*this, true, xc, y);
     }
     __device__ __forceinline__ double value_edge(int e, double xc, double y) const {
         if (poly && e + 1 < nx) {
@@ -398,22 +491,24 @@ struct NoiseBSpline64 {
             poly_load4(poly + ((size_t)iy * (size_t)nx + (size_t)e) * 4, q0, q1, q2, v0);
             return poly_value(q0, q1, q2, v0, t, dy);
         }
-        if (!xconst || e + 1 >= nx) return value(xc, y);
-        int iy, xs[4], iyn[4];
-        double fy, wy[4];
-        grid_locate(y, dy, inv_dy, dy_pow2, ny, iy, fy);
-        wrap4(e, nx, xs);
-        wrap4(iy, ny, iyn);
-        bsw_value(fy, wy);
-        double v = 0;
+        if (kb >= 0) {
+            int ix, iy;
+            FxFrac fx, fy;
+            if (fx_locate(y, dy, inv_dy, ky, ny, iy, fy)) {
+                long long E[4];
+                if (xconst && e + 1 < nx) {
+                    fx_rows_const(e, iy, E);
+                } else if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
+                    fx_rows(ix, fx, iy, E);
+                } else {
+                    return bspline_slow(*this, false, xc, y);
+                }
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            double row = 0;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) row += c(xs[a], iyn[b]) * wy[b];
-            v += wxc[a] * row;
+                for (int b = 0; b < 4; ++b) E[b] >>= 1;
+                return __dmul_rn(fx_to_double(fx_cubic_6v(E, fy)), (xconst && e + 1 < nx) ? fx_v_c : fx_v_g);
+            }
         }
-        return v;
+        return bspline_slow(*this, false, xc, y);
     }
     // sample, filtered_noise.h:103-134
     __device__ __forceinline__ void sample(double x, double y, double &v,
@@ -445,6 +540,33 @@ struct NoiseBSpline64 {
         dvdy_ = dy_pow2 ? gy * inv_dy : gy / dy;
     }
 };
+
+static __device__ __noinline__ double bspline_slow_call(const double *coef, int nx, int ny, double dx,
+                                                        double dy, double x, double y,
+                                                        bool deriv QEW_OOB_WORDS) {
+    NoiseBSpline64 nz;
+    nz.coef = coef;
+    nz.nx = nx;
+    nz.ny = ny;
+    nz.dx = dx;
+    nz.dy = dy;
+    nz.inv_dx = 1.0 / dx;
+    nz.inv_dy = 1.0 / dy;
+    nz.dx_pow2 = dbl_is_pow2(dx);
+    nz.dy_pow2 = dbl_is_pow2(dy);
+#ifdef QEW_BOUNDS_CHECK
+    nz.oob = oob;
+#endif
+    return deriv ? nz.dvdy(x, y) : nz.value(x, y);
+}
+__device__ __forceinline__ double bspline_slow(const NoiseBSpline64 &nz, bool deriv, double x,
+                                               double y) {
+#ifdef QEW_BOUNDS_CHECK
+    return bspline_slow_call(nz.coef, nz.nx, nz.ny, nz.dx, nz.dy, x, y, deriv, nz.oob);
+#else
+    return bspline_slow_call(nz.coef, nz.nx, nz.ny, nz.dx, nz.dy, x, y, deriv);
+#endif
+}
 
 // ------------------------------------------- reference-exact FP64 arithmetic
 // The reference is ISO C++ evaluated expression by expression: every a*b+c is
@@ -648,17 +770,19 @@ static inline bool qew_is_pow2(double d) {
     const double m = frexp(d, &e);
     return d > 0 && m == 0.5;
 }
+// A spacing that the fixed-point locate may divide by (NoiseBSpline64::div_by):
+// in [2^-500, 2^500], not the one mantissa (all ones) Markstein's theorem
+// leaves out.
+static inline bool qew_fixed_div_ok(double d) {
+    uint64_t b;
+    memcpy(&b, &d, sizeof(b));
+    const int ef = (int)(b >> 52);
+    return ef >= 523 && ef <= 1523 && (b & 0x000FFFFFFFFFFFFFull) != 0x000FFFFFFFFFFFFFull;
+}
 static inline NoiseBSpline64 make_bspline64(const qew_field *f, int n = 0,
                                             double physical_size = 0) {
     NoiseBSpline64 nz;
     nz.xconst = (n > 0 && n == f->nx && physical_size == f->Lx && qew_is_pow2(f->dx));
-    {
-        const double t = 0.5, s6 = 1.0 / 6.0, t2 = t * t, t3 = t2 * t, omt = 1.0 - t;
-        nz.wxc[0] = omt * omt * omt * s6;  // the host twin of bsw_value(0.5)
-        nz.wxc[1] = (4.0 - 6.0 * t2 + 3.0 * t3) * s6;
-        nz.wxc[2] = (1.0 + 3.0 * t + 3.0 * t2 - 3.0 * t3) * s6;
-        nz.wxc[3] = t3 * s6;
-    }
     nz.coef = f->coef64;
     nz.nx = f->nx;
     nz.ny = f->ny;
@@ -675,6 +799,18 @@ static inline NoiseBSpline64 make_bspline64(const qew_field *f, int n = 0,
         int e;
         const double m = frexp(f->dy, &e);  // dy = m 2^e
         nz.ky = (f->dy > 0 && m == 0.5) ? 1 - e : kPolyNotPow2;
+        const double mx = frexp(f->dx, &e);
+        nz.kx = (f->dx > 0 && mx == 0.5) ? 1 - e : kPolyNotPow2;
+    }
+    nz.kb = -1;
+    nz.fx_dv_c = nz.fx_v_c = nz.fx_dv_g = nz.fx_v_g = 0.0;
+    if (f->fixb >= 0 && qew_fixed_div_ok(f->dx) && qew_fixed_div_ok(f->dy)) {
+        const int K = f->fixb - 1022;  // |coefficient| < 2^K
+        nz.kb = f->fixb;
+        nz.fx_dv_c = ldexp(1.0, K - 53) / (48.0 * f->dy);
+        nz.fx_v_c = ldexp(1.0, K - 51) / 288.0;
+        nz.fx_dv_g = ldexp(1.0, K - 58) / f->dy;
+        nz.fx_v_g = ldexp(1.0, K - 56) / 6.0;
     }
 #ifdef QEW_BOUNDS_CHECK
     nz.oob = qew_bounds_words();

@@ -132,7 +132,7 @@ k_langevin_run(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, dou
                 for (int q = 0; q < 2; ++q) {
                     const int j = j0 + q;
                     if (j >= cnt) break;
-                    const double g = site_gradient(s_h[j], s_h[j + 1], s_h[j + 2], s_dv[j],
+                    const double g = site_gradient<Noise>(s_h[j], s_h[j + 1], s_h[j + 2], s_dv[j],
                                                    s_dv[j + 1], s_sl[j], s_sl[j + 1], L, lt, f, arc);
                     const double z = q ? z1 : z0;
                     nxt[base + j] = (b > 0) ? s_h[j + 1] + (-a * g + b * z) : s_h[j + 1] + -a * g;
@@ -220,7 +220,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
                 }
                 __syncthreads();
                 for (int r = lo + t; r < hi; r += kRunBS) {
-                    const double gr = site_gradient(hA[r - 1], hA[r], hA[r + 1], dv[r - 1], dv[r],
+                    const double gr = site_gradient<Noise>(hA[r - 1], hA[r], hA[r + 1], dv[r - 1], dv[r],
                                                     sl[r - 1], sl[r], L, lt, f, arc);
                     hB[r] = (b > 0) ? hA[r] + (-a * gr + b * zz[r]) : hA[r] + -a * gr;
                 }
@@ -359,7 +359,7 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
     QEW_CUDA(ctx, cudaMemcpyAsync(d_drift, h_drift, (size_t)steps * 8, cudaMemcpyHostToDevice, ctx->stream));
     QEW_CUDA(ctx, cudaMemcpyAsync(d_diff, h_diff, (size_t)steps * 8, cudaMemcpyHostToDevice, ctx->stream));
     QEW_CUDA(ctx, cudaMemcpyAsync(d_rs, rs.data(), (size_t)steps * 8, cudaMemcpyHostToDevice, ctx->stream));
-    LineDx L = make_line_dx(p->physical_size, n);
+    LineDx L = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     double lt = p->line_tension, fd = p->driving_force;
     int model = p->model;
     uint64_t seed = l->seed;

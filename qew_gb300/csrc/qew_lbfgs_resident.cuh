@@ -71,7 +71,7 @@ __device__ qew_lbfgs_result lbfgs_team(Team &T, const Noise &nz, double *__restr
     __shared__ double s_agg[2 * kTeamMaxCtas];
     __shared__ LbfgsShared sh;
     const int t0 = T.tid(), ts = T.stride();
-    const LineDx dx = make_line_dx(P.physical_size, n);
+    const LineDx dx = make_line_dx(P.physical_size, n, P.line_tension, P.driving_force);
     const double lt = P.line_tension, f = P.driving_force;
     const int model = P.model;
     const bool arc = (model == QEW_MODEL_ARCLENGTH);

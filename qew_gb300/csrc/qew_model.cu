@@ -28,7 +28,7 @@ qew_status objective_impl(qew_ctx *ctx, const qew_field *field, const At &at, in
                           const qew_params *p, double *h_out) {
     if (!ctx || !field || !p || !h_out || n < 1)
         return qew_fail(ctx, QEW_ERR_INVALID, "objective: bad arguments");
-    const LineDx dx = make_line_dx(p->physical_size, n);
+    const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     const int blocks = objective_blocks(n);
     QEW_TRY(qew_dispatch_noise(ctx, field, [&](auto nz) -> qew_status {
         k_objective<decltype(nz), At, kObjBS><<<blocks, kObjBS, 0, ctx->stream>>>(
@@ -80,7 +80,7 @@ qew_status qew_gradient_enqueue(qew_ctx *ctx, const qew_field *field, const doub
                                 const qew_params *p, int precision, double *d_grad) {
     if (!ctx || !field || !p || !d_h || !d_grad || n < 1)
         return qew_fail(ctx, QEW_ERR_INVALID, "gradient: bad arguments");
-    const LineDx dx = make_line_dx(p->physical_size, n);
+    const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     const int blocks = (n + kGradBS - 1) / kGradBS;
     if (precision == QEW_PREC_FP32_SPLIT) {
         if (field->kind != QEW_FIELD_BSPLINE || !field->coef32)

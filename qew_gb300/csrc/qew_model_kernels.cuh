@@ -23,7 +23,7 @@ __device__ __forceinline__ double edge_energy(const Noise &nz, int i, int ip, do
                                               int model) {
     // Unfused where a contraction would change the rounding (1 + s^2, the
     // f*h term), so the reference-exact functor reproduces its operations.
-    const double dh_dx = L.div(hip - hi);
+    const double dh_dx = noise_is_ref<Noise>::value ? L.div(hip - hi) : (hip - hi) * L.inv_dx;
     double line_energy;
     if (model == QEW_MODEL_LINEAR)
         line_energy = lt * dh_dx * dh_dx * 0.5;
@@ -36,7 +36,11 @@ __device__ __forceinline__ double edge_energy(const Noise &nz, int i, int ip, do
 }
 
 // Edge pass of gradient(), qew_model.h:163-175: dV/dy at the midpoint of edge
-// (e, e+1) and, for arclength, the normalised slope dh/sqrt(1+dh^2).
+// (e, e+1) and, for arclength, the normalised slope dh/sqrt(1+dh^2). Except
+// for the reference-exact functor the slope is dh * rsqrt(1 + dh^2) with dh
+// by multiplication: 9 FP64 instructions where the square root and the
+// divisions take 27 or more (an FP64 instruction of a warp occupies its
+// scheduler's FP64 unit for 64 cycles).
 template <class Noise>
 __device__ __forceinline__ void edge_gradient(const Noise &nz, int e, int n, double he,
                                               double hep, const LineDx &L, bool arc, double &dv,
@@ -47,23 +51,38 @@ __device__ __forceinline__ void edge_gradient(const Noise &nz, int e, int n, dou
     dv = noise_dvdy_edge(nz, e, xc, hc);
     sl = 0.0;
     if (arc) {
-        const double dh = L.div(hep - he);
-        sl = dh / sqrt(__dadd_rn(1.0, __dmul_rn(dh, dh)));
+        if constexpr (noise_is_ref<Noise>::value) {
+            const double dh = L.div(hep - he);
+            sl = dh / sqrt(__dadd_rn(1.0, __dmul_rn(dh, dh)));
+        } else {
+            const double dh = (hep - he) * L.inv_dx;
+            sl = dh * rsqrt(fma(dh, dh, 1.0));
+        }
     }
 }
 
-// Per-site combine, qew_model.h:177-193.
+// Per-site combine, qew_model.h:177-193. Except for the reference-exact
+// functor with the factors folded, as the cell-polynomial gradient does:
+//   grad = c_el d2h + (dx/2)(dvl + dvr) - dx f    (linear, c_el = -Gamma/dx)
+//        = Gamma (sll - slr) + (dx/2)(dvl + dvr) - dx f    (arclength),
+// 5 and 4 FP64 instructions for 9 and 8.
+template <class Noise>
 __device__ __forceinline__ double site_gradient(double hm, double h0, double hp, double dvl,
                                                 double dvr, double sll, double slr,
                                                 const LineDx &L, double lt, double f, bool arc) {
-    double line_force;
-    if (!arc) {
-        const double d2h = hm + hp - 2.0 * h0;
-        line_force = L.div2(-lt * d2h);
+    if constexpr (noise_is_ref<Noise>::value) {
+        double line_force;
+        if (!arc) {
+            const double d2h = hm + hp - 2.0 * h0;
+            line_force = L.div2(-lt * d2h);
+        } else {
+            line_force = L.div(lt * (sll - slr));
+        }
+        return L.dx * (line_force + 0.5 * (dvl + dvr) - f);
     } else {
-        line_force = L.div(lt * (sll - slr));
+        const double rest = fma(L.half_dx, dvl + dvr, -L.fdx);
+        return arc ? fma(lt, sll - slr, rest) : fma(L.c_el, fma(-2.0, h0, hm + hp), rest);
     }
-    return L.dx * (line_force + 0.5 * (dvl + dvr) - f);
 }
 
 // Fused gradient: CTA of BS sites stages h[base-1 .. base+BS] and the BS+1
@@ -93,7 +112,7 @@ k_gradient(const double *__restrict__ h, int n, LineDx dx, double lt, double f, 
     if (t == 0) edge_gradient(nz, base == 0 ? n - 1 : base - 1, n, s_h[0], s_h[1], dx, arc, s_dv[0], s_sl[0]);
     __syncthreads();
     if (t < cnt)
-        grad[i] = site_gradient(s_h[t], s_h[t + 1], s_h[QEW_IDX(t + 2, BS + 2, oob)], s_dv[t],
+        grad[i] = site_gradient<Noise>(s_h[t], s_h[t + 1], s_h[QEW_IDX(t + 2, BS + 2, oob)], s_dv[t],
                                 s_dv[QEW_IDX(t + 1, BS + 1, oob)], s_sl[t], s_sl[t + 1], dx, lt,
                                 f, arc);
 }

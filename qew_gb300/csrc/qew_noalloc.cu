@@ -117,7 +117,7 @@ extern "C" qew_status qew_objective_noalloc(const qew_field *field, const double
         cudaGetLastError();
         return QEW_ERR_CUDA;
     }
-    const LineDx dx = make_line_dx(p->physical_size, n);
+    const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     const int blocks = (n + kNoAllocBS - 1) / kNoAllocBS;  // <= kNoAllocMaxBlocks
     return qew_dispatch_noise(nullptr, field, [&](auto nz) -> qew_status {
         k_objective<decltype(nz), LineAt, kNoAllocBS><<<blocks, kNoAllocBS, 0, stream>>>(

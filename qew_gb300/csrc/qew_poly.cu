@@ -255,11 +255,11 @@ qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count
     g.n = n;
     g.ky = poly_scale_exponent(f->dy);
     g.half_inv_dy = 0.5 / f->dy;
-    g.L = make_line_dx(p->physical_size, n);
-    g.c_el = -p->line_tension / g.L.dx;
+    g.L = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
+    g.c_el = g.L.c_el;
     g.lt = p->line_tension;
-    g.half_dx = 0.5 * g.L.dx;
-    g.fdx = g.L.dx * p->driving_force;
+    g.half_dx = g.L.half_dx;
+    g.fdx = g.L.fdx;
     int hx;
     const bool f0 = p->driving_force == 0.0 && frexp(g.half_dx, &hx) == 0.5;
     g.half_dx_exp = hx - 1;  // half_dx == 2^(hx-1) when f0

@@ -17,6 +17,12 @@ namespace {
 
 constexpr int kBS = 256;
 
+// The plain form and the site velocities keep the 16-tap sum on a field that
+// holds the cell-polynomial store.
+template <class Noise>
+void drop_poly(Noise &) {}
+void drop_poly(NoiseBSpline64 &nz) { nz.poly = nullptr; }
+
 // One colour of one sweep (rosso_krauth.h:154-165): thread k owns site 2k+color.
 template <class Noise>
 __global__ void k_rk_colour(Noise nz, double *__restrict__ h, double *__restrict__ adv, int n,
@@ -76,12 +82,13 @@ qew_status qew_rk_block_plain(qew_ctx *ctx, const qew_field *field, double *d_h,
     for (int sweep = 0; sweep < rp->max_sweeps; ++sweep) {
         for (int color = 0; color < 2; ++color) {
             auto colour = [&](auto nz) -> qew_status {
+                drop_poly(nz);
                 k_rk_colour<<<(half + kBS - 1) / kBS, kBS, 0, ctx->stream>>>(
                     nz, d_h, adv, n, dx, p->line_tension, p->driving_force, p->model, color, rk);
                 return qew_launch_check(ctx, "rk_colour");
             };
             QEW_TRY(precision == QEW_PREC_FP64_REFERENCE ? qew_dispatch_noise_ref(ctx, field, colour)
-                                                          : qew_dispatch_noise(ctx, field, colour));
+                                                          : qew_dispatch_noise(ctx, field, colour, n, p->physical_size));
         }
         double total_adv;
         QEW_TRY((vec_reduce<SumF, 1, false>(ctx, n, SumF{adv}, &total_adv)));
@@ -115,10 +122,11 @@ qew_status qew_rk_site_velocity(qew_ctx *ctx, const qew_field *field, const doub
         return qew_fail(ctx, QEW_ERR_INVALID, "rk_site_velocity: bad arguments");
     const double dx = p->physical_size / (double)n;
     return qew_dispatch_noise(ctx, field, [&](auto nz) -> qew_status {
+        drop_poly(nz);
         k_rk_velocity<<<(n + kBS - 1) / kBS, kBS, 0, ctx->stream>>>(
             nz, d_h, n, dx, p->line_tension, p->driving_force, p->model, d_vel);
         return qew_launch_check(ctx, "rk_velocity");
-    });
+    }, n, p->physical_size);
 }
 
 qew_status qew_rk_block(qew_ctx *ctx, const qew_field *field, double *d_h, int n,

@@ -112,7 +112,7 @@ __device__ void team_gradient(Team &T, const Noise &nz, const double *__restrict
     for (int i = T.tid(); i < n; i += T.stride()) {
         const int ip = (i + 1 == n) ? 0 : i + 1;
         const int im = (i == 0) ? n - 1 : i - 1;
-        g[i] = (R)site_gradient(T.ld(h + im), T.ld(h + i), T.ld(h + ip), (double)T.ld(ev + im),
+        g[i] = (R)site_gradient<Noise>(T.ld(h + im), T.ld(h + i), T.ld(h + ip), (double)T.ld(ev + im),
                                 (double)T.ld(ev + i), (double)T.ld(es + im), (double)T.ld(es + i),
                                 dx, lt, f, arc);
     }
