@@ -23,67 +23,108 @@
 
 namespace {
 
-// Periodic cubic B-spline prefilter along one axis, in two out-of-place
-// passes over chunks of kChunk samples so that every line is split over many
-// threads: causal y[k] = s[k] + z y[k-1], anticausal w[k] = y[k] + z w[k+1],
-// c = -6 z w. A chunk starts its recursion kWarm samples early (late, for the
-// anticausal pass) from zero, reading the periodic neighbours: the neglected
-// tail is z^kWarm ~ 5e-37 of the signal, so every output equals the exact
-// periodic solve up to rounding, for any N (the warm-up wraps for short N).
-// Lines are m = 0..M-1 at stride `lst`; samples at stride `st`; consecutive
-// threads take consecutive lines so each step's accesses coalesce when
-// lst == 1.
+// Periodic cubic B-spline prefilter along one axis, in one out-of-place pass
+// over chunks of kChunk samples so that every line is split over many
+// threads. The filter's causal and anticausal recursions run side by side on
+// the samples (its partial-fraction form): with y[k] = s[k] + z y[k-1] and
+// w[k] = s[k] + z w[k+1],
+//   c[k] = g (y[k] + z w[k+1]),  g = -6 z / (1 - z^2) = sqrt(3),
+// which equals the cascade c = -6 z anticausal(causal(s)). A chunk starts
+// each recursion kWarm samples away from zero, reading the periodic
+// neighbours: the neglected tail is z^kWarm = 5e-19 of the signal, so every
+// output equals the exact periodic solve up to rounding, for any N (the
+// warm-up wraps for short N). Lines are m = 0..M-1 at stride `lst`; samples
+// at stride `st`; consecutive threads take consecutive lines so each step's
+// accesses coalesce when lst == 1. FP64-bound: 4 instructions a sample (5
+// with the gain, which the last axis applies for both, times the field's
+// scale where one is given) and a half for the warm-ups. 4096 x 1024, both
+// axes: 284 -> 109 us (the cascade's four passes before).
 constexpr double kPole = -0.26794919243112270;  // sqrt(3) - 2
-constexpr int kChunk = 256;
-constexpr int kWarm = 64;
+constexpr int kChunk = 64;
+constexpr int kWarm = 32;
+constexpr int kPreBS = 128;
 
 __device__ __forceinline__ int pmod(long k, int N) {
     long r = k % N;
     return (int)(r < 0 ? r + N : r);
 }
 
-__global__ void k_prefilter_causal(const double *__restrict__ in, double *__restrict__ out,
-                                   int N, long st, int M, long lst) {
-    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
+// What the last axis's pass does besides: the gain of both axes (times
+// *scale), the FP32 copy (out32, or null) and the largest |c|'s bits
+// (max_bits, or null).
+struct PrefilterEnd {
+    double gain;
+    const double *scale;
+    float *out32;
+    unsigned long long *max_bits;
+};
+
+template <bool kEnd>
+__global__ void __launch_bounds__(kPreBS)
+k_prefilter(const double *__restrict__ in, double *out, int N, long st, int M, long lst,
+            PrefilterEnd end) {
+    const long tid = blockIdx.x * (long)kPreBS + threadIdx.x;
     const int nchunks = (N + kChunk - 1) / kChunk;
-    if (tid >= (long)M * nchunks) return;
-    const int m = (int)(tid % M), c = (int)(tid / M);
-    const double *a = in + (long)m * lst;
-    double *b = out + (long)m * lst;
-    const int k0 = c * kChunk, k1 = min(k0 + kChunk, N);
-    double y = 0.0;
-    for (int k = k0 - kWarm; k < k0; ++k) y = a[(long)pmod(k, N) * st] + kPole * y;
-    for (int k = k0; k < k1; ++k) {
-        y = a[(long)k * st] + kPole * y;
-        b[(long)k * st] = y;
+    unsigned long long mx = 0;
+    if (tid < (long)M * nchunks) {
+        const int m = (int)(tid % M), c = (int)(tid / M);
+        const double *a = in + (long)m * lst;
+        double *b = out + (long)m * lst;
+        const int k0 = c * kChunk, k1 = min(k0 + kChunk, N);
+        double y = 0.0;
+        int k = pmod((long)k0 - kWarm, N);
+#pragma unroll 8
+        for (int q = 0; q < kWarm; ++q) {
+            y = fma(kPole, y, a[(long)k * st]);
+            k = (k + 1 == N) ? 0 : k + 1;
+        }
+#pragma unroll 8
+        for (k = k0; k < k1; ++k) {
+            y = fma(kPole, y, a[(long)k * st]);
+            b[(long)k * st] = y;
+        }
+        const double gain = kEnd ? (end.scale ? end.gain * *end.scale : end.gain) : 1.0;
+        double w = 0.0;
+        k = pmod((long)k1 - 1 + kWarm, N);
+#pragma unroll 8
+        for (int q = 0; q < kWarm; ++q) {
+            w = fma(kPole, w, a[(long)k * st]);
+            k = (k == 0) ? N - 1 : k - 1;
+        }
+#pragma unroll 8
+        for (k = k1 - 1; k >= k0; --k) {
+            double v = fma(kPole, w, b[(long)k * st]);
+            w = fma(kPole, w, a[(long)k * st]);
+            if (kEnd) {
+                v *= gain;
+                const unsigned long long vb =
+                    (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+                mx = vb > mx ? vb : mx;
+                if (end.out32) end.out32[(long)m * lst + (long)k * st] = (float)v;
+            }
+            b[(long)k * st] = v;
+        }
+    }
+    if (kEnd && end.max_bits) {  // bit patterns of |c| are ordered like the numbers
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long q = __shfl_xor_sync(0xffffffffu, mx, o);
+            mx = q > mx ? q : mx;
+        }
+        if ((threadIdx.x & 31) == 0) atomicMax(end.max_bits, mx);
     }
 }
 
-__global__ void k_prefilter_anticausal(const double *__restrict__ in, double *__restrict__ out,
-                                       int N, long st, int M, long lst) {
-    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    const int nchunks = (N + kChunk - 1) / kChunk;
-    if (tid >= (long)M * nchunks) return;
-    const int m = (int)(tid % M), c = (int)(tid / M);
-    const double *a = in + (long)m * lst;
-    double *b = out + (long)m * lst;
-    const int k0 = c * kChunk, k1 = min(k0 + kChunk, N);
-    const double gain = -6.0 * kPole;
-    double w = 0.0;
-    for (int k = k1 - 1 + kWarm; k >= k1; --k) w = a[(long)pmod(k, N) * st] + kPole * w;
-    for (int k = k1 - 1; k >= k0; --k) {
-        w = a[(long)k * st] + kPole * w;
-        b[(long)k * st] = gain * w;
-    }
-}
-
-qew_status prefilter_axis(qew_ctx *ctx, double *a, double *work, int N, long st, int M,
-                          long lst) {
+qew_status prefilter_axis(qew_ctx *ctx, const double *in, double *out, int N, long st, int M,
+                          long lst, const PrefilterEnd *end) {
     const long threads = (long)M * ((N + kChunk - 1) / kChunk);
-    const unsigned blocks = (unsigned)((threads + 255) / 256);
-    k_prefilter_causal<<<blocks, 256, 0, ctx->stream>>>(a, work, N, st, M, lst);
-    k_prefilter_anticausal<<<blocks, 256, 0, ctx->stream>>>(work, a, N, st, M, lst);
-    return qew_launch_check(ctx, "prefilter", 2);
+    const unsigned blocks = (unsigned)((threads + kPreBS - 1) / kPreBS);
+    if (end)
+        k_prefilter<true><<<blocks, kPreBS, 0, ctx->stream>>>(in, out, N, st, M, lst, *end);
+    else
+        k_prefilter<false><<<blocks, kPreBS, 0, ctx->stream>>>(in, out, N, st, M, lst,
+                                                               PrefilterEnd{});
+    return qew_launch_check(ctx, "prefilter");
 }
 
 // [nx][ny] -> [ny][nx] through a 32x33 shared tile.
@@ -100,12 +141,6 @@ __global__ void k_transpose(const double *__restrict__ in, double *__restrict__ 
         const int j = j0 + r, i = i0 + threadIdx.x;
         if (i < nx && j < ny) out[(size_t)j * nx + i] = tile[threadIdx.x][r];
     }
-}
-
-__global__ void k_to_fp32(const double *__restrict__ in, float *__restrict__ out, size_t n) {
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
-         k += (size_t)gridDim.x * blockDim.x)
-        out[k] = (float)in[k];
 }
 
 // E[j][e] = sum_a w_a(1/2) c[j][(e - 1 + a) mod nx], FP64 sum rounded once to
@@ -126,25 +161,6 @@ __global__ void k_edge_fp32(const double *__restrict__ c, float *__restrict__ ou
     }
 }
 
-// Largest |c| as its bit pattern (ordered like the number; infinities and NaNs
-// above every finite one) into *out, which the caller clears.
-__global__ void __launch_bounds__(256) k_max_abs_bits(const double *__restrict__ c, size_t n,
-                                                      unsigned long long *out) {
-    unsigned long long m = 0;
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
-         k += (size_t)gridDim.x * blockDim.x) {
-        const unsigned long long b =
-            (unsigned long long)__double_as_longlong(c[k]) & 0x7FFFFFFFFFFFFFFFull;
-        m = b > m ? b : m;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long q = __shfl_xor_sync(0xffffffffu, m, o);
-        m = q > m ? q : m;
-    }
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
-
 template <class Noise>
 __global__ void k_sample(Noise nz, const double *__restrict__ x, const double *__restrict__ y,
                          int m, double *v, double *dvdx, double *dvdy) {
@@ -163,59 +179,154 @@ __global__ void k_sample(Noise nz, const double *__restrict__ x, const double *_
 // (the real-space form of exp(-(2 pi xi f)^2 / 2) in Fourier space; taps to
 // |k| <= ceil(5 xi), normalised so the sum of squared taps is 1), in the
 // reference's host layout [nx][ny].
-__global__ void k_white_noise(double *w, int nx, int ny, uint64_t seed) {
+// The filter runs in 64-bit fixed point (qew_fix.cuh): the noise is bounded
+// (|z| < 8.58 from 53-bit uniforms), so it and the taps lose nothing, and a
+// tap pair costs four 32 x 32 + 64-bit multiply-adds (about 5 cycles each) where
+// FP64 takes two 64-cycle instructions: 306 -> 150 us an axis of a 4096 x 1024
+// field at xi = 4 (41 taps). A sample is X = X1 2^30 + X0 in units 2^-F,
+// |X| < 2^59; a tap T = T1 2^30 + T0 in units 2^-q, q such that the taps'
+// sum is at most 2^58.
+constexpr double kNoiseMax = 8.58;  // sqrt(2 ln 2^53) = 8.572
+
+__global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_t seed, int F) {
     const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
     const int pairs = (ny + 1) / 2;
     if (tid >= (long)nx * pairs) return;
     const int i = (int)(tid / pairs), jp = (int)(tid % pairs);
-    double z0, z1;
-    philox_normal_pair(seed, (uint64_t)i, (uint32_t)jp, z0, z1);
-    w[(size_t)i * ny + 2 * jp] = z0;
-    if (2 * jp + 1 < ny) w[(size_t)i * ny + 2 * jp + 1] = z1;
+    uint32_t c[4] = {(uint32_t)jp, 0u, (uint32_t)i, 0u};
+    philox4x32_10(c, seed);
+    const uint64_t a = ((((uint64_t)c[0]) << 32) | c[1]) >> 11;
+    const uint64_t b = ((((uint64_t)c[2]) << 32) | c[3]) >> 11;
+    long long z0, z1;
+    int k;
+    fx_normal_pair(a + 1, b, g_fx_logs, g_fx_turns, z0, z1, k);  // z 2^k, k <= -F
+    const int sh = min(-k - F, 63);
+    w[(size_t)i * ny + 2 * jp] = z0 >> sh;
+    if (2 * jp + 1 < ny) w[(size_t)i * ny + 2 * jp + 1] = z1 >> sh;
 }
 
-// out[i][j] = sum_k taps[k] * in[(i + k - R) mod nx][j]   (axis 0), or along j (axis 1).
-__global__ void k_gauss_conv(const double *__restrict__ in, double *__restrict__ out, int nx,
-                             int ny, const double *__restrict__ taps, int R, int axis) {
-    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
+// out[i][j] = sum_k taps[k] * in[(i + k - R) mod nx][j]   (axis 0), or along j
+// (axis 1); symmetric taps, tap[k] for distance k. The partial products of
+// weight 2^60, 2^30 and 1 have sums of their own, the lower two folded every
+// four pairs before they can overflow (2^61 a pair). kLast: FP64 out, times
+// 2^exp; else fixed point again, shifted right by exp.
+template <bool kLast>
+__global__ void __launch_bounds__(256)
+k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int nx, int ny,
+             const int2 *__restrict__ tap, int R, int axis, int exp) {
+    const long tid = blockIdx.x * 256l + threadIdx.x;
     if (tid >= (long)nx * ny) return;
-    const int i = (int)(tid / ny), j = (int)(tid % ny);
-    double acc = 0.0;
-    for (int k = -R; k <= R; ++k) {
-        const double t = taps[k + R];
-        if (axis == 0)
-            acc += t * in[(size_t)pmod((long)i + k, nx) * ny + j];
-        else
-            acc += t * in[(size_t)i * ny + pmod((long)j + k, ny)];
+    const int i = (int)(tid / ny), j = (int)(tid - (long)i * ny);
+    const int n = axis ? ny : nx, at = axis ? j : i;
+    const long st = axis ? 1 : ny;
+    const long long *line = in + (axis ? (size_t)i * ny : (size_t)j);
+    long long P = 0, M = 0, A = 0;
+    unsigned long long L = 0;
+    auto add = [&](int x1, int x0, int2 t) {
+        P += (long long)x1 * t.x;
+        M += (long long)x1 * t.y;
+        M += (long long)x0 * t.x;  // x0 < 2^31
+        L += (unsigned long long)(unsigned)x0 * (unsigned)t.y;
+    };
+    auto fold = [&]() {
+        A += (M >> 14) + (long long)(L >> 44);
+        M = 0;
+        L = 0;
+    };
+    constexpr int kLow = (1 << 30) - 1;
+    {
+        const long long x = line[(long)at * st];
+        add((int)(x >> 30), (int)x & kLow, __ldg(tap));
     }
-    out[tid] = acc;
+    if (at >= R && at + R < n) {
+        const long long *lo = line + (long)at * st, *hi = lo;
+        for (int k0 = 1; k0 <= R; k0 += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int k = k0 + u;
+                if (k > R) break;
+                lo -= st;
+                hi += st;
+                const long long a = *lo, b = *hi;
+                add((int)(a >> 30) + (int)(b >> 30), ((int)a & kLow) + ((int)b & kLow),
+                    __ldg(tap + k));
+            }
+            fold();
+        }
+    } else {
+        int kl = at, kh = at;
+        for (int k = 1; k <= R; ++k) {
+            kl = (kl == 0) ? n - 1 : kl - 1;
+            kh = (kh + 1 == n) ? 0 : kh + 1;
+            const long long a = line[(long)kl * st], b = line[(long)kh * st];
+            add((int)(a >> 30) + (int)(b >> 30), ((int)a & kLow) + ((int)b & kLow),
+                __ldg(tap + k));
+            if ((k & 3) == 0) fold();
+        }
+    }
+    fold();
+    const long long v = (P << 5) + (A >> 11);  // units of 2^55
+    if (kLast)
+        ((double *)out)[tid] = fx_to_double(v, exp);
+    else
+        ((long long *)out)[tid] = v >> exp;
 }
 
-__global__ void k_scale_inplace(double *a, size_t n, const double *scale) {
-    const double s = *scale;
-    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
-         k += (size_t)gridDim.x * blockDim.x)
-        a[k] *= s;
-}
-
-// Population mean and std of n values -> scale = amplitude / std (one CTA).
-__global__ void k_std_scale(const double *__restrict__ a, size_t n, double amplitude,
-                            double *scale) {
-    __shared__ double s_w[32];
-    double s1 = 0.0;
-    for (size_t k = threadIdx.x; k < n; k += blockDim.x) s1 += a[k];
-    s1 = block_sum<1024>(s1, s_w);
-    __shared__ double s_mean;
-    if (threadIdx.x == 0) s_mean = s1 / (double)n;
+// Population mean and std of n values in two passes (the second about the
+// mean): per-block partial sums, the last block to arrive adds them in block
+// order. stat[0] = mean after the first pass; stat[1] = amplitude / std after
+// the second. One CTA read the field twice at one SM's bandwidth: 3.45 ms of
+// a 4096 x 1024 field's 4.8 ms, these passes take 17 and 24 us.
+constexpr int kMomBS = 256;
+template <bool kCentred>
+__global__ void __launch_bounds__(kMomBS)
+k_moment(const double *__restrict__ a, size_t n, double amplitude, double *partials,
+         unsigned int *counter, double *stat) {
+    __shared__ double s_w[kMomBS / 32];
+    __shared__ bool s_last;
+    const double mean = kCentred ? stat[0] : 0.0;
+    const size_t step = (size_t)gridDim.x * kMomBS;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+    size_t k = blockIdx.x * (size_t)kMomBS + threadIdx.x;
+    auto term = [&](double v, double s) { return kCentred ? fma(v - mean, v - mean, s) : s + v; };
+    for (; k + 3 * step < n; k += 4 * step) {
+        const double v0 = a[k], v1 = a[k + step], v2 = a[k + 2 * step], v3 = a[k + 3 * step];
+        s0 = term(v0, s0);
+        s1 = term(v1, s1);
+        s2 = term(v2, s2);
+        s3 = term(v3, s3);
+    }
+    for (; k < n; k += step) s0 = term(a[k], s0);
+    const double bs = block_sum<kMomBS>((s0 + s1) + (s2 + s3), s_w);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = bs;
+        __threadfence();
+        s_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
     __syncthreads();
-    const double mean = s_mean;
-    double s2 = 0.0;
-    for (size_t k = threadIdx.x; k < n; k += blockDim.x) {
-        const double d = a[k] - mean;
-        s2 += d * d;
+    if (!s_last) return;
+    double v = 0.0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kMomBS) v += __ldcg(partials + b);
+    const double tot = block_sum<kMomBS>(v, s_w);
+    if (threadIdx.x == 0) {
+        if (kCentred)
+            stat[1] = amplitude / sqrt(tot / (double)n);
+        else
+            stat[0] = tot / (double)n;
+        *counter = 0u;
     }
-    s2 = block_sum<1024>(s2, s_w);
-    if (threadIdx.x == 0) *scale = amplitude / sqrt(s2 / (double)n);
+}
+
+// stat (2 doubles on the device) of n values; scratch: the context's reduction arena.
+qew_status field_moments(qew_ctx *ctx, const double *a, size_t n, double amplitude, double *stat) {
+    const int blocks = (int)std::min<size_t>(
+        std::min<size_t>((n + 4 * kMomBS - 1) / (4 * kMomBS), (size_t)ctx->num_sms * 6),
+        QEW_RED_MAX_BLOCKS);
+    k_moment<false><<<blocks, kMomBS, 0, ctx->stream>>>(a, n, amplitude, ctx->red_partials,
+                                                        ctx->red_counter, stat);
+    k_moment<true><<<blocks, kMomBS, 0, ctx->stream>>>(a, n, amplitude, ctx->red_partials,
+                                                       ctx->red_counter, stat);
+    return qew_launch_check(ctx, "field_moments", 2);
 }
 
 // Real part of the inverse transform times 1/(nx ny) (the backward
@@ -233,21 +344,35 @@ double fft_freq(int k, int n) {
     return (double)ks / (double)n;
 }
 
-std::vector<double> gauss_taps(double xi, int &R) {
+// Taps 0..R of the normalised symmetric filter in fixed point (units 2^-q),
+// and the bound on the filter's gain (the taps' sum).
+std::vector<int2> gauss_taps(double xi, int &R, int &q, double &gain) {
     R = (xi > 0) ? (int)ceil(5.0 * xi) : 0;
-    std::vector<double> t(2 * R + 1);
+    std::vector<double> t(R + 1);
     double s2 = 0.0;
     for (int k = -R; k <= R; ++k) {
         const double v = (xi > 0) ? exp(-0.5 * (double)k * k / (xi * xi)) : 1.0;
-        t[k + R] = v;
+        if (k >= 0) t[k] = v;
         s2 += v * v;
     }
-    for (double &v : t) v /= sqrt(s2);
-    return t;
+    gain = 0.0;
+    for (int k = 0; k <= R; ++k) {
+        t[k] /= sqrt(s2);
+        gain += (k ? 2.0 : 1.0) * t[k];
+    }
+    q = 58 - std::max(0, (int)ceil(log2(gain)));
+    std::vector<int2> T(R + 1);
+    for (int k = 0; k <= R; ++k) {
+        const long long v = llrint(ldexp(t[k], q));
+        T[k] = make_int2((int)(v >> 30), (int)(v & ((1 << 30) - 1)));
+    }
+    return T;
 }
 
+// scale (a device number, or null) multiplies the field.
 qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int nx,
-                       int ny, double Lx, double Ly, int store, qew_field **out) {
+                       int ny, double Lx, double Ly, int store, qew_field **out,
+                       const double *scale = nullptr) {
     if (!ctx || !out || !src || nx <= 0 || ny <= 0 || !(Lx > 0) || !(Ly > 0) ||
         (store & (QEW_STORE_FP64 | QEW_STORE_FP32)) == 0)
         return qew_fail(ctx, QEW_ERR_INVALID, "field_create: bad arguments");
@@ -272,10 +397,12 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
     f->dx = Lx / nx;  // filtered_noise.cpp:87
     f->dy = Ly / ny;
     double *tmp = nullptr, *c64 = nullptr;
+    unsigned long long *d_max = nullptr;
     f->stream = ctx->stream;
     auto cleanup = [&](qew_status s) {
         qew_free_async(tmp, ctx->stream);
         qew_free_async(c64, ctx->stream);
+        qew_free_async(d_max, ctx->stream);
         qew_free_async(f->coef32, ctx->stream);
         qew_free_async(f->edge32, ctx->stream);
         qew_free_async(f->poly64, ctx->stream);
@@ -286,29 +413,33 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
     if (qew_alloc_async(ctx, (void **)&tmp, N * sizeof(double)) != QEW_OK ||
         qew_alloc_async(ctx, (void **)&c64, N * sizeof(double)) != QEW_OK)
         return cleanup(QEW_ERR_NOMEM);
-    cudaError_t e = cudaMemcpyAsync(tmp, src, N * sizeof(double),
-                                    src_on_device ? cudaMemcpyDeviceToDevice
-                                                  : cudaMemcpyHostToDevice,
-                                    ctx->stream);
-    if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "field upload: %s", cudaGetErrorString(e)));
+    cudaError_t e = cudaSuccess;
+    if (!src_on_device) {
+        e = cudaMemcpyAsync(c64, src, N * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
+        if (e != cudaSuccess)
+            return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "field upload: %s", cudaGetErrorString(e)));
+        src = c64;
+    }
+    if (qew_alloc_async(ctx, (void **)&d_max, sizeof(*d_max)) != QEW_OK)
+        return cleanup(QEW_ERR_NOMEM);
+    e = cudaMemsetAsync(d_max, 0, sizeof(*d_max), ctx->stream);
+    if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
+    if (store & QEW_STORE_FP32)
+        if (qew_alloc_async(ctx, (void **)&f->coef32, N * sizeof(float)) != QEW_OK)
+            return cleanup(QEW_ERR_NOMEM);
     // x pass in the host layout (lines j, stride ny), transpose, y pass in
-    // the x-fastest layout (lines i, stride nx); c64 doubles as the work
-    // buffer of the first pass.
-    qew_status st = prefilter_axis(ctx, tmp, c64, nx, ny, ny, 1);
+    // the x-fastest layout (lines i, stride nx), each out of place; the y pass
+    // applies the gain, writes the FP32 copy and takes the largest coefficient
+    qew_status st = prefilter_axis(ctx, src, tmp, nx, ny, ny, 1, nullptr);
     if (st != QEW_OK) return cleanup(st);
     k_transpose<<<dim3((ny + 31) / 32, (nx + 31) / 32), dim3(32, 8), 0, ctx->stream>>>(tmp, c64, nx, ny);
     st = qew_launch_check(ctx, "transpose");
     if (st != QEW_OK) return cleanup(st);
-    st = prefilter_axis(ctx, c64, tmp, ny, nx, nx, 1);
+    const PrefilterEnd end{36.0 * kPole * kPole / ((1.0 - kPole * kPole) * (1.0 - kPole * kPole)),
+                           scale, f->coef32, d_max};
+    st = prefilter_axis(ctx, c64, tmp, ny, nx, nx, 1, &end);
     if (st != QEW_OK) return cleanup(st);
-    if (store & QEW_STORE_FP32) {
-        if (qew_alloc_async(ctx, (void **)&f->coef32, N * sizeof(float)) != QEW_OK)
-            return cleanup(QEW_ERR_NOMEM);
-        const int blocks = ctx->num_sms * 8;
-        k_to_fp32<<<blocks, 256, 0, ctx->stream>>>(c64, f->coef32, N);
-        st = qew_launch_check(ctx, "to_fp32");
-        if (st != QEW_OK) return cleanup(st);
-    }
+    std::swap(tmp, c64);
     if (store & QEW_STORE_FP32_EDGE) {
         if (qew_alloc_async(ctx, (void **)&f->edge32, N * sizeof(float)) != QEW_OK)
             return cleanup(QEW_ERR_NOMEM);
@@ -324,19 +455,12 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
         if (st != QEW_OK) return cleanup(st);
     }
     // the bound of the fixed-point gather (qew_fix.cuh)
-    unsigned long long max_bits = 0, *d_max = (unsigned long long *)tmp;
-    if (store & QEW_STORE_FP64) {
-        e = cudaMemsetAsync(d_max, 0, sizeof(*d_max), ctx->stream);
-        if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
-        const int blocks = (int)std::min<size_t>((N + 2047) / 2048, (size_t)ctx->num_sms * 8);
-        k_max_abs_bits<<<blocks, 256, 0, ctx->stream>>>(c64, N, d_max);
-        st = qew_launch_check(ctx, "max_abs");
-        if (st != QEW_OK) return cleanup(st);
-        e = cudaMemcpyAsync(&max_bits, d_max, sizeof(max_bits), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
-    }
-    e = cudaStreamSynchronize(ctx->stream);
+    unsigned long long max_bits = 0;
+    e = cudaMemcpyAsync(&max_bits, d_max, sizeof(max_bits), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "field build: %s", cudaGetErrorString(e)));
+    qew_free_async(d_max, ctx->stream);
+    d_max = nullptr;
     const int max_exp = (int)(max_bits >> 52);
     f->fixb = max_bits == 0 ? 1023 : (max_exp >= 256 && max_exp <= 1792) ? max_exp : -1;
     qew_free_async(tmp, ctx->stream);
@@ -376,36 +500,44 @@ qew_status qew_field_create_generated(qew_ctx *ctx, int nx, int ny, double Lx, d
         return qew_fail(ctx, QEW_ERR_INVALID, "field_create_generated: bad arguments");
     QEW_CUDA(ctx, cudaSetDevice(ctx->device));
     const size_t N = (size_t)nx * ny;
-    int Rx, Ry;
-    const std::vector<double> tx = gauss_taps(xi_x_cells, Rx), ty = gauss_taps(xi_y_cells, Ry);
-    double *w = nullptr, *t = nullptr, *taps = nullptr;
+    int Rx, Ry, qx, qy;
+    double gx, gy;
+    const std::vector<int2> tx = gauss_taps(xi_x_cells, Rx, qx, gx);
+    const std::vector<int2> ty = gauss_taps(xi_y_cells, Ry, qy, gy);
+    // samples in [-2^59, 2^59): 2^-F1 for the noise, 2^-F2 after the y filter
+    const int F1 = 59 - (int)ceil(log2(kNoiseMax));
+    const int F2 = 59 - std::max(0, (int)ceil(log2(kNoiseMax * gy)));
+    long long *w = nullptr, *t = nullptr;
+    double *stat = nullptr;
     auto cleanup = [&](qew_status s) {
         qew_free_async(w, ctx->stream);
         qew_free_async(t, ctx->stream);
-        qew_free_async(taps, ctx->stream);
+        qew_free_async(stat, ctx->stream);
         return s;
     };
     if (qew_alloc_async(ctx, (void **)&w, N * sizeof(double)) != QEW_OK ||
         qew_alloc_async(ctx, (void **)&t, N * sizeof(double)) != QEW_OK ||
-        qew_alloc_async(ctx, (void **)&taps, (tx.size() + ty.size() + 1) * sizeof(double)) != QEW_OK)
+        qew_alloc_async(ctx, (void **)&stat, 2 * sizeof(double) + (tx.size() + ty.size()) * sizeof(int2)) !=
+            QEW_OK)
         return cleanup(QEW_ERR_NOMEM);
-    double *tapx = taps, *tapy = taps + tx.size(), *scale = tapy + ty.size();
-    cudaError_t e = cudaMemcpyAsync(tapx, tx.data(), tx.size() * sizeof(double),
+    int2 *tapx = (int2 *)(stat + 2), *tapy = tapx + tx.size();
+    cudaError_t e = cudaMemcpyAsync(tapx, tx.data(), tx.size() * sizeof(int2),
                                     cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(tapy, ty.data(), ty.size() * sizeof(double), cudaMemcpyHostToDevice,
+        e = cudaMemcpyAsync(tapy, ty.data(), ty.size() * sizeof(int2), cudaMemcpyHostToDevice,
                             ctx->stream);
     if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
     const long pairs = (long)nx * ((ny + 1) / 2);
-    k_white_noise<<<(unsigned)((pairs + 255) / 256), 256, 0, ctx->stream>>>(w, nx, ny, seed);
+    k_white_noise<<<(unsigned)((pairs + 255) / 256), 256, 0, ctx->stream>>>(w, nx, ny, seed, F1);
     const unsigned blocks = (unsigned)((N + 255) / 256);
-    k_gauss_conv<<<blocks, 256, 0, ctx->stream>>>(w, t, nx, ny, tapy, Ry, 1);
-    k_gauss_conv<<<blocks, 256, 0, ctx->stream>>>(t, w, nx, ny, tapx, Rx, 0);
-    k_std_scale<<<1, 1024, 0, ctx->stream>>>(w, N, amplitude, scale);
-    k_scale_inplace<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(w, N, scale);
-    qew_status st = qew_launch_check(ctx, "field_generate", 5);
+    // a filtered sum is in units of 2^(55 - F - q) (k_gauss_conv)
+    k_gauss_conv<false><<<blocks, 256, 0, ctx->stream>>>(w, t, nx, ny, tapy, Ry, 1, F1 + qy - 55 - F2);
+    k_gauss_conv<true><<<blocks, 256, 0, ctx->stream>>>(t, w, nx, ny, tapx, Rx, 0, 55 - F2 - qx);
+    qew_status st = qew_launch_check(ctx, "field_generate", 3);
     if (st != QEW_OK) return cleanup(st);
-    st = field_build(ctx, w, true, nx, ny, Lx, Ly, store_flags, out);
+    st = field_moments(ctx, (const double *)w, N, amplitude, stat);
+    if (st != QEW_OK) return cleanup(st);
+    st = field_build(ctx, (const double *)w, true, nx, ny, Lx, Ly, store_flags, out, stat + 1);
     return cleanup(st);
 }
 
@@ -478,13 +610,12 @@ qew_status qew_field_create_seeded(qew_ctx *ctx, int nx, int ny, double Lx, doub
     if (cufftSetStream(plan, ctx->stream) != CUFFT_SUCCESS ||
         cufftExecZ2Z(plan, spec, spec, CUFFT_INVERSE) != CUFFT_SUCCESS)
         return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "field_create_seeded: inverse FFT failed"));
-    double *scale = w + N;
+    double *stat = w + N;
     k_real_part<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(spec, N, 1.0 / (double)N, w);
-    k_std_scale<<<1, 1024, 0, ctx->stream>>>(w, N, amplitude, scale);
-    k_scale_inplace<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(w, N, scale);
-    qew_status st = qew_launch_check(ctx, "field_seeded", 3);
+    qew_status st = qew_launch_check(ctx, "field_seeded");
+    if (st == QEW_OK) st = field_moments(ctx, w, N, amplitude, stat);
     if (st != QEW_OK) return cleanup(st);
-    return cleanup(field_build(ctx, w, true, nx, ny, Lx, Ly, store_flags, out));
+    return cleanup(field_build(ctx, w, true, nx, ny, Lx, Ly, store_flags, out, stat + 1));
 }
 
 qew_status qew_field_create_analytic(qew_ctx *ctx, int kind, double p0, double p1, double p2,

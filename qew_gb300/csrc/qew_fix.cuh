@@ -25,12 +25,12 @@ struct FxFrac {
     int t1, t0;
 };
 
-__device__ __forceinline__ FxFrac fx_frac(unsigned long long t64) {  // t = t64 * 2^-64
+__host__ __device__ __forceinline__ FxFrac fx_frac(unsigned long long t64) {  // t = t64 * 2^-64
     return FxFrac{(int)(t64 >> 33), (int)((unsigned)(t64 >> 2) & 0x7fffffffu)};
 }
 
 // floor-like (w * t): within 2 units of w * t. |w| < 2^62.
-__device__ __forceinline__ long long fx_mul(long long w, FxFrac t) {
+__host__ __device__ __forceinline__ long long fx_mul(long long w, FxFrac t) {
     const int w1 = (int)(w >> 31);
     const int w0 = (int)((unsigned)w & 0x7fffffffu);
     const long long mid = (long long)w1 * t.t0 + (long long)w0 * t.t1;
@@ -38,15 +38,35 @@ __device__ __forceinline__ long long fx_mul(long long w, FxFrac t) {
 }
 
 // u >> s for s >= 0, zero from 64 on (the PTX shift clamps its amount).
-__device__ __forceinline__ unsigned long long fx_shr(unsigned long long u, int s) {
+__host__ __device__ __forceinline__ unsigned long long fx_shr(unsigned long long u, int s) {
+#ifdef __CUDA_ARCH__
     unsigned long long r;
     asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(u), "r"(s));
     return r;
+#else
+    return s < 64 ? u >> s : 0ull;
+#endif
 }
-__device__ __forceinline__ unsigned long long fx_shl(unsigned long long u, int s) {
+__host__ __device__ __forceinline__ unsigned long long fx_shl(unsigned long long u, int s) {
+#ifdef __CUDA_ARCH__
     unsigned long long r;
     asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(u), "r"(s));
     return r;
+#else
+    return s < 64 ? u << s : 0ull;
+#endif
+}
+// Leading zeros (64 for 0).
+__host__ __device__ __forceinline__ int fx_clz(unsigned long long u) {
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)u);
+#else
+    return u ? __builtin_clzll(u) : 64;
+#endif
+}
+// The limbs of a signed number v * 2^-62, |v| < 2^62.
+__host__ __device__ __forceinline__ FxFrac fx_limbs(long long v) {
+    return FxFrac{(int)(v >> 31), (int)((unsigned)v & 0x7fffffffu)};
 }
 
 // An FP64 number c, |c| < 2^K with K = kb - 1022, in units of
@@ -62,16 +82,20 @@ __device__ __forceinline__ long long fx_tap(double c, int kb) {
     return ((long long)fx_shr(m, s) ^ sg) - sg;
 }
 
-// r as an FP64 number, rounded to nearest (ties away from zero): the integer
-// form of the conversion, which the FP64 unit would take 64 cycles for.
-__device__ __forceinline__ double fx_to_double(long long r) {
+// The bits of r * 2^k as an FP64 number, rounded to nearest (ties away from
+// zero), for a result in the normal range: the integer form of the
+// conversion, which the FP64 unit would take 64 cycles for.
+__host__ __device__ __forceinline__ unsigned long long fx_double_bits(long long r, int k) {
     const long long sg = r >> 63;
     const unsigned long long a = (unsigned long long)((r ^ sg) - sg);
-    const int lz = __clzll((long long)a);
+    const int lz = fx_clz(a);
     const unsigned long long n = fx_shl(a, lz);  // leading bit at 63 (0 for r == 0)
     const unsigned long long m = (n >> 11) + ((n >> 10) & 1ull);
-    const unsigned long long b = ((unsigned long long)(unsigned)(1085 - lz) << 52) + m;
-    return __longlong_as_double(a ? (long long)(b | ((unsigned long long)sg << 63)) : 0ll);
+    const unsigned long long b = ((unsigned long long)(unsigned)(1085 + k - lz) << 52) + m;
+    return a ? (b | ((unsigned long long)sg << 63)) : 0ull;
+}
+__device__ __forceinline__ double fx_to_double(long long r, int k = 0) {
+    return __longlong_as_double((long long)fx_double_bits(r, k));
 }
 
 // floor(g) and the fraction of g = a * 2^k for a field of n cells, from the
@@ -121,15 +145,14 @@ __device__ __forceinline__ long long fx_cubic_6v(const long long E[4], FxFrac t)
 __device__ __forceinline__ void fx_weights(FxFrac t, FxFrac w[4]) {
     const long long one = (1ll << 62) - 1;
     const FxFrac sixth{357913941, 715827882};  // 2^62 / 6
-    auto frac = [](long long v) { return FxFrac{(int)(v >> 31), (int)((unsigned)v & 0x7fffffffu)}; };
     const long long T = ((long long)t.t1 << 31) | (long long)t.t0;
     const long long o = one - T;
-    const FxFrac fo = frac(o);
+    const FxFrac fo = fx_limbs(o);
     const long long t2 = fx_mul(T, t), o3 = fx_mul(fx_mul(o, fo), fo), t3 = fx_mul(t2, t);
     const long long w0 = fx_mul(o3, sixth), w3 = fx_mul(t3, sixth);
     const long long w1 = 3074457345618258603ll - t2 + (t3 >> 1);  // 2/3 - t^2 + t^3/2
-    w[0] = frac(w0);
-    w[1] = frac(w1);
-    w[2] = frac(one - w0 - w1 - w3);
-    w[3] = frac(w3);
+    w[0] = fx_limbs(w0);
+    w[1] = fx_limbs(w1);
+    w[2] = fx_limbs(one - w0 - w1 - w3);
+    w[3] = fx_limbs(w3);
 }
