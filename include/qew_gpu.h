@@ -85,13 +85,13 @@ enum { QEW_STORE_FP64 = 1, QEW_STORE_FP32 = 2, QEW_STORE_FP32_EDGE = 4,
 /* FP64_POLY (only together with FP64) adds, for the same lines (one point
  * per field column), the FP64 cell polynomials of the x-filtered field: for
  * column e and row cell j the cubic V(e + 1/2, (j + t) dy), t in [0, 1), as
- * four FP64 numbers {q0, q1, q2, v0} with dV/dy = q0 + t (q1 + t q2) and
- * V = v0 + dy t (q0 + t (q1/2 + t q2/3)), computed once in FP64 from the
- * prefiltered coefficients (4x the FP64 coefficient memory, 32 bytes per
+ * four 64-bit fixed-point numbers, taken from the prefiltered coefficients
+ * when the field is built (4x the FP64 coefficient memory, 32 bytes per
  * cell). The FP64 gradient on such a line then reads one 32-byte cell per
- * edge and evaluates two FMAs instead of the 16-tap tensor sum. Results stay
- * within 1e-15 of the gradient scale of the reference's order; they are not
- * bitwise equal to it (QEW_PREC_FP64_REFERENCE keeps that order). */
+ * edge and evaluates two integer products instead of the 16-tap tensor sum.
+ * Results stay within 1e-15 of the gradient scale of the reference's order;
+ * they are not bitwise equal to it (QEW_PREC_FP64_REFERENCE keeps that
+ * order). */
 
 /* Precision of the gather in the model kernels. FP64 is the drop-in (parity)
  * form: it uses the FP64_POLY store when the field holds it and the line has

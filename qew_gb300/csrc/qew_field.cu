@@ -405,7 +405,7 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
         qew_free_async(d_max, ctx->stream);
         qew_free_async(f->coef32, ctx->stream);
         qew_free_async(f->edge32, ctx->stream);
-        qew_free_async(f->poly64, ctx->stream);
+        qew_free_async(f->poly, ctx->stream);
         cudaStreamSynchronize(ctx->stream);
         delete f;
         return s;
@@ -449,9 +449,9 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
         if (st != QEW_OK) return cleanup(st);
     }
     if (store & QEW_STORE_FP64_POLY) {
-        if (qew_alloc_async(ctx, (void **)&f->poly64, 4 * N * sizeof(double)) != QEW_OK)
+        if (qew_alloc_async(ctx, (void **)&f->poly, 4 * N * sizeof(long long)) != QEW_OK)
             return cleanup(QEW_ERR_NOMEM);
-        st = qew_poly_store_build(ctx, c64, nx, ny, f->dy, f->poly64);
+        st = qew_poly_store_build(ctx, c64, nx, ny, d_max, f->poly);
         if (st != QEW_OK) return cleanup(st);
     }
     // the bound of the fixed-point gather (qew_fix.cuh)
@@ -462,7 +462,12 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
     qew_free_async(d_max, ctx->stream);
     d_max = nullptr;
     const int max_exp = (int)(max_bits >> 52);
+    // (1023 for the zero field; outside the range no fixed point and no store)
     f->fixb = max_bits == 0 ? 1023 : (max_exp >= 256 && max_exp <= 1792) ? max_exp : -1;
+    if (f->fixb < 0 && f->poly) {
+        qew_free_async(f->poly, ctx->stream);
+        f->poly = nullptr;
+    }
     qew_free_async(tmp, ctx->stream);
     tmp = nullptr;
     if (store & QEW_STORE_FP64) {
@@ -637,12 +642,12 @@ qew_status qew_field_destroy(qew_field *f) {
     if (!f) return QEW_OK;
     cudaSetDevice(f->device);
     // the coefficients may be in use on any stream: wait for the device
-    const bool held = f->coef64 || f->coef32 || f->edge32 || f->poly64;
+    const bool held = f->coef64 || f->coef32 || f->edge32 || f->poly;
     if (held) cudaDeviceSynchronize();
     qew_free_async(f->coef64, f->stream);
     qew_free_async(f->coef32, f->stream);
     qew_free_async(f->edge32, f->stream);
-    qew_free_async(f->poly64, f->stream);
+    qew_free_async(f->poly, f->stream);
     if (held) cudaStreamSynchronize(f->stream);
     delete f;
     return QEW_OK;
@@ -655,7 +660,7 @@ void qew_field_release_on(qew_field *f, cudaStream_t stream) {
     qew_free_async(f->coef64, stream);
     qew_free_async(f->coef32, stream);
     qew_free_async(f->edge32, stream);
-    qew_free_async(f->poly64, stream);
+    qew_free_async(f->poly, stream);
     delete f;
 }
 

@@ -98,46 +98,78 @@ __device__ __forceinline__ double fx_to_double(long long r, int k = 0) {
     return __longlong_as_double((long long)fx_double_bits(r, k));
 }
 
-// floor(g) and the fraction of g = a * 2^k for a field of n cells, from the
-// bits of a: false for what the reference's fold has to see (negative or
-// non-finite a, g >= 2^30, a height whose cell is the last one of a period
-// above the first, where the reference's division may round up).
+// Row cell and fraction of g = a * 2^k in a period of n cells, from the bits
+// of a: the numbers that the reference's fold gives (filtered_noise.h:80-92),
+// which rounds a negative g's sum with the period to FP64. False for what the
+// FP64 code has to decide: non-finite or subnormal a, |g| >= 2^30, and the
+// last cell of a period other than the first two about zero, where the
+// reference's division by the period may round up.
 __device__ __forceinline__ bool fx_cell(double a, int k, int n, int &iy, FxFrac &t) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-    const int ef = (int)(b >> 52);  // sign bit and biased exponent
+    const int ef = (int)(b >> 52) & 0x7FF;
     const int e = ef + k - 1023;
-    if (ef == 0 || ef >= 2047 || e > 29) {
+    if (ef == 0 || ef == 2047 || e > 29) {
         iy = 0;
         t = FxFrac{0, 0};
-        return b == 0ull;
+        return (b << 1) == 0ull;
     }
     const unsigned long long m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
     const int up = 12 + e;  // fraction bits to the top of 64 (the integer part leaves)
-    t = fx_frac(up >= 0 ? fx_shl(m, up) : fx_shr(m, -up));
+    unsigned long long f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
     iy = e >= 0 ? (int)fx_shr(m, 52 - e) : 0;
-    if (iy >= n) {
-        const int q = iy / n;
-        iy -= q * n;
-        return iy + 1 < n;
+    bool ok = true;
+    if ((long long)b < 0) {
+        if (n == 1) return false;
+        ok = iy < n;
+        iy = f ? -iy - 1 : -iy;
+        f = 0ull - f;
+        iy %= n;
+        if (iy < 0) iy += n;
+        ok = ok || iy + 1 < n;
+        if (iy > 0) {  // round g + period to FP64 (to nearest even)
+            const int drop = 43 - __clz(iy);  // 12 + floor(log2(iy))
+            const unsigned long long add = ((1ull << (drop - 1)) - 1ull) + ((f >> drop) & 1ull);
+            const bool carry = f + add < f;
+            f = ((f + add) >> drop) << drop;
+            if (carry) {
+                f = 0ull;
+                iy = (iy + 1 == n) ? 0 : iy + 1;
+            }
+        }
+    } else if (iy >= n) {
+        iy %= n;
+        ok = iy + 1 < n;
     }
-    return true;
+    t = fx_frac(f);
+    return ok;
 }
 
-// The four stencil rows' sums E (|E| <= 2^58) at fraction t, times 2:
-// dV/dt = (E2 - E0)/2 + t (u + t w/2), u = E0 - 2 E1 + E2,
-// w = (E3 - E0) - 3 (E2 - E1): the derivative of filtered_noise.h:33-62's
-// cubic, summed in the unit of E.
-__device__ __forceinline__ long long fx_cubic_dt2(const long long E[4], FxFrac t) {
-    const long long u = E[0] + E[2] - 2 * E[1];
-    const long long w = (E[3] - E[0]) - 3 * (E[2] - E[1]);
-    return (E[2] - E[0]) + fx_mul(2 * u + fx_mul(w, t), t);
-}
-// The value, times 6 (|E| <= 2^57): (E0 + 4 E1 + E2) + t (3 (E2 - E0) + t (3 u + t w)).
-__device__ __forceinline__ long long fx_cubic_6v(const long long E[4], FxFrac t) {
+// The cubic along y in one cell, from the four stencil rows' sums E
+// (|E| <= 2^57.6, in some unit): with u = E0 - 2 E1 + E2 and
+// w = (E3 - E0) - 3 (E2 - E1) (filtered_noise.h:33-62 expanded in t)
+//   2 dV/dt = p + t (2u + t w),   6 V = v + t (3p + t (3u + t w)),
+// p = E2 - E0, v = E0 + 4 E1 + E2. Every bracket is a mean of differences of
+// E, so it stays below 12 max|E| < 2^62 (fx_mul's range).
+struct FxCubic {
+    long long v, p, u2, w;  // u2 = 2u
+};
+__device__ __forceinline__ FxCubic fx_cubic(const long long E[4]) {
     const long long s = E[0] + E[2];
-    const long long u = s - 2 * E[1];
-    const long long w = (E[3] - E[0]) - 3 * (E[2] - E[1]);
-    return s + 4 * E[1] + fx_mul(3 * (E[2] - E[0]) + fx_mul(3 * u + fx_mul(w, t), t), t);
+    return FxCubic{s + 4 * E[1], E[2] - E[0], 2 * s - 4 * E[1], (E[3] - E[0]) - 3 * (E[2] - E[1])};
+}
+__device__ __forceinline__ long long fx_dt2(const FxCubic &c, FxFrac t) {
+    return c.p + fx_mul(c.u2 + fx_mul(c.w, t), t);
+}
+__device__ __forceinline__ long long fx_6v(const FxCubic &c, FxFrac t) {
+    return c.v + fx_mul(3 * c.p + fx_mul(c.u2 + (c.u2 >> 1) + fx_mul(c.w, t), t), t);
+}
+// One cell of the cell-polynomial store: 32 bytes, 32-byte aligned.
+__device__ __forceinline__ FxCubic fx_load_cell(const long long *p) {
+    FxCubic c;
+    asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(c.v), "=l"(c.p), "=l"(c.u2), "=l"(c.w)
+        : "l"(p));
+    return c;
 }
 
 // The cubic B-spline weights (filtered_noise.h:33-44) at fraction t, in units
@@ -156,3 +188,33 @@ __device__ __forceinline__ void fx_weights(FxFrac t, FxFrac w[4]) {
     w[2] = fx_limbs(one - w0 - w1 - w3);
     w[3] = fx_limbs(w3);
 }
+
+// 1 / sqrt(1 + dh^2). As FP64 instructions the root takes 7 of 64 cycles each;
+// here it is in units of 2^-62 from the single precision root w0 and its
+// exact error r = 1 - w0^2 - (w0 dh)^2 to second order (the third is below
+// 2^-62), about 100 cycles of integer instructions. |dh| outside [2^-30, 2^8)
+// takes FP64's rsqrt (the small ones: 1 to rounding).
+__device__ __forceinline__ double fx_invroot(double dh) {
+    const unsigned hi = (unsigned)__double2hiint(dh), lo = (unsigned)__double2loint(dh);
+    const int x = (int)((hi >> 20) & 0x7FFu) - 1023;  // |dh| in [2^x, 2^(x+1))
+    if (x < -30 || x > 7) return rsqrt(fma(dh, dh, 1.0));
+    const unsigned mh = (hi & 0x000FFFFFu) | 0x00100000u;
+    // |dh| = M 2^(x - 61), M in [2^61, 2^62)
+    const unsigned long long M = ((unsigned long long)__funnelshift_l(lo, mh, 9) << 32) |
+                                 (unsigned long long)(lo << 9);
+    const float f = __int_as_float((int)(((x + 127) << 23) | (__funnelshift_l(lo, mh, 3) & 0x7FFFFF)));
+    const float w0f = rsqrtf(fmaf(f, f, 1.0f));
+    const unsigned w0 = (unsigned)(w0f * 2147483648.0f);  // 2^-31, at most 2^31
+    // t = w0 |dh| in units of 2^-62 (below 2^62: w0 |dh| < 1 by more than r)
+    const unsigned long long p = (M >> 31) * w0 + (((M & 0x7fffffffull) * w0) >> 31);  // 2^(x-61)
+    const unsigned long long t = x < 0 ? fx_shr(p, -1 - x) : fx_shl(p, x + 1);
+    const long long ww = (long long)((unsigned long long)w0 * w0);  // w0^2, 2^-62
+    const long long r = (1ll << 62) - ww - fx_mul((long long)t, fx_limbs((long long)t));  // |r| < 2^42
+    const long long r1 = r >> 20;
+    const long long c = (r >> 1) + ((3 * ((r1 * r1) >> 22)) >> 3);
+    // w = w0 (1 + c)
+    const long long w = ((long long)w0 << 31) + (((c >> 10) * (long long)w0) >> 21);
+    return fx_to_double(w, -62);
+}
+// dh / sqrt(1 + dh^2)
+__device__ __forceinline__ double fx_slope(double dh) { return __dmul_rn(dh, fx_invroot(dh)); }

@@ -65,7 +65,7 @@ struct qew_field {
     double *coef64 = nullptr;  // [ny][nx], x fastest
     float *coef32 = nullptr;   // [ny][nx], x fastest
     float *edge32 = nullptr;   // [ny][nx]: coefficients filtered along x at e + 1/2
-    double *poly64 = nullptr;  // [ny][nx][4]: FP64 cell polynomials of the x-filtered field
+    long long *poly = nullptr;  // [ny][nx][4]: cell polynomials of the x-filtered field (FxCubic)
     int fixb = -1;  // biased exponent of the largest |coefficient| (qew_fix.cuh), -1: none usable
     cudaStream_t stream = nullptr;  // stream the coefficients were allocated on
 };
@@ -227,72 +227,8 @@ __host__ __device__ __forceinline__ LineDx make_line_dx(double physical_size, in
     return L;
 }
 
-// ------------------------------------------ FP64 cell-polynomial store
-// (QEW_STORE_FP64_POLY): per (row cell j, column e) the cubic of the
-// x-filtered field at x = e + 1/2 in the row fraction t, as
-// {q0, q1, q2, v0} with dV/dy = q0 + t (q1 + t q2) and
-// V = v0 + dy t (q0 + t (q1/2 + t q2/3)); qew_poly.cuh derives it.
-// Marker for a row spacing that is not a power of two.
+// Marker for a spacing that is not a power of two.
 constexpr int kPolyNotPow2 = 1 << 20;
-
-// 256-bit read-only load of one cell {q0, q1, q2, v0} (32-byte aligned).
-__device__ __forceinline__ void poly_load4(const double *p, double &q0, double &q1, double &q2,
-                                           double &v0) {
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-        : "=d"(q0), "=d"(q1), "=d"(q2), "=d"(v0)
-        : "l"(p));
-}
-__device__ __forceinline__ void poly_load3(const double *p, double &q0, double &q1, double &q2) {
-    double v0;
-    poly_load4(p, q0, q1, q2, v0);
-}
-
-// g = a * 2^k. When g is finite, normal and in [0, ny) (ny < 2^30): iy =
-// floor(g), t = g - iy exactly, and true; otherwise false (negative, >= ny,
-// non-finite or subnormal heights take the reference's fold instead). Only
-// integer operations on the bits of a.
-__device__ __forceinline__ bool poly_cell_exact(double a, int k, int ny, int &iy, double &t) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
-    const int ef = (int)(b >> 52);  // sign bit and biased exponent
-    if (ef == 0) {                  // +0 (or a subnormal: the slow path)
-        iy = 0;
-        t = 0.0;
-        return b == 0ull;
-    }
-    if (ef >= 2047) return false;   // negative, infinite or NaN
-    const int eb = ef + k;          // biased exponent of g
-    if (eb <= 0) return false;
-    const int e = eb - 1023;
-    if (e < 0) {                    // g in (0, 1): cell 0, t = g
-        iy = 0;
-        t = __longlong_as_double((long long)(b + ((unsigned long long)(long long)k << 52)));
-        return true;
-    }
-    if (e > 29) return false;
-    const unsigned long long m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-    const int sh = 52 - e;          // 23 .. 52 fraction bits
-    iy = (int)(m >> sh);
-    if (iy >= ny) return false;
-    const unsigned long long fb = m & ((1ull << sh) - 1ull);
-    if (fb == 0ull) {
-        t = 0.0;
-        return true;
-    }
-    const int top = 63 - __clzll((long long)fb);  // leading bit of the fraction, < sh
-    const unsigned long long mant = (fb << (52 - top)) & 0x000FFFFFFFFFFFFFull;
-    t = __longlong_as_double((long long)(((unsigned long long)(top - sh + 1023) << 52) | mant));
-    return true;
-}
-
-// dV/dy and V of a cell at fraction t.
-__device__ __forceinline__ double poly_dvdy(double q0, double q1, double q2, double t) {
-    return fma(fma(q2, t, q1), t, q0);
-}
-__device__ __forceinline__ double poly_value(double q0, double q1, double q2, double v0, double t,
-                                             double dy) {
-    const double third = 1.0 / 3.0;
-    return fma(dy * t, fma(fma(q2 * third, t, 0.5 * q1), t, q0), v0);
-}
 
 struct NoiseBSpline64;
 // NoiseBSpline64::dvdy (deriv) / value out of line: the FP64 16-tap sum, for
@@ -314,14 +250,14 @@ struct NoiseBSpline64 {
     // grid x = e + 1/2 exactly, so its cell is e and its x weights are those
     // of t = 1/2 (bit-identical to locating it).
     bool xconst;
-    // The field's FP64 cell-polynomial store when it serves this line (one
-    // point per field column), else null; ky: y * 2^ky == y / dy exactly
-    // (kPolyNotPow2 when dy is not a power of two); kx the same for x.
-    const double *__restrict__ poly;
+    // The field's cell-polynomial store (QEW_STORE_FP64_POLY) when it serves
+    // this line (one point per field column), else null. ky: y * 2^ky == y / dy
+    // exactly (kPolyNotPow2 when dy is not a power of two); kx the same for x.
+    const long long *__restrict__ poly;
     int ky, kx;
     // The 16-tap sums in 64-bit fixed point (qew_fix.cuh): the field's bound
     // kb (-1: FP64 sums) and the units of 2 dV/dt / dy and of 6 V, for the
-    // constant x weights (xconst) and for general ones.
+    // constant x weights (xconst and the store) and for general ones.
     int kb;
     double fx_dv_c, fx_v_c, fx_dv_g, fx_v_g;
     QEW_OOB_MEMBER
@@ -392,14 +328,6 @@ struct NoiseBSpline64 {
         }
     }
 
-    // Row cell and fraction of height y: from y's bits when dy is a power of
-    // two and y / dy lies in [0, ny), else the reference's locate.
-    __device__ __forceinline__ void poly_row(double y, int &iy, double &t) const {
-        const bool ok = (ky != kPolyNotPow2) ? poly_cell_exact(y, ky, ny, iy, t)
-                                              : poly_cell_exact(y * inv_dy, 0, ny, iy, t);
-        if (!ok) grid_locate(y, dy, inv_dy, dy_pow2, ny, iy, t);
-    }
-
     __device__ __forceinline__ double c(int ix, int iy) const {
         ix = QEW_IDX(ix, nx, oob);
         iy = QEW_IDX(iy, ny, oob);
@@ -448,67 +376,104 @@ struct NoiseBSpline64 {
         }
         return dy_pow2 ? dg * inv_dy : dg / dy;
     }
-    // dV/dy / V at the midpoint of edge e (xc its physical x). With the
-    // cell-polynomial store: one 32-byte cell and two FMAs (the wrap edge,
-    // e = nx - 1, is not at a half-integer column and keeps the 16 taps).
-    // Without it, the 16 taps in fixed point; what its locate declines
-    // (negative or huge heights, non-finite ones) is summed in FP64. The last
-    // product is never contracted, so every kernel gets the same bits.
-    __device__ __forceinline__ double dvdy_edge(int e, double xc, double y) const {
-        if (poly && e + 1 < nx) {
-            int iy;
-            double t, q0, q1, q2;
-            poly_row(y, iy, t);
-            iy = QEW_IDX(iy, ny, oob);
-            e = QEW_IDX(e, nx, oob);
-            poly_load3(poly + ((size_t)iy * (size_t)nx + (size_t)e) * 4, q0, q1, q2);
-            return poly_dvdy(q0, q1, q2, t);
-        }
-        if (kb >= 0) {
-            int ix, iy;
-            FxFrac fx, fy;
-            if (fx_locate(y, dy, inv_dy, ky, ny, iy, fy)) {
-                long long E[4];
-                if (xconst && e + 1 < nx) {
-                    fx_rows_const(e, iy, E);
-                    return __dmul_rn(fx_to_double(fx_cubic_dt2(E, fy)), fx_dv_c);
-                }
-                if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
-                    fx_rows(ix, fx, iy, E);
-                    return __dmul_rn(fx_to_double(fx_cubic_dt2(E, fy)), fx_dv_g);
-                }
-            }
-        }
-        return bspline_slow(*this, true, xc, y);
+    // Whether edge e sits at a half-integer column with the constant x
+    // weights: every one but the wrap edge (e = nx - 1, at x = (n - 1) dx / 2),
+    // on the store or on a grid that makes it exact.
+    __device__ __forceinline__ bool fx_const(int e) const {
+        return (poly || xconst) && e + 1 < nx;
     }
-    __device__ __forceinline__ double value_edge(int e, double xc, double y) const {
-        if (poly && e + 1 < nx) {
-            int iy;
-            double t, q0, q1, q2, v0;
-            poly_row(y, iy, t);
+    // The cubic along y of edge e in row cell iy, constant x weights: one
+    // 32-byte cell of the store, or the 16 taps; the same integers either way.
+    __device__ __forceinline__ FxCubic fx_const_cell(int e, int iy) const {
+        if (poly) {
             iy = QEW_IDX(iy, ny, oob);
             e = QEW_IDX(e, nx, oob);
-            poly_load4(poly + ((size_t)iy * (size_t)nx + (size_t)e) * 4, q0, q1, q2, v0);
-            return poly_value(q0, q1, q2, v0, t, dy);
+            return fx_load_cell(poly + ((size_t)iy * (size_t)nx + (size_t)e) * 4);
         }
+        long long E[4];
+        fx_rows_const(e, iy, E);
+        return fx_cubic(E);
+    }
+    // Row cell and fraction of the edge midpoint at height a / 2.
+    // (On the store of a spacing that is no power of two by one product, within
+    // an ulp of the quotient.)
+    __device__ __forceinline__ bool fx_row(double a, int &iy, FxFrac &t) const {
+        if (poly && ky == kPolyNotPow2) return fx_cell(a * (0.5 * inv_dy), 0, ny, iy, t);
+        return fx_locate(a, 2.0 * dy, 0.5 * inv_dy, ky == kPolyNotPow2 ? ky : ky - 1, ny, iy, t);
+    }
+    // dV/dy of an edge e < nx - 1 on the store.
+    __device__ __forceinline__ double dvdy_edge_store(int e, double a) const {
+        int iy;
+        FxFrac fy;
+        if (!fx_row(a, iy, fy)) {
+            double t;
+            grid_locate(a * 0.5, dy, inv_dy, dy_pow2, ny, iy, t);
+            if (!(t >= 0.0)) return a - a;  // NaN
+            fy = fx_frac((unsigned long long)(fmin(t, 1.0 - 0x1p-53) * 0x1p64));
+        }
+        return __dmul_rn(fx_to_double(fx_dt2(fx_const_cell(e, iy), fy)), fx_dv_c);
+    }
+    // dV/dy / V at the midpoint of edge e (xc its physical x, a the sum of its
+    // two heights) in fixed point; what its locate declines (negative or huge
+    // heights, non-finite ones) is summed in FP64. The last product is never
+    // contracted, so every kernel gets the same bits.
+    __device__ __forceinline__ double dvdy_edge_sum(int e, double xc, double a) const {
         if (kb >= 0) {
             int ix, iy;
             FxFrac fx, fy;
-            if (fx_locate(y, dy, inv_dy, ky, ny, iy, fy)) {
-                long long E[4];
-                if (xconst && e + 1 < nx) {
-                    fx_rows_const(e, iy, E);
-                } else if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
+            if (fx_row(a, iy, fy)) {
+                if (fx_const(e))
+                    return __dmul_rn(fx_to_double(fx_dt2(fx_const_cell(e, iy), fy)), fx_dv_c);
+                if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
+                    long long E[4];
                     fx_rows(ix, fx, iy, E);
-                } else {
-                    return bspline_slow(*this, false, xc, y);
+                    return __dmul_rn(fx_to_double(fx_dt2(fx_cubic(E), fy)), fx_dv_g);
                 }
-#pragma unroll
-                for (int b = 0; b < 4; ++b) E[b] >>= 1;
-                return __dmul_rn(fx_to_double(fx_cubic_6v(E, fy)), (xconst && e + 1 < nx) ? fx_v_c : fx_v_g);
             }
         }
-        return bspline_slow(*this, false, xc, y);
+        return bspline_slow(*this, true, xc, a * 0.5);
+    }
+    __device__ __forceinline__ double value_edge_sum(int e, double xc, double a) const {
+        if (kb >= 0) {
+            int ix, iy;
+            FxFrac fx, fy;
+            if (fx_row(a, iy, fy)) {
+                if (fx_const(e))
+                    return __dmul_rn(fx_to_double(fx_6v(fx_const_cell(e, iy), fy)), fx_v_c);
+                if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
+                    long long E[4];
+                    fx_rows(ix, fx, iy, E);
+                    return __dmul_rn(fx_to_double(fx_6v(fx_cubic(E), fy)), fx_v_g);
+                }
+            }
+        }
+        return bspline_slow(*this, false, xc, a * 0.5);
+    }
+    // Both at once, from one cell: the numbers that the two give.
+    __device__ __forceinline__ void both_edge_sum(int e, double xc, double a, double &v,
+                                                  double &dv) const {
+        if (kb >= 0) {
+            int ix, iy;
+            FxFrac fx, fy;
+            if (fx_row(a, iy, fy)) {
+                const bool cst = fx_const(e);
+                if (cst || fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
+                    FxCubic q;
+                    if (cst) {
+                        q = fx_const_cell(e, iy);
+                    } else {
+                        long long E[4];
+                        fx_rows(ix, fx, iy, E);
+                        q = fx_cubic(E);
+                    }
+                    v = __dmul_rn(fx_to_double(fx_6v(q, fy)), cst ? fx_v_c : fx_v_g);
+                    dv = __dmul_rn(fx_to_double(fx_dt2(q, fy)), cst ? fx_dv_c : fx_dv_g);
+                    return;
+                }
+            }
+        }
+        v = bspline_slow(*this, false, xc, a * 0.5);
+        dv = bspline_slow(*this, true, xc, a * 0.5);
     }
     // sample, filtered_noise.h:103-134
     __device__ __forceinline__ void sample(double x, double y, double &v,
@@ -746,22 +711,34 @@ __device__ __forceinline__ unsigned long long *qew_noise_oob(const NoiseBSpline6
 }
 #endif
 
-// Edge accessors for every functor: the B-spline one has its own fast path.
+// Edge accessors for every functor, at the midpoint a / 2 of an edge whose
+// heights add up to a: the B-spline one has its own path.
 template <class Noise>
-__device__ __forceinline__ double noise_dvdy_edge(const Noise &nz, int, double xc, double y) {
-    return nz.dvdy(xc, y);
+__device__ __forceinline__ double noise_dvdy_edge(const Noise &nz, int, double xc, double a) {
+    return nz.dvdy(xc, a * 0.5);
 }
 template <class Noise>
-__device__ __forceinline__ double noise_value_edge(const Noise &nz, int, double xc, double y) {
-    return nz.value(xc, y);
+__device__ __forceinline__ double noise_value_edge(const Noise &nz, int, double xc, double a) {
+    return nz.value(xc, a * 0.5);
 }
 __device__ __forceinline__ double noise_dvdy_edge(const NoiseBSpline64 &nz, int e, double xc,
-                                                  double y) {
-    return nz.dvdy_edge(e, xc, y);
+                                                  double a) {
+    return nz.dvdy_edge_sum(e, xc, a);
 }
 __device__ __forceinline__ double noise_value_edge(const NoiseBSpline64 &nz, int e, double xc,
-                                                   double y) {
-    return nz.value_edge(e, xc, y);
+                                                   double a) {
+    return nz.value_edge_sum(e, xc, a);
+}
+
+template <class Noise>
+__device__ __forceinline__ void noise_both_edge(const Noise &nz, int e, double xc, double a,
+                                                double &v, double &dv) {
+    v = noise_value_edge(nz, e, xc, a);
+    dv = noise_dvdy_edge(nz, e, xc, a);
+}
+__device__ __forceinline__ void noise_both_edge(const NoiseBSpline64 &nz, int e, double xc, double a,
+                                                double &v, double &dv) {
+    nz.both_edge_sum(e, xc, a, v, dv);
 }
 
 // Host helpers building the functors from a field handle.
@@ -792,9 +769,7 @@ static inline NoiseBSpline64 make_bspline64(const qew_field *f, int n = 0,
     nz.inv_dy = 1.0 / f->dy;
     nz.dx_pow2 = qew_is_pow2(f->dx);
     nz.dy_pow2 = qew_is_pow2(f->dy);
-    nz.poly = (f->poly64 && f->coef64 && n > 0 && n == f->nx && physical_size == f->Lx)
-                  ? f->poly64
-                  : nullptr;
+    nz.poly = (f->poly && n > 0 && n == f->nx && physical_size == f->Lx) ? f->poly : nullptr;
     {
         int e;
         const double m = frexp(f->dy, &e);  // dy = m 2^e
@@ -808,9 +783,9 @@ static inline NoiseBSpline64 make_bspline64(const qew_field *f, int n = 0,
         const int K = f->fixb - 1022;  // |coefficient| < 2^K
         nz.kb = f->fixb;
         nz.fx_dv_c = ldexp(1.0, K - 53) / (48.0 * f->dy);
-        nz.fx_v_c = ldexp(1.0, K - 51) / 288.0;
+        nz.fx_v_c = ldexp(1.0, K - 52) / 288.0;
         nz.fx_dv_g = ldexp(1.0, K - 58) / f->dy;
-        nz.fx_v_g = ldexp(1.0, K - 56) / 6.0;
+        nz.fx_v_g = ldexp(1.0, K - 57) / 6.0;
     }
 #ifdef QEW_BOUNDS_CHECK
     nz.oob = qew_bounds_words();

@@ -30,33 +30,30 @@ __device__ __forceinline__ double edge_energy(const Noise &nz, int i, int ip, do
     else
         line_energy = lt * (sqrt(__dadd_rn(1.0, __dmul_rn(dh_dx, dh_dx))) - 1.0);
     const double xc = (double)(i + ip) * 0.5 * L.dx;
-    const double hc = (hip + hi) * 0.5;
-    return L.dx * __dsub_rn(__dadd_rn(line_energy, noise_value_edge(nz, i, xc, hc)),
+    return L.dx * __dsub_rn(__dadd_rn(line_energy, noise_value_edge(nz, i, xc, hip + hi)),
                             __dmul_rn(f, hi));
 }
 
 // Edge pass of gradient(), qew_model.h:163-175: dV/dy at the midpoint of edge
 // (e, e+1) and, for arclength, the normalised slope dh/sqrt(1+dh^2). Except
-// for the reference-exact functor the slope is dh * rsqrt(1 + dh^2) with dh
-// by multiplication: 9 FP64 instructions where the square root and the
-// divisions take 27 or more (an FP64 instruction of a warp occupies its
-// scheduler's FP64 unit for 64 cycles).
+// for the reference-exact functor dh comes by multiplication and the root in
+// fixed point: 3 FP64 instructions where the square root and the divisions
+// take 27 or more (an FP64 instruction of a warp occupies its scheduler's
+// FP64 unit for 64 cycles).
 template <class Noise>
 __device__ __forceinline__ void edge_gradient(const Noise &nz, int e, int n, double he,
                                               double hep, const LineDx &L, bool arc, double &dv,
                                               double &sl) {
     const int ep = (e + 1 == n) ? 0 : e + 1;
     const double xc = (double)(e + ep) * 0.5 * L.dx;
-    const double hc = (hep + he) * 0.5;
-    dv = noise_dvdy_edge(nz, e, xc, hc);
+    dv = noise_dvdy_edge(nz, e, xc, hep + he);
     sl = 0.0;
     if (arc) {
         if constexpr (noise_is_ref<Noise>::value) {
             const double dh = L.div(hep - he);
             sl = dh / sqrt(__dadd_rn(1.0, __dmul_rn(dh, dh)));
         } else {
-            const double dh = (hep - he) * L.inv_dx;
-            sl = dh * rsqrt(fma(dh, dh, 1.0));
+            sl = fx_slope((hep - he) * L.inv_dx);
         }
     }
 }

@@ -149,12 +149,12 @@ __device__ __forceinline__ unsigned long long *qew_noise_oob(const NoiseSplit32 
 }
 #endif
 __device__ __forceinline__ double noise_dvdy_edge(const NoiseSplit32 &nz, int e, double xc,
-                                                  double y) {
-    return nz.dvdy_edge(e, xc, y);
+                                                  double a) {
+    return nz.dvdy_edge(e, xc, a * 0.5);
 }
 __device__ __forceinline__ double noise_value_edge(const NoiseSplit32 &nz, int e, double xc,
-                                                   double y) {
-    return nz.value_edge(e, xc, y);
+                                                   double a) {
+    return nz.value_edge(e, xc, a * 0.5);
 }
 
 static inline NoiseSplit32 make_split32(const qew_field *f, int n, double physical_size) {

@@ -1,35 +1,26 @@
 // qew_poly.cu -- FP64 gradient on the cell-polynomial store (QEW_STORE_FP64_POLY).
 //
 // gradient() (qew_model.h:149-193) of lines with one point per field column,
-// in FP64 throughout: the edge pass reads one 32-byte cell of the store per
-// edge (the x-filtered field's cubic in the row fraction, built once with the
-// field) and evaluates dV/dy with two FMAs; the per-site combine is the
-// reference's, with its factors folded:
+// heights and gradients in FP64: the edge pass reads one 32-byte cell of the
+// store per edge (the x-filtered field's cubic in the row fraction, built
+// once with the field) and evaluates dV/dy in 64-bit fixed point; the
+// per-site combine is the reference's, with its factors folded:
 //   grad_i = dx (F_el,i + (dv_{i-1} + dv_i)/2 - f)
 //          = c_el d2h_i + (dx/2)(dv_{i-1} + dv_i) - dx f        (linear,
-//            c_el = -Gamma/dx, d2h_i = (h_{i-1} + h_{i+1}) - 2 h_i as the reference forms it)
+//            c_el = -Gamma/dx)
 //          = Gamma (s_{i-1} - s_i) + (dx/2)(dv_{i-1} + dv_i) - dx f  (arclength).
-// The row cell and fraction of each edge midpoint come from the bits of
-// h_e + h_{e+1} when the row spacing is a power of two (qew_poly.cuh), so an
-// edge of the linear model costs 3 FP64 instructions and a site 5.
 //
-// At f = 0 with dx/2 a power of two 2^k (kF0) the combine's first term is an
-// exact scaling: (dx/2)(dv_{i-1} + dv_i) == dv'_{i-1} + dv'_i bit for bit
-// with dv' = 2^k dv, and each edge forms dv' by adding k to the exponent
-// field of dv (integer instructions; the FP64 multiply where dv or dv' is
-// zero, subnormal or non-finite). A site then costs 4 FP64 instructions
-// instead of 5.
-//
-// Launch: persistent, batched (lines stored n apart), one CTA per resident
-// slot; each CTA walks tiles of kTile sites gridDim.x apart and copies the
-// next tile's heights into its spare shared buffer with cp.async while the
-// current tile's gathers are in flight. The wrap edge of each line (at
-// x = (n - 1) dx / 2, not a half-integer column) takes the 16-tap path.
+// Two kernels:
+//   k_gradient_poly_walk  the linear model: every step up to the last two
+//     multiply-adds in integers (below);
+//   k_gradient_poly       arclength: FP64 heights and combine, the cell and
+//     the slope's root in fixed point.
 #include <algorithm>
 #include <climits>
 #include <cmath>
 
 #include "qew_internal.cuh"
+#include "qew_model_kernels.cuh"
 #include "qew_poly.cuh"
 #include "qew_tune.cuh"
 
@@ -39,49 +30,22 @@ constexpr int kBS = 256;
 constexpr int kMinCtas = 4;  // 64 registers a thread: up to 4 resident CTAs per SM
 
 struct PolyGeom {
-    const double *poly;   // [ny][nx][4]
-    NoiseBSpline64 nz;    // 16-tap path of the wrap edge and the reference's fold
+    NoiseBSpline64 nz;    // the store, and the 16-tap path of the wrap edge
     int n;
-    int ky;               // (h_e + h_ep) * 2^ky = midpoint in row cells, or kPolyNotPow2
-    double half_inv_dy;   // 0.5 / dy when the spacing is not a power of two
+    int ky;               // (h_e + h_ep) [* recip] * 2^ky = midpoint in row cells
+    FxFrac recip;         // mantissa of 1 / (2 dy) in [1/2, 1) (not a power of two)
     LineDx L;
-    double c_el;          // -Gamma / dx
     double lt;            // Gamma
-    double half_dx, fdx;  // dx / 2, dx f
-    int half_dx_exp;      // k with dx / 2 == 2^k (the kF0 form)
+    double half_unit;     // dx / 2 * the unit of an edge's integer dV/dy
+    float inv_ny;
 };
 
-// v * scale for a zero, subnormal or non-finite v or result: a call of its
-// own, so the compiler cannot evaluate the multiply for every lane and
-// select (which would put the FP64 instruction back on every edge).
-__device__ __noinline__ double scale_pow2_slow(double v, double scale) { return v * scale; }
-
-// v * 2^k (scale == 2^k), exact: the exponent field moves by k when v and
-// the result are normal.
-__device__ __forceinline__ double scale_pow2(double v, int k, double scale) {
-    const int hi = __double2hiint(v);
-    const int e = (hi >> 20) & 0x7FF;
-    if (e != 0 && e + k >= 1 && e + k <= 2046)
-        return __hiloint2double(hi + (k << 20), __double2loint(v));
-    return scale_pow2_slow(v, scale);
-}
-
-// dV/dy at the midpoint of edge (e, e + 1 mod n) of heights he, hep.
-__device__ __forceinline__ double poly_edge_dvdy(const PolyGeom &g, int e, double he,
-                                                 double hep) {
-    const double a = hep + he;  // the reference's (h_ip + h_i), qew_model.h:168
-    if (e + 1 < g.n) {
-        int iy;
-        double t;
-        poly_locate(a, g.ky, g.half_inv_dy, g.nz, iy, t);
-        iy = QEW_IDX(iy, g.nz.ny, g.nz.oob);
-        e = QEW_IDX(e, g.nz.nx, g.nz.oob);
-        double q0, q1, q2;
-        poly_load3(g.poly + ((size_t)iy * (size_t)g.nz.nx + (size_t)e) * 4, q0, q1, q2);
-        return poly_dvdy(q0, q1, q2, t);
-    }
-    const double xc = (double)e * 0.5 * g.L.dx;  // (i + ip) dx / 2 with ip = 0
-    return g.nz.dvdy(xc, a * 0.5);
+// dV/dy of an edge that the integers do not cover (the wrap edge, a chunk of
+// FP64 sums): out of line, so that its general path takes no registers of
+// the kernels' loops.
+__device__ __noinline__ double walk_edge_rare(const PolyGeom &g, int e, double sum) {
+    const int ep = (e + 1 == g.n) ? 0 : e + 1;
+    return g.nz.dvdy_edge_sum(e, (double)(e + ep) * 0.5 * g.L.dx, sum);
 }
 
 // 8-byte asynchronous global -> shared copy.
@@ -90,13 +54,19 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
-template <bool kArc, int kItems, bool kF0>
+// Persistent, batched (lines stored n apart), one CTA per resident slot; each
+// CTA walks tiles of kTile sites gridDim.x apart and copies the next tile's
+// heights into its spare shared buffer with cp.async while the current
+// tile's gathers are in flight. Bound about equally by 10 FP64 instructions a
+// point and by issue: 8 lines of 2^20 points 262 -> 178 us.
+template <int kItems>
 __global__ void __launch_bounds__(kBS, kMinCtas)
-k_gradient_poly(const double *__restrict__ h, PolyGeom g, double *__restrict__ grad, int count) {
+k_gradient_poly(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
+                double *__restrict__ grad, int count) {
     constexpr int kTile = kBS * kItems;
     __shared__ double s_h[2][kTile + 2];
     __shared__ double s_dv[kTile + 1];
-    __shared__ double s_sl[kArc ? kTile + 1 : 1];
+    __shared__ double s_sl[kTile + 1];
     const int n = g.n;
     const int per_line = (n + kTile - 1) / kTile;
     const int t = threadIdx.x;
@@ -141,12 +111,8 @@ k_gradient_poly(const double *__restrict__ h, PolyGeom g, double *__restrict__ g
         auto edge = [&](int e, int slot) {
             slot = QEW_IDX(slot, kTile + 1, g.nz.oob);
             const double he = sh[slot], hep = sh[slot + 1];
-            const double dv = poly_edge_dvdy(g, e, he, hep);
-            s_dv[slot] = kF0 ? scale_pow2(dv, g.half_dx_exp, g.half_dx) : dv;
-            if (kArc) {
-                const double dh = g.L.div(hep - he);
-                s_sl[slot] = dh * rsqrt(1.0 + dh * dh);
-            }
+            s_dv[slot] = e + 1 < n ? g.nz.dvdy_edge_store(e, hep + he) : walk_edge_rare(g, e, hep + he);
+            s_sl[slot] = fx_slope((hep - he) * g.L.inv_dx);
         };
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
@@ -160,16 +126,9 @@ k_gradient_poly(const double *__restrict__ h, PolyGeom g, double *__restrict__ g
         for (int k = 0; k < kItems; ++k) {
             const int j = QEW_IDX(t + k * kBS, kTile, g.nz.oob);
             if (t + k * kBS >= cnt) break;
-            const double rest = kF0 ? s_dv[j] + s_dv[j + 1]
-                                    : fma(g.half_dx, s_dv[j] + s_dv[j + 1], -g.fdx);
-            double gr;
-            if (kArc) {
-                gr = fma(g.lt, s_sl[j] - s_sl[j + 1], rest);
-            } else {
-                const double d2h = fma(-2.0, sh[j + 1], sh[j] + sh[j + 2]);
-                gr = fma(g.c_el, d2h, rest);
-            }
-            __stcs(out + j, gr);
+            __stcs(out + j, site_gradient<NoiseBSpline64>(
+                                sh[j], sh[j + 1], sh[j + 2], s_dv[j], s_dv[j + 1], s_sl[j],
+                                s_sl[j + 1], g.L, g.lt, 0.0, true));
         }
         line = nline;
         idx = nidx;
@@ -177,127 +136,258 @@ k_gradient_poly(const double *__restrict__ h, PolyGeom g, double *__restrict__ g
     asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
-// {q0, q1, q2, v0} of every (row cell j, column e) from the FP64
-// coefficients c ([ny][nx]); see qew_poly.cuh for the formulas. Each thread
-// walks kStoreRows row cells of one column and filters each coefficient row
-// along x once: cell j takes the filtered values of rows j-1..j+2 from a
-// window of four, so a cell costs one x-filter (4 FP64 instructions) and the
-// combination (11) instead of four x-filters. FP64-instruction bound.
+// ------------------------------------------------------------ integer walk
+// The linear gradient with the heights themselves as integers. A warp takes
+// chunks of 255 consecutive sites, the 256 edges about them in 8 steps of 32;
+// the chunk's 257 heights become signed integers in the unit 2^-8 of the ulp
+// of the largest one: exactly, but for bits of heights more than 2^8
+// below it, cut at 2^-8 of the ulp that FP64 sums beside the largest round
+// at. The midpoint sum, its row cell (folded into the field's period) and
+// fraction, dV/dy and the second difference of the heights are then integer
+// sums and products, and a site takes two FP64 instructions (the combine)
+// for seven before:
+//   grad = c_el d2h + (half_unit (R_l + R_r) - dx f).
+// A chunk with a non-finite height, or heights too small or too large beside
+// the row spacing, takes the FP64 sums of k_gradient_poly. Chunks start at
+// multiples of 255 of their line, whatever the launch, so every launch shape
+// and batch gives the same bits.
+constexpr int kWalkSteps = 8;
+constexpr int kWalkEdges = 32 * kWalkSteps;
+constexpr int kWalkSites = kWalkEdges - 1;
+constexpr int kWalkGuard = 8;
+
+// R = dV/dy of edge e < n - 1 in the store's unit from the integer sum a of
+// its heights, whose midpoint in row cells is a 2^-sh, |a 2^-sh| < 2^22.
+// kPow2: a power-of-two row spacing; else a is first multiplied by the
+// spacing's reciprocal mantissa (62 bits).
+template <bool kPow2>
+__device__ __forceinline__ long long walk_edge(const PolyGeom &g, int e, long long a, int sh) {
+    if (!kPow2) a = fx_mul(a, g.recip);
+    int c = (int)(a >> sh);  // floor
+    const FxFrac t = fx_frac((unsigned long long)a << (64 - sh));
+    if ((unsigned)c >= (unsigned)g.nz.ny) {  // fold into the period: the quotient is off by 1 at most
+        c -= __float2int_rd((float)c * g.inv_ny) * g.nz.ny;
+        if (c < 0) c += g.nz.ny;
+        if (c >= g.nz.ny) c -= g.nz.ny;
+    }
+    c = QEW_IDX(c, g.nz.ny, g.nz.oob);
+    e = QEW_IDX(e, g.nz.nx, g.nz.oob);
+    return fx_dt2(fx_load_cell(g.nz.poly + ((size_t)c * (size_t)g.nz.nx + (size_t)e) * 4), t);
+}
+
+// v of the next lane; the last lane gets `wrap` of the first one.
+__device__ __forceinline__ long long lane_next(long long v, long long wrap, int lane) {
+    return __shfl_sync(0xffffffffu, lane == 0 ? wrap : v, (lane + 1) & 31);
+}
+
+// Gradient of site i from FP64 sums and edges.
+__device__ __noinline__ void walk_site_rare(const PolyGeom &g, const double *hl, double *out, int i) {
+    const int n = g.n;
+    const int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
+    const double hm = __ldg(hl + im), h0 = __ldg(hl + i), hp = __ldg(hl + ip);
+    const double dvl = walk_edge_rare(g, im, hm + h0), dvr = walk_edge_rare(g, i, h0 + hp);
+    __stcs(out + i, site_gradient<NoiseBSpline64>(hm, h0, hp, dvl, dvr, 0.0, 0.0, g.L, g.lt, 0.0,
+                                                  false));
+}
+
+template <int kMin, bool kPow2>
+__global__ void __launch_bounds__(kBS, kMin)
+k_gradient_poly_walk(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
+                     double *__restrict__ grad, int chunks, long long units) {
+    const int n = g.n;
+    const int lane = threadIdx.x & 31;
+    const long long u = (long long)blockIdx.x * (kBS / 32) + (threadIdx.x >> 5);
+    if (u >= units) return;
+    const int line = (int)(u / chunks);
+    const int s0 = (int)(u - (long long)line * chunks) * kWalkSites;
+    const double *hl = h + (size_t)line * (size_t)n;
+    double *out = grad + (size_t)line * (size_t)n;
+    // step k's edges are s0 - 1 + 32 k + lane, each with the site at its
+    // right end; the two sites of the wrap edge are done apart
+    if (s0 == 0 && lane == 0) walk_site_rare(g, hl, out, 0);
+    if (s0 + kWalkSites >= n && lane == 1) walk_site_rare(g, hl, out, n - 1);
+    double x[kWalkSteps];
+#pragma unroll
+    for (int k = 0; k < kWalkSteps; ++k) {
+        const int i = s0 - 1 + 32 * k + lane;
+        x[k] = __ldg(hl + (i < 0 ? n - 1 : i < n ? i : 0));
+    }
+    const int il = s0 - 1 + kWalkEdges;
+    const double last = __ldg(hl + (il < n ? il : 0));  // right end of the last edge
+    // the largest exponent of the chunk
+    unsigned mx = (unsigned)__double2hiint(last) << 1;
+#pragma unroll
+    for (int k = 0; k < kWalkSteps; ++k) mx = max(mx, (unsigned)__double2hiint(x[k]) << 1);
+    mx = __reduce_max_sync(0xffffffffu, mx) >> 21;
+    // midpoint in cells = a 2^-sh for a in units of 2^(mx - 1075 - guard)
+    const int sh = 1075 + kWalkGuard - (int)mx - g.ky;
+    if (!(mx < 2047u && mx > 200u && sh >= 40 && sh <= 63)) {
+        for (int j = lane; j < kWalkSites; j += 32)
+            if (s0 + j > 0 && s0 + j + 1 < n) walk_site_rare(g, hl, out, s0 + j);
+        return;
+    }
+    auto fix = [&](double v) {
+        const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+        const unsigned m = (hi & 0x000FFFFFu) | 0x00100000u;
+        const unsigned long long w =
+            ((unsigned long long)__funnelshift_l(lo, m, kWalkGuard) << 32) |
+            (unsigned long long)(lo << kWalkGuard);
+        const long long sg = (long long)((int)hi >> 31);
+        return ((long long)fx_shr(w, (int)(mx - ((hi >> 20) & 0x7FFu))) ^ sg) - sg;
+    };
+    const int ek = (int)mx - 1075 - kWalkGuard;
+    long long H = fix(x[0]), Rb = 0, sb = 0;  // Rb, sb: edge and slope of the step before
+#pragma unroll
+    for (int k = 0; k <= kWalkSteps; ++k) {
+        long long R = 0, sl = 0;
+        if (k < kWalkSteps) {
+            const long long Hn = fix(k + 1 < kWalkSteps ? x[k + 1 < kWalkSteps ? k + 1 : 0] : last);
+            const long long Hp = lane_next(H, Hn, lane);
+            const int e = s0 - 1 + 32 * k + lane;
+            R = walk_edge<kPow2>(g, e >= 0 && e + 1 < n ? e : 0, H + Hp, sh);
+            sl = Hp - H;
+            H = Hn;
+        }
+        if (k > 0) {  // the sites of the step before
+            const int i = s0 + 32 * (k - 1) + lane;
+            const long long S = Rb + lane_next(Rb, R, lane);
+            const long long D = lane_next(sb, sl, lane) - sb;
+            if (i > 0 && i + 1 < n && (k < kWalkSteps || lane < 31))
+                __stcs(out + i, fma(g.L.c_el, fx_to_double(D, ek),
+                                    fma(g.half_unit, fx_to_double(S), -g.L.fdx)));
+        }
+        Rb = R;
+        sb = sl;
+    }
+}
+
+// FxCubic of every (row cell j, column e) from the FP64 coefficients c
+// ([ny][nx]). Each thread walks kStoreRows row cells of one column and
+// filters each coefficient row along x once: cell j takes the filtered values
+// of rows j-1..j+2 from a window of four. Integer arithmetic, about 120
+// cycles of a warp a cell; bound by its writes (32 bytes a cell).
 constexpr int kStoreRows = 32;
 constexpr int kStoreBS = 256;
 
-__device__ __forceinline__ double x_filter(const double *__restrict__ r, int em, int e, int ep,
-                                           int ep2) {
-    const double w0 = 1.0 / 48.0, w1 = 23.0 / 48.0;
-    return __fma_rn(w0, __ldg(r + ep2),
-                    __fma_rn(w1, __ldg(r + ep), __fma_rn(w1, __ldg(r + e), w0 * __ldg(r + em))));
-}
-
 __global__ void __launch_bounds__(kStoreBS) k_poly_store(const double *__restrict__ c, int nx,
-                                                         int ny, double inv_dy,
-                                                         double *__restrict__ out) {
+                                                         int ny,
+                                                         const unsigned long long *max_bits,
+                                                         long long *__restrict__ out) {
     const int e = blockIdx.x * kStoreBS + threadIdx.x;
     if (e >= nx) return;
+    const unsigned long long mb = *max_bits;
+    const int kb = mb == 0 ? 1023 : (int)(mb >> 52);
     const int j0 = blockIdx.y * kStoreRows;
     const int j1 = min(ny, j0 + kStoreRows);
-    const int em = (e == 0) ? nx - 1 : e - 1;
-    const int ep = (e + 1 == nx) ? 0 : e + 1;
-    const int ep2 = (ep + 1 == nx) ? 0 : ep + 1;
-    const double half_inv_dy = 0.5 * inv_dy, s6 = 1.0 / 6.0;
+    int xs[4];
+    wrap4(e, nx, xs);
     int r = (j0 == 0) ? ny - 1 : j0 - 1;  // row j0-1, periodic
-    double E0 = x_filter(c + (size_t)r * nx, em, e, ep, ep2);
-    r = (r + 1 == ny) ? 0 : r + 1;
-    double E1 = x_filter(c + (size_t)r * nx, em, e, ep, ep2);
-    r = (r + 1 == ny) ? 0 : r + 1;
-    double E2 = x_filter(c + (size_t)r * nx, em, e, ep, ep2);
+    auto next_row = [&]() {
+        const double *row = c + (size_t)r * nx;
+        r = (r + 1 == ny) ? 0 : r + 1;
+        return ((fx_tap<4>(__ldg(row + xs[0]), kb) + fx_tap<4>(__ldg(row + xs[3]), kb)) +
+                23 * (fx_tap<4>(__ldg(row + xs[1]), kb) + fx_tap<4>(__ldg(row + xs[2]), kb))) >>
+               5;
+    };
+    long long E[4];
+    E[0] = next_row();
+    E[1] = next_row();
+    E[2] = next_row();
     for (int j = j0; j < j1; ++j) {
-        r = (r + 1 == ny) ? 0 : r + 1;  // row j+2
-        const double E3 = x_filter(c + (size_t)r * nx, em, e, ep, ep2);
-        const double s02 = E0 + E2;
-        const double q0 = (E2 - E0) * half_inv_dy;
-        const double q1 = __fma_rn(-2.0, E1, s02) * inv_dy;
-        const double q2 = __fma_rn(3.0, E1 - E2, E3 - E0) * half_inv_dy;
-        const double v0 = __fma_rn(4.0, E1, s02) * s6;
-        double *o = out + ((size_t)j * (size_t)nx + (size_t)e) * 4;  // 32-byte aligned
-        asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(o), "d"(q0), "d"(q1),
-                     "d"(q2), "d"(v0)
+        E[3] = next_row();
+        const FxCubic q = fx_cubic(E);
+        long long *o = out + ((size_t)j * (size_t)nx + (size_t)e) * 4;  // 32-byte aligned
+        asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(o), "l"(q.v), "l"(q.p),
+                     "l"(q.u2), "l"(q.w)
                      : "memory");
-        E0 = E1;
-        E1 = E2;
-        E2 = E3;
+        E[0] = E[1];
+        E[1] = E[2];
+        E[2] = E[3];
     }
 }
 
 }  // namespace
 
-bool qew_poly_applies(const qew_field *f, int n, const qew_params *p) {
-    return f && f->kind == QEW_FIELD_BSPLINE && f->poly64 && f->coef64 && n == f->nx &&
-           p->physical_size == f->Lx;
-}
-
-qew_status qew_poly_store_build(qew_ctx *ctx, const double *c, int nx, int ny, double dy,
-                                double *out) {
+qew_status qew_poly_store_build(qew_ctx *ctx, const double *c, int nx, int ny,
+                                const unsigned long long *max_bits, long long *out) {
     if ((ny + kStoreRows - 1) / kStoreRows > 65535)
         return qew_fail(ctx, QEW_ERR_INVALID, "poly store: more than 2^21 field rows");
     const dim3 grid((unsigned)((nx + kStoreBS - 1) / kStoreBS),
                     (unsigned)((ny + kStoreRows - 1) / kStoreRows));
-    k_poly_store<<<grid, kStoreBS, 0, ctx->stream>>>(c, nx, ny, 1.0 / dy, out);
+    k_poly_store<<<grid, kStoreBS, 0, ctx->stream>>>(c, nx, ny, max_bits, out);
     return qew_launch_check(ctx, "poly_store");
 }
 
 qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count,
                                      const double *d_h, int n, const qew_params *p,
                                      double *d_grad) {
-    if (!qew_poly_applies(f, n, p)) return QEW_ERR_UNSUPPORTED;
+    if (!f || f->kind != QEW_FIELD_BSPLINE || !f->coef64) return QEW_ERR_UNSUPPORTED;
     PolyGeom g{};
-    g.poly = f->poly64;
     g.nz = make_bspline64(f, n, p->physical_size);
+    if (!g.nz.poly || g.nz.kb < 0) return QEW_ERR_UNSUPPORTED;
     g.n = n;
-    g.ky = poly_scale_exponent(f->dy);
-    g.half_inv_dy = 0.5 / f->dy;
+    const bool pow2 = qew_is_pow2(f->dy);
+    {
+        // 1 / (2 dy) = m 2^ky; the double's error as a second term
+        const double d = 2.0 * f->dy, q = 1.0 / d;
+        int e;
+        const double m = frexp(q, &e);
+        const long long M = llrint(ldexp(m, 62)) + llrint(ldexp(q * fma(-q, d, 1.0), 62 - e));
+        g.ky = pow2 ? e - 1 : e;
+        g.recip = fx_limbs(std::min(M, (1ll << 62) - 1));
+    }
     g.L = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
-    g.c_el = g.L.c_el;
     g.lt = p->line_tension;
-    g.half_dx = g.L.half_dx;
-    g.fdx = g.L.fdx;
-    int hx;
-    const bool f0 = p->driving_force == 0.0 && frexp(g.half_dx, &hx) == 0.5;
-    g.half_dx_exp = hx - 1;  // half_dx == 2^(hx-1) when f0
+    g.half_unit = g.L.half_dx * g.nz.fx_dv_c;
+    g.inv_ny = 1.0f / (float)f->ny;
     const bool arc = (p->model == QEW_MODEL_ARCLENGTH);
-    // Candidates: sites per thread {1, 2, 4} x resident CTAs per SM {2, 3, 4};
-    // every one computes the same numbers (the per-site arithmetic does not
-    // depend on the tiling). Hand-chosen default: 2 sites, 4 CTAs.
-    static const char *const names[9] = {"1 site x 2 CTA/SM", "1 site x 3 CTA/SM",
-                                          "1 site x 4 CTA/SM", "2 sites x 2 CTA/SM",
-                                          "2 sites x 3 CTA/SM", "2 sites x 4 CTA/SM",
-                                          "4 sites x 2 CTA/SM", "4 sites x 3 CTA/SM",
-                                          "4 sites x 4 CTA/SM"};
+    const bool walk = !arc && std::isfinite(g.half_unit);
+    // Candidates; every one computes the same numbers (the per-site
+    // arithmetic does not depend on the launch): sites per thread {1, 2, 4} x
+    // resident CTAs per SM {2, 3, 4}, default 2 sites, 4 CTAs; for the walk
+    // (a chunk per warp) registers for {4, 5, 6} resident CTAs per SM, default
+    // 5: 86.3, 84.8 and 87.5 us on 8 lines of 2^20 points.
+    static const char *const tile_names[9] = {"1 site x 2 CTA/SM", "1 site x 3 CTA/SM",
+                                              "1 site x 4 CTA/SM", "2 sites x 2 CTA/SM",
+                                              "2 sites x 3 CTA/SM", "2 sites x 4 CTA/SM",
+                                              "4 sites x 2 CTA/SM", "4 sites x 3 CTA/SM",
+                                              "4 sites x 4 CTA/SM"};
+    static const char *const walk_names[3] = {"walk, 4 CTA/SM", "walk, 5 CTA/SM", "walk, 6 CTA/SM"};
     auto launch = [&](int c) -> qew_status {
         const int items = 1 << (c / 3);
         const int ctas = 2 + c % 3;
+        if (walk) {
+            const int chunks = (n + kWalkSites - 1) / kWalkSites;
+            const long long units = (long long)chunks * count;
+            const long long blocks = (units + kBS / 32 - 1) / (kBS / 32);
+            if (blocks > INT_MAX)
+                return qew_fail(ctx, QEW_ERR_INVALID, "gradient: more than 2^31 tiles");
+#define QEW_WALK_LAUNCH(M) \
+    (pow2 ? k_gradient_poly_walk<M, true><<<(unsigned)blocks, kBS, 0, ctx->stream>>>(              \
+                d_h, g, d_grad, chunks, units)                                                     \
+          : k_gradient_poly_walk<M, false><<<(unsigned)blocks, kBS, 0, ctx->stream>>>(             \
+                d_h, g, d_grad, chunks, units))
+            if (c == 0) QEW_WALK_LAUNCH(4);
+            else if (c == 1) QEW_WALK_LAUNCH(5);
+            else QEW_WALK_LAUNCH(6);
+#undef QEW_WALK_LAUNCH
+            return qew_launch_check(ctx, "gradient_poly");
+        }
         const long long tiles = (long long)((n + kBS * items - 1) / (kBS * items)) * count;
         if (tiles > INT_MAX)
             return qew_fail(ctx, QEW_ERR_INVALID, "gradient: more than 2^31 tiles");
         const int grid = (int)std::min<long long>(tiles, (long long)ctas * ctx->num_sms);
-#define QEW_POLY_LAUNCH(A, I, F) \
-    k_gradient_poly<A, I, F><<<grid, kBS, 0, ctx->stream>>>(d_h, g, d_grad, count)
-#define QEW_POLY_ITEMS(A, F)                       \
-    if (items == 1) QEW_POLY_LAUNCH(A, 1, F);      \
-    else if (items == 2) QEW_POLY_LAUNCH(A, 2, F); \
-    else QEW_POLY_LAUNCH(A, 4, F)
-        if (arc) {
-            if (f0) { QEW_POLY_ITEMS(true, true); } else { QEW_POLY_ITEMS(true, false); }
-        } else {
-            if (f0) { QEW_POLY_ITEMS(false, true); } else { QEW_POLY_ITEMS(false, false); }
-        }
-#undef QEW_POLY_ITEMS
+#define QEW_POLY_LAUNCH(I) \
+    k_gradient_poly<I><<<grid, kBS, 0, ctx->stream>>>(d_h, g, d_grad, count)
+        if (items == 1) QEW_POLY_LAUNCH(1);
+        else if (items == 2) QEW_POLY_LAUNCH(2);
+        else QEW_POLY_LAUNCH(4);
 #undef QEW_POLY_LAUNCH
         return qew_launch_check(ctx, "gradient_poly");
     };
-    int cand = 5;
+    int cand = walk ? 1 : 5;
     QEW_TRY(qew_tune_pick(ctx, kTuneGradientPoly,
-                          qew_tune_class((long long)n * count, (arc ? 1 : 0) + (f0 ? 2 : 0)), 9,
-                          5, names, launch,
-                          &cand));
+                          qew_tune_class((long long)n * count, (arc ? 1 : 0) + (walk ? 2 : 0) + (pow2 ? 4 : 0)),
+                          walk ? 3 : 9, cand, walk ? walk_names : tile_names, launch, &cand));
     return launch(cand);
 }
