@@ -103,6 +103,7 @@ k_langevin_run(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, dou
     const bool arc = (model == QEW_MODEL_ARCLENGTH);
     const int t = threadIdx.x;
     double *cur = h, *nxt = tmp;
+    unsigned int arrivals = 0;
     for (int k = 0; k < steps; ++k) {
         const double a = drift[k], b = diff[k];
         const uint64_t rs = rstep[k];
@@ -140,7 +141,7 @@ k_langevin_run(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, dou
             }
             __syncthreads();
         }
-        if (!grid_sync_bounded(sync, gridDim.x)) return;
+        if (!grid_sync_bounded(sync, gridDim.x, arrivals)) return;
         double *sw = cur;
         cur = nxt;
         nxt = sw;
@@ -183,6 +184,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
     const int s0 = blockIdx.x * seg;
     const int S = max(0, min(seg, n - s0));
     double *cur = h, *nxt = tmp;
+    unsigned int arrivals = 0;
     for (int k0 = 0; k0 < steps; k0 += K) {
         const int Kr = min(K, steps - k0);
         if (S > 0) {
@@ -231,7 +233,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
             }
             for (int r = Kr + t; r < Kr + S; r += kRunBS) nxt[s0 + r - Kr] = hA[r];
         }
-        if (!grid_sync_bounded(sync, gridDim.x)) return;
+        if (!grid_sync_bounded(sync, gridDim.x, arrivals)) return;
         double *sw = cur;
         cur = nxt;
         nxt = sw;

@@ -17,16 +17,10 @@ namespace {
 
 constexpr int kBS = 256;
 
-// The plain form and the site velocities keep the 16-tap sum on a field that
-// holds the cell-polynomial store.
-template <class Noise>
-void drop_poly(Noise &) {}
-void drop_poly(NoiseBSpline64 &nz) { nz.poly = nullptr; }
-
 // One colour of one sweep (rosso_krauth.h:154-165): thread k owns site 2k+color.
 template <class Noise>
 __global__ void k_rk_colour(Noise nz, double *__restrict__ h, double *__restrict__ adv, int n,
-                            double dx, double lt, double f, int model, int color, RkP rp) {
+                            LineDx dx, double lt, double f, int model, int color, RkP rp) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = 2 * k + color;
     if (i >= n) return;
@@ -40,7 +34,7 @@ __global__ void k_rk_colour(Noise nz, double *__restrict__ h, double *__restrict
 }
 
 template <class Noise>
-__global__ void k_rk_velocity(Noise nz, const double *__restrict__ h, int n, double dx, double lt,
+__global__ void k_rk_velocity(Noise nz, const double *__restrict__ h, int n, LineDx dx, double lt,
                               double f, int model, double *__restrict__ vel) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -68,7 +62,7 @@ qew_status qew_rk_validate(qew_ctx *ctx, int n, const qew_params *p, const qew_r
 qew_status qew_rk_block_plain(qew_ctx *ctx, const qew_field *field, double *d_h, int n,
                               const qew_params *p, const qew_rk_params *rp, qew_rk_result *res,
                               int precision) {
-    const double dx = p->physical_size / (double)n;
+    const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     QEW_TRY(qew_scratch_reserve(ctx, sizeof(double) * (size_t)n));
     double *adv = (double *)ctx->scratch;
     QEW_CUDA(ctx, cudaMemsetAsync(adv, 0, sizeof(double) * (size_t)n, ctx->stream));
@@ -82,7 +76,6 @@ qew_status qew_rk_block_plain(qew_ctx *ctx, const qew_field *field, double *d_h,
     for (int sweep = 0; sweep < rp->max_sweeps; ++sweep) {
         for (int color = 0; color < 2; ++color) {
             auto colour = [&](auto nz) -> qew_status {
-                drop_poly(nz);
                 k_rk_colour<<<(half + kBS - 1) / kBS, kBS, 0, ctx->stream>>>(
                     nz, d_h, adv, n, dx, p->line_tension, p->driving_force, p->model, color, rk);
                 return qew_launch_check(ctx, "rk_colour");
@@ -120,9 +113,8 @@ qew_status qew_rk_site_velocity(qew_ctx *ctx, const qew_field *field, const doub
     QEW_RANGE();
     if (!ctx || !field || !d_h || !p || !d_vel || n < 1)
         return qew_fail(ctx, QEW_ERR_INVALID, "rk_site_velocity: bad arguments");
-    const double dx = p->physical_size / (double)n;
+    const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     return qew_dispatch_noise(ctx, field, [&](auto nz) -> qew_status {
-        drop_poly(nz);
         k_rk_velocity<<<(n + kBS - 1) / kBS, kBS, 0, ctx->stream>>>(
             nz, d_h, n, dx, p->line_tension, p->driving_force, p->model, d_vel);
         return qew_launch_check(ctx, "rk_velocity");

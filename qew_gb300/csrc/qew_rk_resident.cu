@@ -3,9 +3,9 @@
 // on the device, with a grid barrier between colours instead of a kernel
 // launch, and the sweep's total advance reduced deterministically (per-CTA
 // partials summed in CTA order by every CTA). Each site's forward zero is
-// evaluated by a group of lanes (rk_forward_zero_group: several march points
-// or bisection levels per round) that replays the serial search exactly, so
-// both forms produce bit-identical lines.
+// evaluated by a group of lanes (rk_forward_zero_fast, or several march points
+// or bisection levels per round in rk_forward_zero_group) with the serial
+// search's result exactly, so both forms produce bit-identical lines.
 //
 // The grid barrier spins on a generation word with a bounded number of polls;
 // if it gives up it raises an error flag, every CTA leaves the sweep loop, and
@@ -28,16 +28,28 @@ constexpr int kRkBS = 32;  // one warp per CTA: a 16384-site line still spreads 
 #ifndef QEW_RK_WARPS_PER_SM
 #define QEW_RK_WARPS_PER_SM 4  // build-time tuning knob (measured on GB300)
 #endif
-// kRkGroup lanes per site (8: 7 march points or 3 bisection levels per round;
-// 4: 3 points or 2 levels; 2: the serial search with each velocity's two
-// gathers on the two lanes; 1: the serial search). All widths give the same
-// result; the launch picks one by the budgets below.
+
+// Sum of part[0..nb), the same in every lane of the warp (kRkBS = 32): a
+// lane's strided terms, then a butterfly.
+__device__ __forceinline__ double warp_sum_partials(const double *part, unsigned nb) {
+    double v = 0.0;
+    for (unsigned b = threadIdx.x; b < nb; b += 32) v += __ldcg(part + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// kRkGroup lanes per site (8 or 2: the fast search of qew_rk_device.cuh where
+// it applies, else 7 march points or 3 bisection levels per round on 8 lanes,
+// the serial search with each velocity's two gathers on the two lanes; 1: the
+// serial search). All widths give the same result; the launch picks one by
+// the budgets below.
 template <class Noise, int kRkGroup>
 __global__ void __launch_bounds__(kRkBS)
-k_rk_resident(Noise nz, double *__restrict__ h, double *__restrict__ adv, int n, double dx,
-              double lt, double f, int model, RkP rp, double *partials, GridSync *sync,
-              qew_rk_result *out) {
+k_rk_resident(Noise nz, double *__restrict__ h, int n, LineDx dx, double lt, double f, int model,
+              RkP rp, double *partials, GridSync *sync, qew_rk_result *out) {
     const unsigned int nb = gridDim.x;
+    unsigned int arrivals = 0;
     const int gtid = blockIdx.x * kRkBS + threadIdx.x;
     const int gstride = nb * kRkBS;
     const int half = n / 2;
@@ -50,10 +62,8 @@ k_rk_resident(Noise nz, double *__restrict__ h, double *__restrict__ adv, int n,
     for (int i = gtid; i < n; i += gstride) acc += h[i];
     acc = block_sum<kRkBS>(acc, s_w);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc;
-    if (!grid_sync_bounded(sync, nb)) return;
-    double mean_h0 = 0.0;
-    for (unsigned int b = 0; b < nb; ++b) mean_h0 += __ldcg(partials + b);
-    mean_h0 /= (double)n;
+    if (!grid_sync_bounded(sync, nb, arrivals)) return;
+    const double mean_h0 = warp_sum_partials(partials, nb) / (double)n;
 
     qew_rk_result res{};
     double cum_adv = 0.0;
@@ -66,37 +76,36 @@ k_rk_resident(Noise nz, double *__restrict__ h, double *__restrict__ adv, int n,
                 const int im = (i == 0) ? n - 1 : i - 1;
                 const int ip = (i + 1 == n) ? 0 : i + 1;
                 bool found = false;
-                const double hi = __ldcg(h + i);
+                const double hi = __ldcg(h + i), hl = __ldcg(h + im), hr = __ldcg(h + ip);
                 double hnew;
-                if constexpr (kRkGroup == 1) {
-                    hnew = rk_forward_zero(nz, i, n, dx, lt, f, model, hi, __ldcg(h + im),
-                                           __ldcg(h + ip), rp, found);
-                } else if constexpr (kRkGroup == 2) {
-                    hnew = rk_forward_zero_pair(nz, i, n, dx, lt, f, model, hi, __ldcg(h + im),
-                                                __ldcg(h + ip), rp, found, glane, gmask);
-                    __syncwarp(gmask);  // both lanes have read h[i]
-                } else {
-                    hnew = rk_forward_zero_group<kRkGroup>(nz, i, n, dx, lt, f, model, hi,
-                                                          __ldcg(h + im), __ldcg(h + ip), rp,
-                                                          found, glane, gmask);
-                    __syncwarp(gmask);  // every lane has read h[i]
+                bool done = false;
+                if constexpr (std::is_same<Noise, NoiseBSpline64>::value && kRkGroup > 1)
+                    done = rk_forward_zero_fast<kRkGroup>(nz, i, n, dx, model, hi, hl, hr, rp,
+                                                          found, hnew, glane, gmask);
+                if (!done) {
+                    if constexpr (kRkGroup == 1)
+                        hnew = rk_forward_zero(nz, i, n, dx, lt, f, model, hi, hl, hr, rp, found);
+                    else if constexpr (kRkGroup == 2)
+                        hnew = rk_forward_zero_pair(nz, i, n, dx, lt, f, model, hi, hl, hr, rp,
+                                                    found, glane, gmask);
+                    else
+                        hnew = rk_forward_zero_group<kRkGroup>(nz, i, n, dx, lt, f, model, hi, hl,
+                                                               hr, rp, found, glane, gmask);
                 }
+                if constexpr (kRkGroup > 1) __syncwarp(gmask);  // every lane has read h[i]
                 if (glane == 0) {
-                    const double a = hnew - hi;
-                    adv[i] = a;
                     h[i] = hnew;
-                    local += a;
+                    local += hnew - hi;
                 }
             }
-            if (color == 0 && !grid_sync_bounded(sync, nb)) return;
+            if (color == 0 && !grid_sync_bounded(sync, nb, arrivals)) return;
         }
         // sweep total: per-CTA partials (double-buffered by sweep parity)
         double *part = partials + nb * (1 + (sweep & 1));
         local = block_sum<kRkBS>(local, s_w);
         if (threadIdx.x == 0) part[blockIdx.x] = local;
-        if (!grid_sync_bounded(sync, nb)) return;
-        double total_adv = 0.0;
-        for (unsigned int b = 0; b < nb; ++b) total_adv += __ldcg(part + b);
+        if (!grid_sync_bounded(sync, nb, arrivals)) return;
+        const double total_adv = warp_sum_partials(part, nb);
         cum_adv += total_adv;
         const double mean_adv = cum_adv / (double)n;
         res.sweeps = sweep + 1;
@@ -121,7 +130,7 @@ k_rk_resident(Noise nz, double *__restrict__ h, double *__restrict__ adv, int n,
 qew_status qew_rk_block_resident(qew_ctx *ctx, const qew_field *field, double *d_h, int n,
                                  const qew_params *p, const qew_rk_params *rp, int precision,
                                  qew_rk_result *res) {
-    const double dx = p->physical_size / (double)n;
+    const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
     const RkP rk = rkp_from(rp);
     auto launch = [&](auto nz) -> qew_status {
         using N = decltype(nz);
@@ -131,13 +140,18 @@ qew_status qew_rk_block_resident(qew_ctx *ctx, const qew_field *field, double *d
         // two gathers (the same FP64 work in half the chain). Each form has a
         // warps-per-SM budget (and the resident slots, or the context's share
         // of them); the serial form takes what is left.
-        // Measured (sweeps/s, bitwise-equal results): 8-lane groups win while
-        // they stay within about 2 warps per SM, lane pairs up to about 4,
-        // the serial search beyond; 4-lane groups were never the best.
+        // Measured for 200 sweeps (bitwise-equal results): n = 2048 8-lane
+        // groups 5.8 ms, lane pairs 6.7, one lane 64; n = 4096 5.8 and 6.7;
+        // n = 16384 13.5 and 8.1: 8-lane groups while they stay within about
+        // 4 warps per SM, lane pairs up to 8, the serial search beyond.
         const void *forms[3] = {(const void *)k_rk_resident<N, 8>, (const void *)k_rk_resident<N, 2>,
                                 (const void *)k_rk_resident<N, 1>};
         const int sizes[3] = {8, 2, 1};
-        const long long warps_per_sm[3] = {QEW_RK_WARPS_PER_SM / 2, QEW_RK_WARPS_PER_SM, 0};
+        bool fast = false;  // else half of that (the generic searches do more FP64 work per lane)
+        if constexpr (std::is_same<N, NoiseBSpline64>::value)
+            fast = p->model == QEW_MODEL_LINEAR && nz.kb >= 0;
+        const long long unit = fast ? QEW_RK_WARPS_PER_SM : QEW_RK_WARPS_PER_SM / 2;
+        const long long warps_per_sm[3] = {unit, 2 * unit, 0};
         const long long half = n / 2;
         int grids[3];
         int heuristic = 2, grid_max = 1;
@@ -152,22 +166,20 @@ qew_status qew_rk_block_resident(qew_ctx *ctx, const qew_field *field, double *d
             grid_max = std::max(grid_max, grids[k]);
             if (heuristic == 2 && k < 2 && want <= budget) heuristic = k;
         }
-        // scratch: adv[n], partials[3*grid], sync word, result
-        const size_t off_part = ((size_t)n * sizeof(double) + 255) & ~size_t(255);
+        // scratch: partials[3*grid], sync word, result
+        const size_t off_part = 0;
         const size_t off_sync = (off_part + 3 * (size_t)grid_max * sizeof(double) + 255) & ~size_t(255);
         const size_t off_res = (off_sync + sizeof(GridSync) + 255) & ~size_t(255);
         QEW_TRY(qew_scratch_reserve(ctx, off_res + sizeof(qew_rk_result) + 256));
         char *base = (char *)ctx->scratch;
-        double *adv = (double *)base;
         double *part = (double *)(base + off_part);
         GridSync *sync = (GridSync *)(base + off_sync);
         qew_rk_result *d_res = (qew_rk_result *)(base + off_res);
         double lt = p->line_tension, fd = p->driving_force;
         int model = p->model;
         auto run_form = [&](int k, double *hp, RkP rkk) -> qew_status {
-            QEW_CUDA(ctx, cudaMemsetAsync(adv, 0, (size_t)n * sizeof(double), ctx->stream));
             QEW_TRY(qew_gridsync_init(ctx, sync));
-            void *args[] = {(void *)&nz, (void *)&hp, (void *)&adv, (void *)&n, (void *)&dx,
+            void *args[] = {(void *)&nz, (void *)&hp, (void *)&n, (void *)&dx,
                             (void *)&lt, (void *)&fd, (void *)&model, (void *)&rkk,
                             (void *)&part, (void *)&sync, (void *)&d_res};
             QEW_CUDA(ctx, cudaLaunchCooperativeKernel(forms[k], dim3(grids[k]), dim3(kRkBS), args,
