@@ -27,43 +27,29 @@ constexpr int kEnsBS = 512;
 
 struct EnsJob {
     NoiseBSpline64 nz64;
-#ifdef QEW_BOUNDS_CHECK
-    unsigned long long *oob;
-#endif
-    const float *coef32;
-    const float *edge32;
-    int nx, ny;
-    double fdx, fdy, Lx;
+    NoiseSplit32 nz32;  // coef32 null: no FP32 phase
     double *h;
     int n;
     qew_params p;
     PrecondCoef pc;
 };
 
-__device__ __forceinline__ NoiseSplit32 job_noise32(const EnsJob &j) {
-    NoiseSplit32 nz;
-    nz.coef = j.coef32;
-    nz.nx = j.nx;
-    nz.ny = j.ny;
-    nz.dx = j.fdx;
-    nz.dy = j.fdy;
-    nz.inv_dx = 1.0 / j.fdx;
-    nz.inv_dy = 1.0 / j.fdy;
-    nz.dx_pow2 = dbl_is_pow2(j.fdx);
-    nz.dy_pow2 = dbl_is_pow2(j.fdy);
-    nz.xconst = (j.n == j.nx && j.p.physical_size == j.Lx && nz.dx_pow2);
-    nz.edge = nz.xconst ? j.edge32 : nullptr;
-    nz.inv_dy_f = (float)(1.0 / j.fdy);
-#ifdef QEW_BOUNDS_CHECK
-    nz.oob = j.oob;
-#endif
-    return nz;
+EnsJob make_job(const qew_field *f, double *h, int n, const qew_params &p, int precondition,
+                double shift) {
+    EnsJob j{};
+    j.nz64 = make_bspline64(f, n, p.physical_size);
+    j.nz32 = make_split32(f, n, p.physical_size);
+    j.h = h;
+    j.n = n;
+    j.p = p;
+    if (precondition) j.pc = qew_precond_coef(n, p.line_tension, p.physical_size, shift);
+    return j;
 }
 
 __global__ void __launch_bounds__(kEnsBS, 2)
 k_ensemble(const EnsJob *__restrict__ jobs, const int *__restrict__ order, int count,
            unsigned int *next, LbfgsCfg cfg32, LbfgsCfg cfg64, int use32, double *ws_base,
-           size_t ws_per_cta, size_t npad_max, qew_lbfgs_result *results) {
+           size_t ws_per_cta, qew_lbfgs_result *results) {
     __shared__ int s_job;
     double *ws = ws_base + (size_t)blockIdx.x * ws_per_cta;
     for (;;) {  // bounded: every pass takes a new queue ticket
@@ -75,9 +61,8 @@ k_ensemble(const EnsJob *__restrict__ jobs, const int *__restrict__ order, int c
         const int id = order[k];
         const EnsJob j = jobs[id];
         const size_t npad = ((size_t)j.n + 31) & ~size_t(31);
-        (void)npad_max;
         qew_lbfgs_result r32{};
-        if (use32) r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(job_noise32(j), j.h, j.n, j.p, cfg32, j.pc, ws, npad);
+        if (use32) r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(j.nz32, j.h, j.n, j.p, cfg32, j.pc, ws, npad);
         qew_lbfgs_result r = lbfgs_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws, npad);
         if (threadIdx.x == 0) {
             r.iterations += r32.iterations;
@@ -113,24 +98,7 @@ extern "C" qew_status qew_ensemble_minimize(qew_ctx *ctx, int count, const qew_e
             return qew_fail(ctx, QEW_ERR_INVALID,
                             "ensemble_minimize: line %d needs a B-spline field with FP64%s "
                             "coefficients", k, use32 ? " and FP32" : "");
-        EnsJob &j = jobs[k];
-        j.nz64 = make_bspline64(f, L.n, L.p.physical_size);
-#ifdef QEW_BOUNDS_CHECK
-        j.oob = qew_bounds_words();
-#endif
-        j.coef32 = f->coef32;
-        j.edge32 = f->edge32;
-        j.nx = f->nx;
-        j.ny = f->ny;
-        j.fdx = f->dx;
-        j.fdy = f->dy;
-        j.Lx = f->Lx;
-        j.h = L.d_h;
-        j.n = L.n;
-        j.p = L.p;
-        j.pc = lp.precondition ? qew_precond_coef(L.n, L.p.line_tension, L.p.physical_size,
-                                                  L.precond_shift)
-                               : PrecondCoef{};
+        jobs[k] = make_job(f, L.d_h, L.n, L.p, lp.precondition, L.precond_shift);
         nmax = std::max(nmax, L.n);
     }
     std::vector<int> order(count);
@@ -164,7 +132,7 @@ extern "C" qew_status qew_ensemble_minimize(qew_ctx *ctx, int count, const qew_e
     cfg32.ftol = ep->ftol_fp32;
     cfg32.max_iter = ep->max_iter_fp32 > 0 ? ep->max_iter_fp32 : lp.max_iter;
     k_ensemble<<<grid, kEnsBS, 0, ctx->stream>>>(d_jobs, d_order, count, d_cnt, cfg32, cfg64, use32,
-                                                  (double *)base, ws_per_cta, npad_max, d_res);
+                                                  (double *)base, ws_per_cta, d_res);
     QEW_TRY(qew_launch_check(ctx, "ensemble"));
     QEW_CUDA(ctx, cudaMemcpyAsync(results, d_res, sizeof(qew_lbfgs_result) * count,
                                   cudaMemcpyDeviceToHost, ctx->stream));
@@ -239,7 +207,7 @@ k_serve_static(LaneRing *ring, unsigned int *head, LbfgsCfg cfg32, LbfgsCfg cfg6
         const size_t npad = ((size_t)j.n + 31) & ~size_t(31);
         qew_lbfgs_result r32{};
         if (use32)
-            r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(job_noise32(j), j.h, j.n, j.p, cfg32,
+            r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(j.nz32, j.h, j.n, j.p, cfg32,
                                                            j.pc, ws, npad);
         qew_lbfgs_result r =
             lbfgs_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws, npad);
@@ -323,23 +291,7 @@ qew_status qew_lane_publish(StaticLane *L, const qew_field *f, double *d_h, int 
     if (!L || !f || !d_h || !p || n < 1 || n > L->nmax || f->kind != QEW_FIELD_BSPLINE ||
         !f->coef64 || (L->use32 && !f->coef32))
         return QEW_ERR_INVALID;
-    EnsJob j{};
-    j.nz64 = make_bspline64(f, n, p->physical_size);
-#ifdef QEW_BOUNDS_CHECK
-    j.oob = qew_bounds_words();
-#endif
-    j.coef32 = f->coef32;
-    j.edge32 = f->edge32;
-    j.nx = f->nx;
-    j.ny = f->ny;
-    j.fdx = f->dx;
-    j.fdy = f->dy;
-    j.Lx = f->Lx;
-    j.h = d_h;
-    j.n = n;
-    j.p = *p;
-    j.pc = L->cfg64.precondition ? qew_precond_coef(n, p->line_tension, p->physical_size, shift)
-                                 : PrecondCoef{};
+    const EnsJob j = make_job(f, d_h, n, *p, L->cfg64.precondition, shift);
     const unsigned int idx = L->published;
     L->ring->jobs[idx % kLaneRing] = j;
     __atomic_store_n(&L->ring->published, idx + 1u, __ATOMIC_RELEASE);

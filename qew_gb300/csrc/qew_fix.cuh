@@ -104,18 +104,18 @@ __device__ __forceinline__ double fx_to_double(long long r, int k = 0) {
 // FP64 code has to decide: non-finite or subnormal a, |g| >= 2^30, and the
 // last cell of a period other than the first two about zero, where the
 // reference's division by the period may round up.
-__device__ __forceinline__ bool fx_cell(double a, int k, int n, int &iy, FxFrac &t) {
+__device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &iy, unsigned long long &f) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(a);
     const int ef = (int)(b >> 52) & 0x7FF;
     const int e = ef + k - 1023;
     if (ef == 0 || ef == 2047 || e > 29) {
         iy = 0;
-        t = FxFrac{0, 0};
+        f = 0ull;
         return (b << 1) == 0ull;
     }
     const unsigned long long m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
     const int up = 12 + e;  // fraction bits to the top of 64 (the integer part leaves)
-    unsigned long long f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
+    f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
     iy = e >= 0 ? (int)fx_shr(m, 52 - e) : 0;
     bool ok = true;
     if ((long long)b < 0) {
@@ -140,8 +140,22 @@ __device__ __forceinline__ bool fx_cell(double a, int k, int n, int &iy, FxFrac 
         iy %= n;
         ok = iy + 1 < n;
     }
+    return ok;
+}
+__device__ __forceinline__ bool fx_cell(double a, int k, int n, int &iy, FxFrac &t) {
+    unsigned long long f;
+    const bool ok = fx_cell64(a, k, n, iy, f);
     t = fx_frac(f);
     return ok;
+}
+// f * 2^-64 as a float, rounded to nearest even (the conversion of the exact
+// FP64 fraction; one below 2^-64 is 0 here).
+__device__ __forceinline__ float fx_frac_to_float(unsigned long long f) {
+    const int lz = __clzll((long long)f);
+    const unsigned long long n = fx_shl(f, lz), rem = n << 24;
+    unsigned m = (unsigned)(n >> 40);
+    m += (rem > (1ull << 63) || (rem == (1ull << 63) && (m & 1u))) ? 1u : 0u;
+    return f ? __int_as_float(((126 - lz) << 23) + (int)(m - 0x800000u)) : 0.0f;
 }
 
 // The cubic along y in one cell, from the four stencil rows' sums E

@@ -162,15 +162,21 @@ k_langevin_run(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, dou
 // the results are bitwise those of k_langevin_run; the halo positions are
 // computed by both neighbouring CTAs. One grid barrier per round.
 //
+// A step is a chain of latencies (locate, gather, the integer products, the
+// combine), so a thread takes one edge and one site, and the first half of
+// the threads a pair of increments each (consecutive pairs, so that no lane
+// of their warps idles).
+//
 // Shared memory, in doubles of the region R = seg + 2K: heights (two
 // buffers), edge values, arclength slopes, increments.
 constexpr int kTbBufs = 5;
+constexpr int kTbBS = 256;
 // Dynamic shared memory a launch may take without raising the kernel's limit
 // (48 KB less room for the kernel's static shared memory).
 constexpr int kDefaultDynSmem = 47 * 1024;
 
 template <class Noise, bool NORMAL32>
-__global__ void __launch_bounds__(kRunBS)
+__global__ void __launch_bounds__(kTbBS)
 k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, double f,
                   int model, int steps, const double *__restrict__ drift,
                   const double *__restrict__ diff, const unsigned long long *__restrict__ rstep,
@@ -198,32 +204,46 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
                 return g;
             };
             const int RS = S + 2 * Kr;
-            for (int r = t; r < RS; r += kRunBS) hA[r] = __ldcg(cur + gsite(r));
+            for (int r = t; r < RS; r += kTbBS) hA[r] = __ldcg(cur + gsite(r));
             __syncthreads();
             for (int s = 1; s <= Kr; ++s) {
                 const int k = k0 + s - 1;
                 const double a = drift[k], b = diff[k];
                 const uint64_t rs = rstep[k];
                 const int lo = s, hi = RS - s;  // positions updated at this step
-                for (int r = lo - 1 + t; r < hi; r += kRunBS)
-                    edge_gradient(nz, gsite(r), n, hA[r], hA[r + 1], L, arc, dv[r], sl[r]);
                 if (b > 0) {
-                    for (int r = lo + t; r < hi; r += kRunBS) {
-                        const int g = gsite(r);
-                        if ((g & 1) && r != lo) continue;  // its pair's first site wrote it
-                        double z0, z1;
-                        if (NORMAL32)
-                            philox_normal_pair_f32(seed, rs, (uint32_t)(g >> 1), z0, z1);
-                        else
-                            philox_normal_pair(seed, rs, (uint32_t)(g >> 1), z0, z1);
-                        zz[r] = (g & 1) ? z1 : z0;
-                        if (!(g & 1) && r + 1 < hi && g + 1 < n) zz[r + 1] = z1;
+                    if ((n & 1) == 0) {  // pairs at every second position, across the ring's end too
+                        const int q0 = lo - ((g0 + lo) & 1);
+                        for (int r = q0 + 2 * t; r < hi; r += 2 * kTbBS) {
+                            const uint32_t pair = (uint32_t)(gsite(r) >> 1);
+                            double z0, z1;
+                            if (NORMAL32)
+                                philox_normal_pair_f32(seed, rs, pair, z0, z1);
+                            else
+                                philox_normal_pair(seed, rs, pair, z0, z1);
+                            zz[r] = z0;
+                            zz[r + 1] = z1;  // r + 1 <= hi <= RS - 1
+                        }
+                    } else {
+                        for (int r = lo + t; r < hi; r += kTbBS) {
+                            const int g = gsite(r);
+                            if ((g & 1) && r != lo) continue;  // its pair's first site wrote it
+                            double z0, z1;
+                            if (NORMAL32)
+                                philox_normal_pair_f32(seed, rs, (uint32_t)(g >> 1), z0, z1);
+                            else
+                                philox_normal_pair(seed, rs, (uint32_t)(g >> 1), z0, z1);
+                            zz[r] = (g & 1) ? z1 : z0;
+                            if (!(g & 1) && r + 1 < hi && g + 1 < n) zz[r + 1] = z1;
+                        }
                     }
                 }
+                for (int r = lo - 1 + t; r < hi; r += kTbBS)
+                    edge_gradient(nz, gsite(r), n, hA[r], hA[r + 1], L, arc, dv[r], sl[r]);
                 __syncthreads();
-                for (int r = lo + t; r < hi; r += kRunBS) {
-                    const double gr = site_gradient<Noise>(hA[r - 1], hA[r], hA[r + 1], dv[r - 1], dv[r],
-                                                    sl[r - 1], sl[r], L, lt, f, arc);
+                for (int r = lo + t; r < hi; r += kTbBS) {
+                    const double gr = site_gradient<Noise>(hA[r - 1], hA[r], hA[r + 1], dv[r - 1],
+                                                           dv[r], sl[r - 1], sl[r], L, lt, f, arc);
                     hB[r] = (b > 0) ? hA[r] + (-a * gr + b * zz[r]) : hA[r] + -a * gr;
                 }
                 __syncthreads();
@@ -231,7 +251,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
                 hA = hB;
                 hB = sw;
             }
-            for (int r = Kr + t; r < Kr + S; r += kRunBS) nxt[s0 + r - Kr] = hA[r];
+            for (int r = Kr + t; r < Kr + S; r += kTbBS) nxt[s0 + r - Kr] = hA[r];
         }
         if (!grid_sync_bounded(sync, gridDim.x, arrivals)) return;
         double *sw = cur;
@@ -239,7 +259,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
         nxt = sw;
     }
     if (cur != h)
-        for (int i = blockIdx.x * kRunBS + t; i < n; i += gridDim.x * kRunBS) h[i] = __ldcg(cur + i);
+        for (int i = blockIdx.x * kTbBS + t; i < n; i += gridDim.x * kTbBS) h[i] = __ldcg(cur + i);
 }
 
 // Whether a functor gathers from the FP64 cell-polynomial store (a tuning class of its own).
@@ -380,12 +400,13 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
         auto kern = k_langevin_run<decltype(nz), kN32>;
         auto kern_tb = k_langevin_run_tb<decltype(nz), kN32>;
         const int cap = ctx->warp_cap > 0 ? std::max(1, ctx->warp_cap / (kRunBS / 32)) : INT_MAX;
+        const int tb_cap = ctx->warp_cap > 0 ? std::max(1, ctx->warp_cap / (kTbBS / 32)) : INT_MAX;
         // grid, segment and shared memory of candidate c (c >= 1); false when
         // its shared memory or co-residency does not fit
         auto shape = [&](int c, int &grid, int &seg, int &K, size_t &smem) -> bool {
             const int cps = 1 << ((c - 1) / 3);
             K = 8 << ((c - 1) % 3);
-            grid = std::min(std::min(ctx->num_sms * cps, cap), std::max(1, n / 64));
+            grid = std::min(std::min(ctx->num_sms * cps, tb_cap), std::max(1, n / 64));
             seg = (n + grid - 1) / grid;
             grid = (n + seg - 1) / seg;  // no empty CTAs
             smem = (size_t)kTbBufs * (size_t)(seg + 2 * K) * sizeof(double);
@@ -411,7 +432,7 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
                 }
             }
             int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern_tb, kRunBS, smem) !=
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern_tb, kTbBS, smem) !=
                 cudaSuccess) {
                 cudaGetLastError();
                 return false;
@@ -429,7 +450,7 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
                                 (void *)&nsteps, (void *)&d_drift, (void *)&d_diff, (void *)&d_rs,
                                 (void *)&seed,   (void *)&sync,   (void *)&seg,    (void *)&K};
                 QEW_CUDA(ctx, cudaLaunchCooperativeKernel((const void *)kern_tb, dim3(grid),
-                                                          dim3(kRunBS), args, smem, ctx->stream));
+                                                          dim3(kTbBS), args, smem, ctx->stream));
                 return qew_launch_check(ctx, "langevin_run");
             }
             int per_sm = 0;
@@ -451,13 +472,11 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
         constexpr int kTuneSteps = 4096, kProbeSteps = 64;
         const int cls = qew_tune_class(n, (kN32 ? 1 : 0) + (model == QEW_MODEL_ARCLENGTH ? 2 : 0) +
                                               (reads_poly_store(nz) ? 4 : 0));
-        // Defaults from measurement at L = 65536: FP32 runs K = 16 steps per
-        // barrier at 2 CTAs per SM (515 against 804 us per 64 steps); FP64
-        // runs one barrier per step, where the FP64 work of a step (the FP64
-        // Box-Muller increments above all) outweighs the barrier and the
-        // halo's extra work made the blocked shapes no faster. A tuned shape
-        // must be 5 % faster than the default on the probe.
-        const int dflt = kN32 ? 5 : 0;
+        // Default from measurement at L = 65536 (us a step): K = 16 steps per
+        // barrier at 2 CTAs per SM, FP64 6.2 against 10.9 with one barrier per
+        // step, FP32 4.0 against 7.9. A tuned shape must be 5 % faster than the
+        // default on the probe.
+        const int dflt = 5;
         int cand = dflt;
         const int cached = qew_tune_cached(ctx->device, kTuneLangevinRun, cls);
         if (ctx->tune_force[kTuneLangevinRun] >= 0 || (cached < 0 && steps >= kTuneSteps)) {

@@ -34,6 +34,8 @@ struct NoiseSplit32 {
     bool dx_pow2, dy_pow2;
     bool xconst;  // as NoiseBSpline64::xconst
     float inv_dy_f;
+    int ky;  // y * 2^ky == y / dy exactly, or kPolyNotPow2; kNoFixedRow: FP64 locate only
+    static constexpr int kNoFixedRow = kPolyNotPow2 + 1;
     QEW_OOB_MEMBER
 
     __device__ __forceinline__ void loc_x(double x, int &ix, float &fx) const {
@@ -45,6 +47,24 @@ struct NoiseSplit32 {
         double f;
         grid_locate(y, dy, inv_dy, dy_pow2, ny, iy, f);
         fy = (float)f;
+    }
+    // The row cell and FP32 fraction at height a / 2: loc_y's numbers from the
+    // bits of a (qew_fix.cuh), where the FP64 locate takes nine FP64
+    // instructions and conversions, 64 cycles of the scheduler's FP64 unit each.
+    __device__ __forceinline__ void loc_y_sum(double a, int &iy, float &fy) const {
+        unsigned long long f = 0;
+        bool ok = false;
+        if (ky < kPolyNotPow2) {
+            ok = fx_cell64(a, ky - 1, ny, iy, f);
+        } else if (ky == kPolyNotPow2) {
+            const unsigned ef = ((unsigned)__double2hiint(a) >> 20) & 0x7FFu;
+            if (ef - 523u <= 1000u)
+                ok = fx_cell64(NoiseBSpline64::div_by(a, 2.0 * dy, 0.5 * inv_dy), 0, ny, iy, f);
+        }
+        if (ok)
+            fy = fx_frac_to_float(f);
+        else
+            loc_y(a * 0.5, iy, fy);
     }
     __device__ __forceinline__ float taps(int ix, float fx, int iy, float fy, bool deriv) const {
         float wx[4], wy[4];
@@ -120,18 +140,19 @@ struct NoiseSplit32 {
         loc_y(y, iy, fy);
         return (double)(taps(ix, fx, iy, fy, true) * inv_dy_f);
     }
-    __device__ __forceinline__ double value_edge(int e, double xc, double y) const {
-        if (!xconst || e + 1 >= nx) return value(xc, y);
+    // At the midpoint a / 2 of edge e (xc its physical x).
+    __device__ __forceinline__ double value_edge_sum(int e, double xc, double a) const {
+        if (!xconst || e + 1 >= nx) return value(xc, a * 0.5);
         int iy;
         float fy;
-        loc_y(y, iy, fy);
+        loc_y_sum(a, iy, fy);
         return (double)(edge ? taps_edge(e, iy, fy, false) : taps(e, 0.5f, iy, fy, false));
     }
-    __device__ __forceinline__ double dvdy_edge(int e, double xc, double y) const {
-        if (!xconst || e + 1 >= nx) return dvdy(xc, y);
+    __device__ __forceinline__ double dvdy_edge_sum(int e, double xc, double a) const {
+        if (!xconst || e + 1 >= nx) return dvdy(xc, a * 0.5);
         int iy;
         float fy;
-        loc_y(y, iy, fy);
+        loc_y_sum(a, iy, fy);
         const float t = edge ? taps_edge(e, iy, fy, true) : taps(e, 0.5f, iy, fy, true);
         return (double)(t * inv_dy_f);
     }
@@ -150,11 +171,11 @@ __device__ __forceinline__ unsigned long long *qew_noise_oob(const NoiseSplit32 
 #endif
 __device__ __forceinline__ double noise_dvdy_edge(const NoiseSplit32 &nz, int e, double xc,
                                                   double a) {
-    return nz.dvdy_edge(e, xc, a * 0.5);
+    return nz.dvdy_edge_sum(e, xc, a);
 }
 __device__ __forceinline__ double noise_value_edge(const NoiseSplit32 &nz, int e, double xc,
                                                    double a) {
-    return nz.value_edge(e, xc, a * 0.5);
+    return nz.value_edge_sum(e, xc, a);
 }
 
 static inline NoiseSplit32 make_split32(const qew_field *f, int n, double physical_size) {
@@ -171,6 +192,12 @@ static inline NoiseSplit32 make_split32(const qew_field *f, int n, double physic
     nz.xconst = (n > 0 && n == f->nx && physical_size == f->Lx && nz.dx_pow2);
     nz.edge = nz.xconst ? f->edge32 : nullptr;
     nz.inv_dy_f = (float)(1.0 / f->dy);
+    {
+        int e;
+        const double m = frexp(f->dy, &e);
+        nz.ky = !qew_fixed_div_ok(f->dy) ? NoiseSplit32::kNoFixedRow
+                                         : (m == 0.5 ? 1 - e : kPolyNotPow2);
+    }
 #ifdef QEW_BOUNDS_CHECK
     nz.oob = qew_bounds_words();
 #endif
