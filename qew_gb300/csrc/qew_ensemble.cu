@@ -19,11 +19,12 @@
 
 #include "qew_lbfgs_internal.cuh"
 #include "qew_lbfgs_resident.cuh"
+#include "qew_lbfgs_gram.cuh"
 #include "qew_noise32.cuh"
 
 namespace {
 
-constexpr int kEnsBS = 512;
+constexpr int kEnsBS = 256;
 
 struct EnsJob {
     NoiseBSpline64 nz64;
@@ -60,10 +61,10 @@ k_ensemble(const EnsJob *__restrict__ jobs, const int *__restrict__ order, int c
         if (k >= count) break;
         const int id = order[k];
         const EnsJob j = jobs[id];
-        const size_t npad = ((size_t)j.n + 31) & ~size_t(31);
+        const size_t npad = gram_npad(j.n, kEnsBS);
         qew_lbfgs_result r32{};
         if (use32) r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(j.nz32, j.h, j.n, j.p, cfg32, j.pc, ws, npad);
-        qew_lbfgs_result r = lbfgs_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws, npad);
+        qew_lbfgs_result r = lbfgs_gram_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws);
         if (threadIdx.x == 0) {
             r.iterations += r32.iterations;
             r.n_func_evals += r32.n_func_evals;
@@ -109,7 +110,7 @@ extern "C" qew_status qew_ensemble_minimize(qew_ctx *ctx, int count, const qew_e
     int per_sm = 0;
     QEW_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_ensemble, kEnsBS, 0));
     const int grid = std::max(1, std::min(count, ctx->num_sms * std::max(per_sm, 1)));
-    const size_t npad_max = ((size_t)nmax + 31) & ~size_t(31);
+    const size_t npad_max = gram_npad(nmax, kEnsBS);
     const size_t ws_per_cta = npad_max * (size_t)(kLbfgsVecs + 2 * (lp.m + 1));
     // layout: [ws (grid x ws_per_cta doubles)][jobs][order][results][counter]
     const size_t off_jobs = ((ws_per_cta * grid * sizeof(double)) + 255) & ~size_t(255);
@@ -204,13 +205,13 @@ k_serve_static(LaneRing *ring, unsigned int *head, LbfgsCfg cfg32, LbfgsCfg cfg6
         if (k < 0) break;
         const EnsJob j = s_job;
         __syncthreads();
-        const size_t npad = ((size_t)j.n + 31) & ~size_t(31);
+        const size_t npad = gram_npad(j.n, kEnsBS);
         qew_lbfgs_result r32{};
         if (use32)
             r32 = lbfgs_block<NoiseSplit32, kEnsBS, float>(j.nz32, j.h, j.n, j.p, cfg32,
                                                            j.pc, ws, npad);
         qew_lbfgs_result r =
-            lbfgs_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws, npad);
+            lbfgs_gram_block<NoiseBSpline64, kEnsBS>(j.nz64, j.h, j.n, j.p, cfg64, j.pc, ws);
         if (threadIdx.x == 0) {
             r.iterations += r32.iterations;
             r.n_func_evals += r32.n_func_evals;
@@ -257,7 +258,7 @@ qew_status qew_lane_create(int device, int nmax, const qew_lbfgs_params *lp, dou
     L->cfg64 = lbfgs_cfg_from(lp);
     L->cfg32 = L->cfg64;
     L->cfg32.ftol = ftol32;
-    const size_t npad_max = ((size_t)nmax + 31) & ~size_t(31);
+    const size_t npad_max = gram_npad(nmax, kEnsBS);
     L->ws_per_cta = npad_max * (size_t)(kLbfgsVecs + 2 * (lp->m + 1));
     auto fail = [&](qew_status s) {
         if (L->ws) cudaFree(L->ws);

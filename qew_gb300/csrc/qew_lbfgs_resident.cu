@@ -24,6 +24,7 @@
 #include "qew_lbfgs_internal.cuh"
 #include "qew_noise32.cuh"
 #include "qew_lbfgs_resident.cuh"
+#include "qew_lbfgs_gram.cuh"
 
 PrecondCoef qew_precond_coef(int n, double kappa, double physical_size, double shift) {
     PrecondCoef pc{};
@@ -47,7 +48,7 @@ PrecondCoef qew_precond_coef(int n, double kappa, double physical_size, double s
 
 namespace {
 
-constexpr int kResBS = 512;
+constexpr int kResBS = 256;  // as the ensemble: a line relaxes the same alone and in a batch
 
 template <int BS>
 __global__ void __launch_bounds__(BS) k_precond_resident(const double *q, double *d, int n,
@@ -59,6 +60,10 @@ __global__ void __launch_bounds__(BS) k_precond_resident(const double *q, double
 
 constexpr int kClusterBS = 256;
 constexpr int kClusterMinN = 2048;
+// Dynamic shared memory for a solve's vectors: up to this, beside the kernels'
+// static 35 KB, they stay on the SM (59 KB per point a thread owns at m = 10);
+// beyond it they lie in global memory.
+constexpr size_t kGramDynSmem = 190 * 1024;
 #ifndef QEW_CLUSTER_POINTS_PER_THREAD
 #define QEW_CLUSTER_POINTS_PER_THREAD 1  // build-time tuning knob (measured on GB300)
 #endif
@@ -73,16 +78,16 @@ struct ClusterLine {
 template <class Noise, int BS>
 __global__ void __launch_bounds__(BS)
 k_lbfgs_cluster(Noise nz, const ClusterLine *__restrict__ lines, int n, LbfgsCfg cfg, double *ws,
-                size_t ws_stride, size_t npad, qew_lbfgs_result *out) {
-    __shared__ double s_w[96];
-    __shared__ double s_red[2 * 3 * kTeamMaxCtas];
+                size_t ws_cta, qew_lbfgs_result *out) {
+    extern __shared__ double s_dyn[];  // the vectors, when ws is null
     cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
     const unsigned size = cl.num_blocks();
-    ClusterTeam<BS> T{s_w, s_red, cl.block_rank(), size};
+    ClusterTeam<BS> T{cl.block_rank(), size};
     const int line = blockIdx.x / size;
     const ClusterLine L = lines[line];
     const qew_lbfgs_result r =
-        lbfgs_team<Noise>(T, nz, L.h, n, L.p, cfg, L.pc, ws + (size_t)line * ws_stride, npad);
+        lbfgs_gram<Noise>(T, nz, L.h, n, L.p, cfg, L.pc,
+                          ws ? ws + (size_t)blockIdx.x * ws_cta : s_dyn);
     if (T.rank() == 0 && threadIdx.x == 0) out[line] = r;
     cl.sync();  // no CTA leaves while another may still write its shared memory
 }
@@ -90,9 +95,9 @@ k_lbfgs_cluster(Noise nz, const ClusterLine *__restrict__ lines, int n, LbfgsCfg
 template <class Noise, int BS>
 __global__ void __launch_bounds__(BS)
 k_lbfgs_single(Noise nz, double *h, int n, qew_params P, LbfgsCfg cfg, PrecondCoef pc,
-               double *ws, size_t npad, qew_lbfgs_result *out) {
-    extern __shared__ double s_dyn[];
-    const qew_lbfgs_result r = lbfgs_block<Noise, BS>(nz, h, n, P, cfg, pc, ws, npad);
+               double *ws, qew_lbfgs_result *out) {
+    extern __shared__ double s_dyn[];  // the vectors, when ws is null
+    const qew_lbfgs_result r = lbfgs_gram_block<Noise, BS>(nz, h, n, P, cfg, pc, ws ? ws : s_dyn);
     if (threadIdx.x == 0) *out = r;
 }
 
@@ -142,17 +147,8 @@ static qew_status lbfgs_cluster_launch(qew_ctx *ctx, const Noise &nz, int csize,
                                        const std::vector<ClusterLine> &lines, int n,
                                        const qew_lbfgs_params *lp, qew_lbfgs_result *res) {
     const int count = (int)lines.size();
-    const size_t npad = ((size_t)n + 31) & ~size_t(31);
-    const size_t wsd = qew_lbfgs_resident_ws_doubles(n, lp->m);
-    const size_t off_lines = (wsd * count * sizeof(double) + 255) & ~size_t(255);
-    const size_t off_res = (off_lines + sizeof(ClusterLine) * count + 255) & ~size_t(255);
-    QEW_TRY(qew_scratch_reserve(ctx, off_res + sizeof(qew_lbfgs_result) * count + 256));
-    char *base = (char *)ctx->scratch;
-    ClusterLine *d_lines = (ClusterLine *)(base + off_lines);
-    qew_lbfgs_result *d_res = (qew_lbfgs_result *)(base + off_res);
-    QEW_CUDA(ctx, cudaMemcpyAsync(d_lines, lines.data(), sizeof(ClusterLine) * count,
-                                  cudaMemcpyHostToDevice, ctx->stream));
-    const LbfgsCfg cfg = lbfgs_cfg_from(lp);
+    auto kern = k_lbfgs_cluster<Noise, kClusterBS>;
+    const size_t ws_cta = gram_ws(n, csize * kClusterBS, kClusterBS, lp->m);  // doubles
     cudaLaunchConfig_t lc = {};
     lc.gridDim = dim3((unsigned)(count * csize));
     lc.blockDim = dim3(kClusterBS);
@@ -164,19 +160,34 @@ static qew_status lbfgs_cluster_launch(qew_ctx *ctx, const Noise &nz, int csize,
     at[0].val.clusterDim.z = 1;
     lc.attrs = at;
     lc.numAttrs = 1;
-    double *ws = (double *)base;
-    QEW_CUDA(ctx, cudaLaunchKernelEx(&lc, k_lbfgs_cluster<Noise, kClusterBS>, nz,
-                                     (const ClusterLine *)d_lines, n, cfg, ws, wsd, npad, d_res));
+    size_t smem = ws_cta * sizeof(double);
+    int clusters = 0;
+    if (smem <= kGramDynSmem &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGramDynSmem) ==
+            cudaSuccess) {
+        lc.dynamicSmemBytes = smem;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &lc) != cudaSuccess) clusters = 0;
+    }
+    cudaGetLastError();
+    if (clusters == 0) smem = 0;
+    lc.dynamicSmemBytes = smem;
+    const size_t wsd = smem ? 0 : ws_cta * csize;
+    const size_t off_lines = (wsd * count * sizeof(double) + 255) & ~size_t(255);
+    const size_t off_res = (off_lines + sizeof(ClusterLine) * count + 255) & ~size_t(255);
+    QEW_TRY(qew_scratch_reserve(ctx, off_res + sizeof(qew_lbfgs_result) * count + 256));
+    char *base = (char *)ctx->scratch;
+    ClusterLine *d_lines = (ClusterLine *)(base + off_lines);
+    qew_lbfgs_result *d_res = (qew_lbfgs_result *)(base + off_res);
+    QEW_CUDA(ctx, cudaMemcpyAsync(d_lines, lines.data(), sizeof(ClusterLine) * count,
+                                  cudaMemcpyHostToDevice, ctx->stream));
+    const LbfgsCfg cfg = lbfgs_cfg_from(lp);
+    QEW_CUDA(ctx, cudaLaunchKernelEx(&lc, kern, nz, (const ClusterLine *)d_lines, n, cfg,
+                                     smem ? (double *)nullptr : (double *)base, ws_cta, d_res));
     QEW_TRY(qew_launch_check(ctx, "lbfgs_cluster"));
     QEW_CUDA(ctx, cudaMemcpyAsync(res, d_res, sizeof(qew_lbfgs_result) * count,
                                   cudaMemcpyDeviceToHost, ctx->stream));
     QEW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return QEW_OK;
-}
-
-size_t qew_lbfgs_resident_ws_doubles(int n, int m) {
-    const size_t npad = ((size_t)n + 31) & ~size_t(31);
-    return npad * (size_t)(kLbfgsVecs + 2 * (m + 1));
 }
 
 qew_status qew_lbfgs_resident(qew_ctx *ctx, const qew_field *field, double *d_h, int n,
@@ -196,20 +207,18 @@ qew_status qew_lbfgs_resident(qew_ctx *ctx, const qew_field *field, double *d_h,
                                     res);
     }, n, p->physical_size));
     if (clustered) return QEW_OK;
-    const size_t npad = ((size_t)n + 31) & ~size_t(31);
-    const size_t wsd = qew_lbfgs_resident_ws_doubles(n, lp->m);
-    const size_t res_off = (wsd * sizeof(double) + 255) & ~size_t(255);
+    const size_t ws_cta = gram_ws(n, kResBS, kResBS, lp->m) * sizeof(double);
+    const size_t smem = ws_cta <= kGramDynSmem ? ws_cta : 0;
+    const size_t res_off = ((smem ? 0 : ws_cta) + 255) & ~size_t(255);
     QEW_TRY(qew_scratch_reserve(ctx, res_off + sizeof(qew_lbfgs_result) + 256));
-    double *ws = (double *)ctx->scratch;
+    double *ws = smem ? nullptr : (double *)ctx->scratch;
     qew_lbfgs_result *d_res = (qew_lbfgs_result *)((char *)ctx->scratch + res_off);
-    LbfgsCfg cfg = lbfgs_cfg_from(lp);
-    PrecondCoef pc{};
-    if (lp->precondition) pc = qew_precond_coef(n, p->line_tension, p->physical_size, lp->precond_shift);
-    const size_t smem = lbfgs_block_smem_bytes(kResBS, lp->m);
+    const LbfgsCfg cfg = lbfgs_cfg_from(lp);
     QEW_TRY(qew_dispatch_noise(ctx, field, [&](auto nz) -> qew_status {
         auto kern = k_lbfgs_single<decltype(nz), kResBS>;
-        QEW_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kern<<<1, kResBS, smem, ctx->stream>>>(nz, d_h, n, *p, cfg, pc, ws, npad, d_res);
+        QEW_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kGramDynSmem));
+        kern<<<1, kResBS, smem, ctx->stream>>>(nz, d_h, n, *p, cfg, pc1, ws, d_res);
         return qew_launch_check(ctx, "lbfgs_resident");
     }, n, p->physical_size));
     QEW_CUDA(ctx, cudaMemcpyAsync(res, d_res, sizeof(qew_lbfgs_result), cudaMemcpyDeviceToHost, ctx->stream));

@@ -1,6 +1,6 @@
 // qew_lbfgs_resident.cuh -- one CTA runs one complete lbfgs_minimize
-// (lbfgs.h:94-287). Shared by the single-line entry point and the batched
-// ensemble kernel.
+// (lbfgs.h:94-287) term by term: the ensemble's FP32 first phase. (FP64 solves
+// go by inner products, qew_lbfgs_gram.cuh, which shares the settings here.)
 #pragma once
 
 #include "qew_team.cuh"
@@ -43,8 +43,6 @@ inline LbfgsCfg lbfgs_cfg_from(const qew_lbfgs_params *lp) {
     return c;
 }
 
-inline size_t lbfgs_block_smem_bytes(int /*bs*/, int /*m*/) { return 0; }
-
 // History bookkeeping of lbfgs.h:107-114, 262-279: `slots` in chronological
 // order, and buffer indices standing in for the reference's View swaps.
 struct LbfgsShared {
@@ -63,12 +61,11 @@ struct LbfgsShared {
 // + spare, m Y rows + spare; Real). Real = float keeps the vectors and their
 // dot products in FP32 (a first phase on FP32 coefficients); positions,
 // energies, reductions across threads and every scalar stay FP64.
-template <class Noise, class Team, class Real = double>
+template <class Noise, class Team, class Real>
 __device__ qew_lbfgs_result lbfgs_team(Team &T, const Noise &nz, double *__restrict__ h,
                                        const int n, const qew_params P, const LbfgsCfg cfg,
                                        const PrecondCoef pc, double *ws, size_t npad) {
     __shared__ double s_b[Team::kBS];
-    __shared__ double s_agg[2 * kTeamMaxCtas];
     __shared__ LbfgsShared sh;
     const int t0 = T.tid(), ts = T.stride();
     const LineDx dx = make_line_dx(P.physical_size, n, P.line_tension, P.driving_force);
@@ -134,7 +131,7 @@ __device__ qew_lbfgs_result lbfgs_team(Team &T, const Noise &nz, double *__restr
             T.sync();
         }
         if (cfg.precondition) {
-            team_precond(T, q, d, n, pc, s_b, s_agg);
+            block_precond<Team::kBS, Real>(q, d, n, pc, s_b, T.s_w);
         } else {
             const double g0 = (hs == 0) ? 1.0 : gamma;
             for (int i = t0; i < n; i += ts) d[i] = (Real)(g0 * q[i]);
@@ -278,10 +275,8 @@ __device__ qew_lbfgs_result lbfgs_team(Team &T, const Noise &nz, double *__restr
     return res;  // identical in every thread
 }
 
-
-// One CTA runs the whole solve (the single-line resident form and the
-// ensemble's CTA per line).
-template <class Noise, int BS, class Real = double>
+// One CTA runs the whole solve.
+template <class Noise, int BS, class Real>
 __device__ qew_lbfgs_result lbfgs_block(const Noise &nz, double *__restrict__ h, const int n,
                                         const qew_params P, const LbfgsCfg cfg,
                                         const PrecondCoef pc, double *ws, size_t npad) {
@@ -290,4 +285,3 @@ __device__ qew_lbfgs_result lbfgs_block(const Noise &nz, double *__restrict__ h,
     return lbfgs_team<Noise, CtaTeam<BS>, Real>(T, nz, h, n, P, cfg, pc, ws, npad);
 }
 
-size_t qew_lbfgs_resident_ws_doubles(int n, int m);
