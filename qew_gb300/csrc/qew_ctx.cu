@@ -93,7 +93,6 @@ qew_status qew_ctx_create(int device, qew_ctx **out) {
         cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
         cudaMalloc(&ctx->red_partials, sizeof(double) * 4 * QEW_RED_MAX_BLOCKS) != cudaSuccess ||
         cudaMalloc(&ctx->red_counter, sizeof(unsigned int) * 8) != cudaSuccess ||
-        cudaMalloc(&ctx->red_out, sizeof(double) * 8) != cudaSuccess ||
         cudaMallocHost(&ctx->host_out, sizeof(double) * 8) != cudaSuccess ||
         cudaMemset(ctx->red_counter, 0, sizeof(unsigned int) * 8) != cudaSuccess ||
         !keep_pool_cache(device) ||
@@ -112,7 +111,6 @@ qew_status qew_ctx_destroy(qew_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     if (ctx->red_partials) cudaFree(ctx->red_partials);
     if (ctx->red_counter) cudaFree(ctx->red_counter);
-    if (ctx->red_out) cudaFree(ctx->red_out);
     if (ctx->host_out) cudaFreeHost(ctx->host_out);
     if (ctx->scratch) cudaFreeAsync(ctx->scratch, ctx->stream);
     cudaStreamSynchronize(ctx->stream);

@@ -30,8 +30,7 @@ struct qew_ctx {
     // reduction scratch: per-block partials + a self-resetting ticket counter
     double *red_partials = nullptr;  // QEW_RED_MAX_BLOCKS * 4 doubles
     unsigned int *red_counter = nullptr;
-    double *red_out = nullptr;       // 8 doubles of device results
-    double *host_out = nullptr;      // pinned 8 doubles
+    double *host_out = nullptr;      // 8 doubles of results: pinned, written by the kernels
     // general scratch arena (grown on demand, never shrunk)
     void *scratch = nullptr;
     size_t scratch_bytes = 0;

@@ -321,7 +321,7 @@ qew_status qew_poly_store_build(qew_ctx *ctx, const double *c, int nx, int ny,
 qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count,
                                      const double *d_h, int n, const qew_params *p,
                                      double *d_grad) {
-    if (!f || f->kind != QEW_FIELD_BSPLINE || !f->coef64) return QEW_ERR_UNSUPPORTED;
+    if (!f || f->kind != QEW_FIELD_BSPLINE || !f->coef64 || !f->poly) return QEW_ERR_UNSUPPORTED;
     PolyGeom g{};
     g.nz = make_bspline64(f, n, p->physical_size);
     if (!g.nz.poly || g.nz.kb < 0) return QEW_ERR_UNSUPPORTED;

@@ -119,14 +119,13 @@ static __global__ void k_neg_copy(int n, const double *__restrict__ x, double *_
     if (i < n) y[i] = -x[i];
 }
 
-// Host wrappers: launch a reduction and read the NV results back (synchronous).
+// Host wrappers: launch a reduction, whose last block writes the NV results
+// into pinned host memory, and read them (synchronous).
 template <class F, int NV, bool MAX>
 qew_status vec_reduce(qew_ctx *ctx, int n, const F &fn, double *res) {
     k_reduce<F, NV, MAX><<<vec_red_blocks(n), kVecBS, 0, ctx->stream>>>(
-        n, fn, ctx->red_partials, ctx->red_counter, ctx->red_out);
+        n, fn, ctx->red_partials, ctx->red_counter, ctx->host_out);
     QEW_TRY(qew_launch_check(ctx, "reduce"));
-    QEW_CUDA(ctx, cudaMemcpyAsync(ctx->host_out, ctx->red_out, sizeof(double) * NV,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
     QEW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     for (int k = 0; k < NV; ++k) res[k] = ctx->host_out[k];
     return QEW_OK;
