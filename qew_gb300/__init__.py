@@ -60,9 +60,15 @@ __all__ = [
 ]
 
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 class Model(enum.IntEnum):  # qew_model.h:20
@@ -143,15 +149,19 @@ class Context:
     def __init__(self, device: int = 0):
         self.lib = _capi.load()
         self.device = device
+        self._stream = None
         h = C.c_void_p()
         _capi.check(self.lib.qew_ctx_create(device, C.byref(h)), None, "qew_ctx_create")
         self.h = h
 
     def sync_stream(self):
         """Run subsequent work on torch's current stream of this device."""
-        torch = _torch()
-        s = torch.cuda.current_stream(self.device).cuda_stream
-        self.lib.qew_ctx_set_stream(self.h, C.c_void_p(s))
+        if self._stream is None:
+            torch = _torch()
+            torch.cuda.init()
+            # the handle alone: the Stream object around it takes 1 us a call
+            self._stream = torch._C._cuda_getCurrentRawStream
+        self.lib.qew_ctx_set_stream(self.h, self._stream(self.device))
 
     def launches(self) -> int:
         return int(self.lib.qew_ctx_launch_count(self.h))
