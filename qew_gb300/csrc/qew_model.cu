@@ -2,22 +2,32 @@
 //
 // gradient: the reference runs two kernels, an edge pass writing dV/dy (and
 // the arclength slope) of every edge to scratch and a per-site combine
-// (qew_model.h:163-193). Here one kernel does both: each CTA computes the
-// edges of its sites plus one halo edge into shared memory, then combines, so
-// the per-edge scratch never touches HBM and one launch replaces two.
+// (qew_model.h:163-193). Here one kernel does both: a CTA of BS threads takes
+// the BS edges of BS - 1 sites and combines them through shared memory, so the
+// per-edge scratch never touches HBM and one launch replaces two; the lines of
+// a batch share the launch. Short lines are bound by one chain of latencies
+// (heights, stencil rows, the integer products, the combine), long ones by the
+// issue of the gather. (With BS sites a CTA, thread 0 took the extra edge after
+// its own and the whole warp waited: 8.2 us a call at 1024 points, now 6.2;
+// three lines of 100003 points 42.9 -> 20.5 us with one launch for all.)
 //
 // objective: the per-edge energy (qew_model.h:61-83) reduced by a fixed
 // grid-stride / warp-shuffle / CTA tree with a last-block final sum, so the
 // result is bit-reproducible for a given n regardless of scheduling. The last
 // block writes the sum into pinned host memory: a call is one launch and one
 // wait (20.7 us at 16384 points; 29.7 with a copy from device memory between).
+#include <algorithm>
+
 #include "qew_internal.cuh"
 #include "qew_model_kernels.cuh"
 #include "qew_poly.cuh"
 
 namespace {
 
-constexpr int kGradBS = 256;
+// 128 threads: a short line spreads over more SMs, each scheduler's FP64 unit
+// serving one warp (1024 points 6.2 us a call, 7.2 with 256 threads; 64 threads
+// the same there but 71.6 against 68.2 us at 2^20 points).
+constexpr int kGradBS = 128;
 constexpr int kObjBS = 256;
 
 int objective_blocks(int n) {
@@ -76,30 +86,52 @@ static qew_status gradient_mapped(qew_ctx *ctx, const qew_field *field, int coun
     return QEW_OK;
 }
 
-qew_status qew_gradient_enqueue(qew_ctx *ctx, const qew_field *field, const double *d_h, int n,
-                                const qew_params *p, int precision, double *d_grad) {
-    if (!ctx || !field || !p || !d_h || !d_grad || n < 1)
-        return qew_fail(ctx, QEW_ERR_INVALID, "gradient: bad arguments");
+// Lines k = 0..count-1, n apart, on the FP64 gathers: one launch for up to
+// 65535 of them.
+static qew_status gradient_fp64(qew_ctx *ctx, const qew_field *field, int count, const double *d_h,
+                                int n, const qew_params *p, int precision, double *d_grad) {
     const LineDx dx = make_line_dx(p->physical_size, n, p->line_tension, p->driving_force);
-    const int blocks = (n + kGradBS - 1) / kGradBS;
+    auto launch = [&](auto nz) -> qew_status {
+        const unsigned blocks = (unsigned)(((long long)n + kGradBS - 2) / (kGradBS - 1));
+        for (int k = 0; k < count; k += 65535) {
+            const size_t off = (size_t)k * (size_t)n;
+            k_gradient<decltype(nz), kGradBS>
+                <<<dim3(blocks, (unsigned)std::min(count - k, 65535)), kGradBS, 0, ctx->stream>>>(
+                    d_h + off, n, dx, p->line_tension, p->driving_force, p->model, nz, d_grad + off);
+            QEW_TRY(qew_launch_check(ctx, "gradient"));
+        }
+        return QEW_OK;
+    };
+    if (precision == QEW_PREC_FP64_REFERENCE) return qew_dispatch_noise_ref(ctx, field, launch);
+    return qew_dispatch_noise(ctx, field, launch, n, p->physical_size);
+}
+
+static qew_status gradient_enqueue(qew_ctx *ctx, const qew_field *field, int count,
+                                   const double *d_h, int n, const qew_params *p, int precision,
+                                   double *d_grad) {
     if (precision == QEW_PREC_FP32_SPLIT) {
         if (field->kind != QEW_FIELD_BSPLINE || !field->coef32)
             return qew_fail(ctx, QEW_ERR_INVALID,
                             "gradient: FP32 split gather needs a B-spline field stored with QEW_STORE_FP32");
-        return qew_gradient_split_enqueue(ctx, field, d_h, n, p, d_grad);
+        for (int k = 0; k < count; ++k)
+            QEW_TRY(qew_gradient_split_enqueue(ctx, field, d_h + (size_t)k * n, n, p,
+                                               d_grad + (size_t)k * n));
+        return QEW_OK;
     }
-    auto launch = [&](auto nz) -> qew_status {
-        k_gradient<decltype(nz), kGradBS><<<blocks, kGradBS, 0, ctx->stream>>>(
-            d_h, n, dx, p->line_tension, p->driving_force, p->model, nz, d_grad);
-        return qew_launch_check(ctx, "gradient");
-    };
-    if (precision == QEW_PREC_FP64_REFERENCE) return qew_dispatch_noise_ref(ctx, field, launch);
-    if (precision != QEW_PREC_FP64)
+    if (precision != QEW_PREC_FP64 && precision != QEW_PREC_FP64_REFERENCE)
         return qew_fail(ctx, QEW_ERR_INVALID, "gradient: unknown precision %d", precision);
-    // the cell-polynomial store, when it serves this line
-    const qew_status s = qew_gradient_poly_enqueue(ctx, field, 1, d_h, n, p, d_grad);
-    if (s != QEW_ERR_UNSUPPORTED) return s;
-    return qew_dispatch_noise(ctx, field, launch, n, p->physical_size);
+    if (precision == QEW_PREC_FP64) {  // the cell-polynomial store, when it serves this line
+        const qew_status s = qew_gradient_poly_enqueue(ctx, field, count, d_h, n, p, d_grad);
+        if (s != QEW_ERR_UNSUPPORTED) return s;
+    }
+    return gradient_fp64(ctx, field, count, d_h, n, p, precision, d_grad);
+}
+
+qew_status qew_gradient_enqueue(qew_ctx *ctx, const qew_field *field, const double *d_h, int n,
+                                const qew_params *p, int precision, double *d_grad) {
+    if (!ctx || !field || !p || !d_h || !d_grad || n < 1)
+        return qew_fail(ctx, QEW_ERR_INVALID, "gradient: bad arguments");
+    return gradient_enqueue(ctx, field, 1, d_h, n, p, precision, d_grad);
 }
 
 extern "C" {
@@ -137,14 +169,7 @@ qew_status qew_gradient_batch(qew_ctx *ctx, const qew_field *field, int count, c
     if (!ctx || !field || !p || !d_h || !d_grad || n < 1 || count < 0)
         return qew_fail(ctx, QEW_ERR_INVALID, "gradient_batch: bad arguments");
     if (count == 0) return QEW_OK;
-    if (precision == QEW_PREC_FP64) {
-        const qew_status s = qew_gradient_poly_enqueue(ctx, field, count, d_h, n, p, d_grad);
-        if (s != QEW_ERR_UNSUPPORTED) return s;
-    }
-    for (int k = 0; k < count; ++k)
-        QEW_TRY(qew_gradient_enqueue(ctx, field, d_h + (size_t)k * n, n, p, precision,
-                                     d_grad + (size_t)k * n));
-    return QEW_OK;
+    return gradient_enqueue(ctx, field, count, d_h, n, p, precision, d_grad);
 }
 
 qew_status qew_gradient_host(qew_ctx *ctx, const qew_field *field, const double *h_h, int n,

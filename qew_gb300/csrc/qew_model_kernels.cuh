@@ -82,36 +82,39 @@ __device__ __forceinline__ double site_gradient(double hm, double h0, double hp,
     }
 }
 
-// Fused gradient: CTA of BS sites stages h[base-1 .. base+BS] and the BS+1
-// edges it needs (its own plus the left halo edge) in shared memory.
+// gradient() of the sites [base, base + BS - 1) of line blockIdx.y: thread t
+// takes the edge left of site base + t, hands it to its neighbour through
+// shared memory, and combines that site.
 template <class Noise, int BS>
 __global__ void __launch_bounds__(BS)
 k_gradient(const double *__restrict__ h, int n, LineDx dx, double lt, double f, int model,
            Noise nz, double *__restrict__ grad) {
-    __shared__ double s_h[BS + 2];
-    __shared__ double s_dv[BS + 1];
-    __shared__ double s_sl[BS + 1];
-    const int base = blockIdx.x * BS;
+    __shared__ double s_dv[BS];
+    __shared__ double s_sl[BS];
+    const int base = blockIdx.x * (BS - 1);
     const int t = threadIdx.x;
     const int i = base + t;
-    const int cnt = min(BS, n - base);
+    const int cnt = min(BS - 1, n - base);
     const bool arc = (model == QEW_MODEL_ARCLENGTH);
 #ifdef QEW_BOUNDS_CHECK
     unsigned long long *oob = qew_noise_oob(nz);
 #endif
-    if (t < cnt) s_h[QEW_IDX(t + 1, BS + 2, oob)] = h[i];
-    if (t == 0) s_h[0] = h[base == 0 ? n - 1 : base - 1];
-    if (t == cnt - 1) s_h[QEW_IDX(cnt + 1, BS + 2, oob)] = h[(i + 1 == n) ? 0 : i + 1];
+    h += (size_t)blockIdx.y * (size_t)n;
+    grad += (size_t)blockIdx.y * (size_t)n;
+    double hm = 0.0, h0 = 0.0, hp = 0.0, dv = 0.0, sl = 0.0;
+    if (t <= cnt) {
+        const int im = i == 0 ? n - 1 : i - 1;
+        hm = h[im];
+        h0 = h[i == n ? 0 : i];
+        if (t < cnt) hp = h[i + 1 == n ? 0 : i + 1];
+        edge_gradient(nz, im, n, hm, h0, dx, arc, dv, sl);
+        s_dv[QEW_IDX(t, BS, oob)] = dv;
+        s_sl[QEW_IDX(t, BS, oob)] = sl;
+    }
     __syncthreads();
     if (t < cnt)
-        edge_gradient(nz, i, n, s_h[t + 1], s_h[QEW_IDX(t + 2, BS + 2, oob)], dx, arc,
-                      s_dv[QEW_IDX(t + 1, BS + 1, oob)], s_sl[t + 1]);
-    if (t == 0) edge_gradient(nz, base == 0 ? n - 1 : base - 1, n, s_h[0], s_h[1], dx, arc, s_dv[0], s_sl[0]);
-    __syncthreads();
-    if (t < cnt)
-        grad[i] = site_gradient<Noise>(s_h[t], s_h[t + 1], s_h[QEW_IDX(t + 2, BS + 2, oob)], s_dv[t],
-                                s_dv[QEW_IDX(t + 1, BS + 1, oob)], s_sl[t], s_sl[t + 1], dx, lt,
-                                f, arc);
+        grad[i] = site_gradient<Noise>(hm, h0, hp, dv, s_dv[QEW_IDX(t + 1, BS, oob)], sl,
+                                       s_sl[QEW_IDX(t + 1, BS, oob)], dx, lt, f, arc);
 }
 
 // Objective with a deterministic two-level reduction: fixed grid-stride
