@@ -602,8 +602,8 @@ qew_status qew_depinning_bisect_ex(qew_ctx *ctx, const qew_field *field,
  * fastest for the rest of the process:
  *   0 QEW_TUNE_GRADIENT_POLY   FP64 store gather: sites per thread {1,2,4} x
  *                              resident CTAs per SM {2,3,4} (9 candidates)
- *   1 QEW_TUNE_GRADIENT_SPLIT  FP32 split gather on the x-filtered store: sites
- *                              per thread {1,2} x CTAs per SM {4,6,8} (6)
+ *   1 QEW_TUNE_GRADIENT_SPLIT  FP32 split gather on the x-filtered store: steps
+ *                              of a warp's chunk {2,3,4} x CTAs per SM (6)
  *   2 QEW_TUNE_RK_SEARCH       Rosso-Krauth forward-zero search: 8-lane groups,
  *                              lane pairs, one lane (3; timed for 8 sweeps on
  *                              a copy of the line advanced 24 sweeps; replaces

@@ -212,19 +212,23 @@ __device__ __forceinline__ void split_edge(const SplitGeom &g, const float wx_ha
     }
 }
 
+// Second difference of three heights in y-cells.
+__device__ __forceinline__ float split_d2(const int *sc, const float *sf) {
+    return (float)(sc[0] + sc[2] - 2 * sc[1]) + (sf[0] + sf[2] - 2.0f * sf[1]);
+}
+// Gradient of a site (qew_model.h:177-193) from its second difference (linear)
+// or the slopes of its two edges (arclength) and their dV/dy.
+__device__ __forceinline__ float split_combine(const SplitGeom &g, float d2, float sl0, float sl1,
+                                               float dv0, float dv1) {
+    const float line_force = g.arc ? g.lt_over_dx * (sl0 - sl1) : -g.lt_dy_over_dx2 * d2;
+    return g.dx_f * (line_force + 0.5f * (dv0 + dv1) - g.f);
+}
 // Gradient at tile site j (height slot j + 1) from the heights either side
-// and the two edges that meet there (qew_model.h:177-193).
+// and the two edges that meet there.
 __device__ __forceinline__ float split_site(const SplitGeom &g, const int *sc, const float *sf,
                                             const float *dv, const float *sl, int j) {
-    float line_force;
-    if (!g.arc) {
-        const float d2 = (float)(sc[j] + sc[j + 2] - 2 * sc[j + 1]) +
-                         (sf[j] + sf[j + 2] - 2.0f * sf[j + 1]);
-        line_force = -g.lt_dy_over_dx2 * d2;
-    } else {
-        line_force = g.lt_over_dx * (sl[j] - sl[j + 1]);
-    }
-    return g.dx_f * (line_force + 0.5f * (dv[j] + dv[j + 1]) - g.f);
+    return split_combine(g, g.arc ? 0.0f : split_d2(sc + j, sf + j), g.arc ? sl[j] : 0.0f,
+                         g.arc ? sl[j + 1] : 0.0f, dv[j], dv[j + 1]);
 }
 
 // One CTA covers a tile of kTile = kBS * kItems consecutive sites of one line
@@ -300,100 +304,126 @@ k_gradient_split(const double *__restrict__ h64, const int *__restrict__ hc,
     }
 }
 
-// 4-byte asynchronous global -> shared copy (completes in the background;
-// cp.async.wait_all waits for the calling thread's own copies).
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
+// A site of the wrap edge (0 or n - 1), from three heights.
+__device__ __noinline__ void split_site_wrap(const SplitGeom &g, const int *hc, const float *hf,
+                                             float *out, int i) {
+    float wx_half[4], dv[2], sl[2];
+    bsw_value_f(0.5f, wx_half);
+    const int at[3] = {i == 0 ? g.n - 1 : i - 1, i, i + 1 == g.n ? 0 : i + 1};
+    int sc[3];
+    float sf[3];
+    for (int k = 0; k < 3; ++k) {
+        sc[k] = hc[at[k]];
+        sf[k] = hf[at[k]];
+    }
+    split_edge<true>(g, wx_half, at[0], sc, sf, 0, dv, sl);
+    split_edge<true>(g, wx_half, i, sc, sf, 1, dv, sl);
+    out[i] = split_site(g, sc, sf, dv, sl, 0);
 }
 
-// Persistent form of the split-heights -> FP32 launch: each CTA walks tiles
-// gridDim.x apart; the next tile's heights are copied asynchronously into the
-// spare shared buffer while the current tile's gathers are in flight, so the
-// height round trip leaves the critical path. Same arithmetic as
-// k_gradient_split, so the same results bit for bit. Used with the x-filtered
-// store, where it measured faster (60.7 vs 63.8 us for 8 lines of 2^20
-// points); with the 16-tap gather it measured slower (86.2 vs 81.4 us).
-template <int kItems>
-__global__ void __launch_bounds__(kBS, QEW_SPLIT_MIN_CTAS)
-k_gradient_split_persist(const int *__restrict__ hc, const float *__restrict__ hf, SplitGeom g,
-                      float *__restrict__ grad, int count) {
-    constexpr int kTile = kBS * kItems;
-    __shared__ int s_c[2][kTile + 2];
-    __shared__ float s_f[2][kTile + 2];
-    __shared__ float s_dv[kTile + 1];
-    __shared__ float s_sl[kTile + 1];
+// The chunk of 32 kSteps - 1 sites from s0 on (k_gradient_split_walk). kInner:
+// every index below lies on the line.
+template <int kSteps, bool kInner>
+__device__ __forceinline__ void split_chunk(const int *__restrict__ hc, const float *__restrict__ hf,
+                                            const SplitGeom &g, float *__restrict__ out, int s0,
+                                            int lane) {
     const int n = g.n;
-    const int per_line = (n + kTile - 1) / kTile;
-    const int t = threadIdx.x;
-    // This CTA's tiles are blockIdx.x + k * gridDim.x in line-major order;
-    // their (line, index in line) advance by a fixed step, one division per CTA.
-    const int step_l = (int)gridDim.x / per_line;
-    const int step_i = (int)gridDim.x - step_l * per_line;
-    auto fetch = [&](int line, int idx, int buf) {  // heights of a tile (+ halo) into buffer buf
-        const int base = idx * kTile;
-        const int cnt = min(kTile, n - base);
-        const int *c = hc + (size_t)line * (size_t)n;
-        const float *f = hf + (size_t)line * (size_t)n;
+    const int e0 = s0 - 1 + lane;  // step k: edge e0 + 32 k, and the site at its right end
+    auto idx = [&](int i) { return kInner ? i : min(max(i, 0), n - 1); };  // clamped: unused
+    // heights at the edge's ends and at the next edge's right end
+    int c[kSteps][3];
+    float f[kSteps][3];
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const int j = t + k * kBS;
-            if (j < cnt) {
-                cp_async4(&s_c[buf][j + 1], c + base + j);
-                cp_async4(&s_f[buf][j + 1], f + base + j);
-            }
-        }
-        if (t == 0) {
-            const int site = base == 0 ? n - 1 : base - 1;
-            cp_async4(&s_c[buf][0], c + site);
-            cp_async4(&s_f[buf][0], f + site);
-        } else if (t == kBS - 1) {
-            const int site = (base + cnt == n) ? 0 : base + cnt;
-            cp_async4(&s_c[buf][cnt + 1], c + site);
-            cp_async4(&s_f[buf][cnt + 1], f + site);
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    };
-    float wx_half[4];
-    bsw_value_f(0.5f, wx_half);
-    int line = (int)blockIdx.x / per_line;
-    int idx = (int)blockIdx.x - line * per_line;
-    if (line < count) fetch(line, idx, 0);
-    for (int buf = 0; line < count; buf ^= 1) {
-        int nline = line + step_l, nidx = idx + step_i;
-        if (nidx >= per_line) {
-            nidx -= per_line;
-            ++nline;
-        }
-        const int base = idx * kTile;
-        const int cnt = min(kTile, n - base);
-        const int *sc = s_c[buf];
-        const float *sf = s_f[buf];
-        asm volatile("cp.async.wait_all;\n" ::: "memory");
-        // Barrier A: this tile's heights (every thread's copies) are in place,
-        // and every thread has left the previous tile, whose buffer (the
-        // other one) may now be refilled and whose edges may be rewritten.
-        __syncthreads();
-        if (nline < count) fetch(nline, nidx, buf ^ 1);
+    for (int k = 0; k < kSteps; ++k)
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const int j = t + k * kBS;
-            if (j < cnt) split_edge<true>(g, wx_half, base + j, sc, sf, j + 1, s_dv, s_sl);
+        for (int b = 0; b < 3; ++b) {
+            c[k][b] = __ldg(hc + idx(e0 + 32 * k + b));
+            f[k][b] = __ldg(hf + idx(e0 + 32 * k + b));
         }
-        if (t == kBS - 1)
-            split_edge<true>(g, wx_half, base == 0 ? n - 1 : base - 1, sc, sf, 0, s_dv, s_sl);
-        __syncthreads();  // barrier B: edges done
-        float *out = grad + (size_t)line * (size_t)n + base;
+#ifdef QEW_BOUNDS_CHECK
+    const size_t oob_n = (size_t)g.nx * (size_t)g.ny;
+#endif
+    // every step's midpoint and taps: 4 kSteps independent loads
+    float fm[kSteps], tap[kSteps][4], el[kSteps];  // el: second difference or slope
+    const unsigned row = 4u * (unsigned)g.nx;  // bytes; nx < 2^30
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            const int j = t + k * kBS;
-            if (j >= cnt) break;
-            __stcs(out + j, split_site(g, sc, sf, s_dv, s_sl, j));
+    for (int k = 0; k < kSteps; ++k) {
+        int cm;
+        split_mid(c[k][0], f[k][0], c[k][1], f[k][1], cm, fm[k]);
+        if ((unsigned)cm >= (unsigned)g.ny) cm = wrap_cell(cm, g.ny);
+        if (g.arc) {
+            const float dh = ((float)(c[k][1] - c[k][0]) + (f[k][1] - f[k][0])) * g.dy_over_dx;
+            el[k] = dh * rsqrtf(1.0f + dh * dh);
+        } else {
+            el[k] = split_d2(c[k], f[k]);
         }
-        line = nline;
-        idx = nidx;
+        const int e = e0 + 32 * k;
+        const char *E = (const char *)(g.edge + (kInner || (e >= 0 && e + 1 < n) ? e : 0));
+        const int y0 = (cm == 0 ? g.ny : cm) - 1;
+        const int y2 = cm + 1 == g.ny ? 0 : cm + 1;
+        const int y3 = y2 + 1 == g.ny ? 0 : y2 + 1;
+        const int y[4] = {y0, cm, y2, y3};
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            tap[k][b] = QEW_LDGP((const float *)(E + (unsigned long long)(unsigned)y[b] * row), g.edge,
+                                 oob_n, g.oob);
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    float dv[kSteps];
+#pragma unroll
+    for (int k = 0; k < kSteps; ++k) {
+        float dwy[4];
+        bsw_deriv_f(fm[k], dwy);
+        dv[k] = 0.0f;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) dv[k] += dwy[b] * tap[k][b];
+        dv[k] *= g.inv_dy_f;
+    }
+    // lane l's right edge is lane l + 1's, lane 31's lane 0's of the next step
+    auto next = [&](const float v[kSteps], int k) {
+        const float w = k + 1 < kSteps ? v[k + 1 < kSteps ? k + 1 : 0] : 0.0f;
+        return __shfl_sync(0xffffffffu, lane == 0 ? w : v[k], (lane + 1) & 31);
+    };
+#pragma unroll
+    for (int k = 0; k < kSteps; ++k) {
+        const int i = e0 + 32 * k + 1;
+        const float dvr = next(dv, k), elr = g.arc ? next(el, k) : 0.0f;
+        if ((kInner || (i > 0 && i + 1 < n)) && (k + 1 < kSteps || lane < 31))
+            __stcs(out + i, split_combine(g, el[k], el[k], elr, dv[k], dvr));
+    }
+}
+
+// Split heights -> FP32 gradient on the x-filtered store. A warp takes a chunk
+// of 32 kSteps - 1 sites: step k's lanes take edges 32 k + lane in order (so
+// every load and store is coalesced) and the steps' gathers are in flight
+// together. No shared memory and no barrier: with tiles of 256 threads the two
+// barriers and the extra edge that one thread took alone left the gathers
+// waiting: 57.2 us for 8 lines of 2^20 points, now 49.2 (0.77 of the measured
+// copy rate on the bytes that DRAM moves; the rest is gather latency at 63 % of
+// the issue slots); a line of 1024 points 7.0 -> 5.3 us. Same arithmetic as
+// k_gradient_split, so the same results bit for bit.
+template <int kSteps, int kMin>
+__global__ void __launch_bounds__(kBS, kMin)
+k_gradient_split_walk(const int *__restrict__ hc, const float *__restrict__ hf,
+                      const __grid_constant__ SplitGeom g, float *__restrict__ grad, int chunks,
+                      long long units) {
+    constexpr int kSites = 32 * kSteps - 1;
+    const int n = g.n;
+    const int lane = threadIdx.x & 31;
+    const long long u = (long long)blockIdx.x * (kBS / 32) + (threadIdx.x >> 5);
+    if (u >= units) return;
+    const int line = (int)(u / chunks);
+    const int s0 = (int)(u - (long long)line * chunks) * kSites;
+    const size_t off = (size_t)line * (size_t)n;
+    hc += off;
+    hf += off;
+    float *out = grad + off;
+    if (s0 > 0 && s0 <= n - 1 - 32 * kSteps) {
+        split_chunk<kSteps, true>(hc, hf, g, out, s0, lane);
+        return;
+    }
+    split_chunk<kSteps, false>(hc, hf, g, out, s0, lane);
+    if (s0 == 0 && lane == 0) split_site_wrap(g, hc, hf, out, 0);
+    if (s0 + kSites >= n && lane == 1) split_site_wrap(g, hc, hf, out, n - 1);
 }
 
 __global__ void k_split_heights(const double *__restrict__ h, int n, double dy, double inv_dy,
@@ -443,32 +473,37 @@ SplitGeom qew_split_geom(const qew_field *f, int n, const qew_params *p) {
 // Split heights in, FP32 gradient out, `count` lines n apart.
 static qew_status split_launch(qew_ctx *ctx, const SplitGeom &g, int count, const int32_t *d_cell,
                                const float *d_frac, float *d_grad, const char *what) {
-    if (g.edge) {  // persistent CTAs, the launch shape chosen by the autotuner
-        // Candidates: sites per thread {1, 2} x resident CTAs per SM {4, 6, 8};
-        // the per-site arithmetic does not depend on them, so every candidate
-        // gives the same bits. Hand-chosen default: 2 sites x 8 CTAs.
-        static const char *const names[6] = {"1 site x 4 CTA/SM", "1 site x 6 CTA/SM",
-                                              "1 site x 8 CTA/SM", "2 sites x 4 CTA/SM",
-                                              "2 sites x 6 CTA/SM", "2 sites x 8 CTA/SM"};
-        auto launch = [&](int c) -> qew_status {
-            const int items = 1 + c / 3;
-            const int ctas = 4 + 2 * (c % 3);
-            const long long tiles =
-                (long long)((g.n + kBS * items - 1) / (kBS * items)) * count;
-            if (tiles > INT_MAX)
+    if (g.edge && g.nx < (1 << 30)) {  // chunks of a warp, the launch shape chosen by the autotuner
+        // Candidates: steps a chunk x registers for so many resident CTAs per
+        // SM; the per-site arithmetic does not depend on them, so every
+        // candidate gives the same bits. On 8 lines of 2^20 points: 67.0, 52.8,
+        // 49.7, 50.4, 49.1 and 49.2 us.
+        static const char *const names[6] = {"2 steps, 5 CTA/SM", "2 steps, 6 CTA/SM",
+                                              "2 steps, 8 CTA/SM", "3 steps, 5 CTA/SM",
+                                              "4 steps, 4 CTA/SM", "4 steps, 5 CTA/SM"};
+        auto launch_as = [&](auto kern, int steps) -> qew_status {
+            const int sites = 32 * steps - 1;
+            const int chunks = (g.n + sites - 1) / sites;
+            const long long units = (long long)chunks * count;
+            const long long blocks = (units + kBS / 32 - 1) / (kBS / 32);
+            if (blocks > INT_MAX)
                 return qew_fail(ctx, QEW_ERR_INVALID, "%s: more than 2^31 tiles", what);
-            const int grid = (int)std::min<long long>(tiles, (long long)ctas * ctx->num_sms);
-            if (items == 1)
-                k_gradient_split_persist<1><<<grid, kBS, 0, ctx->stream>>>(d_cell, d_frac, g,
-                                                                           d_grad, count);
-            else
-                k_gradient_split_persist<2><<<grid, kBS, 0, ctx->stream>>>(d_cell, d_frac, g,
-                                                                           d_grad, count);
+            kern<<<(unsigned)blocks, kBS, 0, ctx->stream>>>(d_cell, d_frac, g, d_grad, chunks, units);
             return qew_launch_check(ctx, what);
         };
-        int cand = 5;
+        auto launch = [&](int c) -> qew_status {
+            switch (c) {
+            case 0: return launch_as(k_gradient_split_walk<2, 5>, 2);
+            case 1: return launch_as(k_gradient_split_walk<2, 6>, 2);
+            case 2: return launch_as(k_gradient_split_walk<2, 8>, 2);
+            case 3: return launch_as(k_gradient_split_walk<3, 5>, 3);
+            case 4: return launch_as(k_gradient_split_walk<4, 4>, 4);
+            default: return launch_as(k_gradient_split_walk<4, 5>, 4);
+            }
+        };
+        int cand = 4;
         QEW_TRY(qew_tune_pick(ctx, kTuneGradientSplit,
-                              qew_tune_class((long long)g.n * count, g.arc), 6, 5, names, launch,
+                              qew_tune_class((long long)g.n * count, g.arc), 6, 4, names, launch,
                               &cand));
         return launch(cand);
     } else {
