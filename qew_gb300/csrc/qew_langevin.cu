@@ -163,9 +163,11 @@ k_langevin_run(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, dou
 // computed by both neighbouring CTAs. One grid barrier per round.
 //
 // A step is a chain of latencies (locate, gather, the integer products, the
-// combine), so a thread takes one edge and one site, and the first half of
-// the threads a pair of increments each (consecutive pairs, so that no lane
-// of their warps idles).
+// combine), so a thread takes one edge and one site, and half of the threads a
+// pair of increments each (consecutive pairs, so that no lane of their warps
+// idles; from the last thread down, so that on a short region the increments
+// and the edges fall to different warps: 4096 sites 4.5 -> 3.7 us a step in
+// FP64, 2.7 -> 2.4 in FP32, 65536 sites 6.3 -> 5.5 and 4.2 -> 4.0).
 //
 // Shared memory, in doubles of the region R = seg + 2K: heights (two
 // buffers), edge values, arclength slopes, increments.
@@ -214,7 +216,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
                 if (b > 0) {
                     if ((n & 1) == 0) {  // pairs at every second position, across the ring's end too
                         const int q0 = lo - ((g0 + lo) & 1);
-                        for (int r = q0 + 2 * t; r < hi; r += 2 * kTbBS) {
+                        for (int r = q0 + 2 * (kTbBS - 1 - t); r < hi; r += 2 * kTbBS) {
                             const uint32_t pair = (uint32_t)(gsite(r) >> 1);
                             double z0, z1;
                             if (NORMAL32)
@@ -225,7 +227,7 @@ k_langevin_run_tb(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, 
                             zz[r + 1] = z1;  // r + 1 <= hi <= RS - 1
                         }
                     } else {
-                        for (int r = lo + t; r < hi; r += kTbBS) {
+                        for (int r = lo + kTbBS - 1 - t; r < hi; r += kTbBS) {
                             const int g = gsite(r);
                             if ((g & 1) && r != lo) continue;  // its pair's first site wrote it
                             double z0, z1;
@@ -473,8 +475,8 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
         const int cls = qew_tune_class(n, (kN32 ? 1 : 0) + (model == QEW_MODEL_ARCLENGTH ? 2 : 0) +
                                               (reads_poly_store(nz) ? 4 : 0));
         // Default from measurement at L = 65536 (us a step): K = 16 steps per
-        // barrier at 2 CTAs per SM, FP64 6.2 against 10.9 with one barrier per
-        // step, FP32 4.0 against 7.9. A tuned shape must be 5 % faster than the
+        // barrier at 2 CTAs per SM, FP64 5.5 against 10.9 with one barrier per
+        // step, FP32 3.9 against 7.9. A tuned shape must be 5 % faster than the
         // default on the probe.
         const int dflt = 5;
         int cand = dflt;
