@@ -23,7 +23,7 @@
 //     are advanced from them.
 //   * a trial evaluates energy and dV/dy from one gather, so an accepted trial
 //     needs no second one.
-// One line of 4096 points (preconditioned, m = 10, 16 CTAs): 10.4-13.8 -> 3.1 ms
+// One line of 4096 points (preconditioned, m = 10, 16 CTAs): 10.4-15.1 -> 2.5 ms
 // a solve, 52 k cycles an iteration, most of them latencies: the two
 // recurrences 8 k, the products 12 k, the trial 10 k. 768 lines of 256 to 4096
 // points on all SMs: 68 -> 45 ms (two CTAs of 256 threads an SM; the long
@@ -433,7 +433,7 @@ __device__ qew_lbfgs_result lbfgs_gram(Team &T, const Noise &nz, double *__restr
             const double x1 = k + 1 < cnt ? fma(alpha, d[at(k + 1)], h[p0 + k + 1]) : fma(alpha, dr, hr);
             const int e = p0 + k, ep = e + 1 == n ? 0 : e + 1;
             double v, dv;
-            noise_both_edge(nz, e, (double)(e + ep) * 0.5 * L.dx, x0 + x1, v, dv);
+            noise_both_edge(nz, e, EdgeX{e + ep, L.dx}, x0 + x1, v, dv);
             const double dh = (x1 - x0) * L.inv_dx;
             double el;
             if (arc) {

@@ -8,7 +8,8 @@
 // a batch share the launch. Short lines are bound by one chain of latencies
 // (heights, stencil rows, the integer products, the combine), long ones by the
 // issue of the gather. (With BS sites a CTA, thread 0 took the extra edge after
-// its own and the whole warp waited: 8.2 us a call at 1024 points, now 6.2;
+// its own and the whole warp waited: 8.2 us a call at 1024 points, 6.2 with one each and 5.2
+// since the wrap edge takes constant weights;
 // three lines of 100003 points 42.9 -> 20.5 us with one launch for all.)
 //
 // objective: the per-edge energy (qew_model.h:61-83) reduced by a fixed

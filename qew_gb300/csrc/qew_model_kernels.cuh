@@ -29,7 +29,7 @@ __device__ __forceinline__ double edge_energy(const Noise &nz, int i, int ip, do
         line_energy = lt * dh_dx * dh_dx * 0.5;
     else
         line_energy = lt * (sqrt(__dadd_rn(1.0, __dmul_rn(dh_dx, dh_dx))) - 1.0);
-    const double xc = (double)(i + ip) * 0.5 * L.dx;
+    const EdgeX xc{i + ip, L.dx};
     return L.dx * __dsub_rn(__dadd_rn(line_energy, noise_value_edge(nz, i, xc, hip + hi)),
                             __dmul_rn(f, hi));
 }
@@ -45,7 +45,7 @@ __device__ __forceinline__ void edge_gradient(const Noise &nz, int e, int n, dou
                                               double hep, const LineDx &L, bool arc, double &dv,
                                               double &sl) {
     const int ep = (e + 1 == n) ? 0 : e + 1;
-    const double xc = (double)(e + ep) * 0.5 * L.dx;
+    const EdgeX xc{e + ep, L.dx};
     dv = noise_dvdy_edge(nz, e, xc, hep + he);
     sl = 0.0;
     if (arc) {

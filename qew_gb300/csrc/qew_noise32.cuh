@@ -140,20 +140,30 @@ struct NoiseSplit32 {
         loc_y(y, iy, fy);
         return (double)(taps(ix, fx, iy, fy, true) * inv_dy_f);
     }
-    // At the midpoint a / 2 of edge e (xc its physical x).
-    __device__ __forceinline__ double value_edge_sum(int e, double xc, double a) const {
-        if (!xconst || e + 1 >= nx) return value(xc, a * 0.5);
-        int iy;
-        float fy;
-        loc_y_sum(a, iy, fy);
-        return (double)(edge ? taps_edge(e, iy, fy, false) : taps(e, 0.5f, iy, fy, false));
+    // Whether edge e sits at x fraction 1/2 of a column, which e becomes: the
+    // wrap edge (at x = (n - 1) dx / 2) does when nx is even.
+    __device__ __forceinline__ bool half_column(int &e, bool &wrap) const {
+        wrap = e + 1 >= nx;
+        if (!xconst || (wrap && (nx & 1))) return false;
+        if (wrap) e = (nx >> 1) - 1;
+        return true;
     }
-    __device__ __forceinline__ double dvdy_edge_sum(int e, double xc, double a) const {
-        if (!xconst || e + 1 >= nx) return dvdy(xc, a * 0.5);
+    // At the midpoint a / 2 of edge e (xc its physical x).
+    __device__ __forceinline__ double value_edge_sum(int e, EdgeX xc, double a) const {
+        bool wrap;
+        if (!half_column(e, wrap)) return value(xc, a * 0.5);
         int iy;
         float fy;
         loc_y_sum(a, iy, fy);
-        const float t = edge ? taps_edge(e, iy, fy, true) : taps(e, 0.5f, iy, fy, true);
+        return (double)(edge && !wrap ? taps_edge(e, iy, fy, false) : taps(e, 0.5f, iy, fy, false));
+    }
+    __device__ __forceinline__ double dvdy_edge_sum(int e, EdgeX xc, double a) const {
+        bool wrap;
+        if (!half_column(e, wrap)) return dvdy(xc, a * 0.5);
+        int iy;
+        float fy;
+        loc_y_sum(a, iy, fy);
+        const float t = edge && !wrap ? taps_edge(e, iy, fy, true) : taps(e, 0.5f, iy, fy, true);
         return (double)(t * inv_dy_f);
     }
     __device__ __forceinline__ void sample(double x, double y, double &v, double &a,
@@ -169,11 +179,11 @@ __device__ __forceinline__ unsigned long long *qew_noise_oob(const NoiseSplit32 
     return nz.oob;
 }
 #endif
-__device__ __forceinline__ double noise_dvdy_edge(const NoiseSplit32 &nz, int e, double xc,
+__device__ __forceinline__ double noise_dvdy_edge(const NoiseSplit32 &nz, int e, EdgeX xc,
                                                   double a) {
     return nz.dvdy_edge_sum(e, xc, a);
 }
-__device__ __forceinline__ double noise_value_edge(const NoiseSplit32 &nz, int e, double xc,
+__device__ __forceinline__ double noise_value_edge(const NoiseSplit32 &nz, int e, EdgeX xc,
                                                    double a) {
     return nz.value_edge_sum(e, xc, a);
 }

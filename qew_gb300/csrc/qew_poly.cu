@@ -45,7 +45,7 @@ struct PolyGeom {
 // the kernels' loops.
 __device__ __noinline__ double walk_edge_rare(const PolyGeom &g, int e, double sum) {
     const int ep = (e + 1 == g.n) ? 0 : e + 1;
-    return g.nz.dvdy_edge_sum(e, (double)(e + ep) * 0.5 * g.L.dx, sum);
+    return g.nz.dvdy_edge_sum(e, EdgeX{e + ep, g.L.dx}, sum);
 }
 
 // 8-byte asynchronous global -> shared copy.

@@ -55,8 +55,7 @@ __device__ __forceinline__ double rk_site_velocity(const Noise &nz, int i, int n
                                                    double hl, double hr) {
     const int im = (i == 0) ? n - 1 : i - 1;
     const int ip = (i + 1 == n) ? 0 : i + 1;
-    const double xcl = (double)(im + i) * 0.5 * L.dx;
-    const double xcr = (double)(i + ip) * 0.5 * L.dx;
+    const EdgeX xcl{im + i, L.dx}, xcr{i + ip, L.dx};
     const double dvl = noise_dvdy_edge(nz, im, xcl, __dadd_rn(hl, hi));  // edge (im, i)
     const double dvr = noise_dvdy_edge(nz, i, xcr, __dadd_rn(hi, hr));   // edge (i, ip)
     return rk_velocity_of<Noise>(dvl, dvr, L, lt, f, model, hi, hl, hr);
@@ -221,7 +220,7 @@ __device__ __forceinline__ double rk_site_velocity_pair(const Noise &nz, int i, 
                                                         int lane, unsigned pmask) {
     const int im = (i == 0) ? n - 1 : i - 1;
     const int ip = (i + 1 == n) ? 0 : i + 1;
-    const double xc = lane ? (double)(i + ip) * 0.5 * L.dx : (double)(im + i) * 0.5 * L.dx;
+    const EdgeX xc{lane ? i + ip : im + i, L.dx};
     const double mine =
         noise_dvdy_edge(nz, lane ? i : im, xc, lane ? __dadd_rn(hi, hr) : __dadd_rn(hl, hi));
     const double other = __shfl_xor_sync(pmask, mine, 1);
@@ -347,11 +346,11 @@ struct RkPlace {
     bool cst;
     FxFrac fx;
 };
-__device__ __forceinline__ bool rk_place(const NoiseBSpline64 &nz, RkPlace &q, int e, double xc,
+__device__ __forceinline__ bool rk_place(const NoiseBSpline64 &nz, RkPlace &q, int e, EdgeX xc,
                                          double a) {
     FxFrac t;
     q.e = e;
-    q.cst = nz.fx_const(e);
+    q.cst = nz.fx_const(q.e);
     if (!nz.fx_row(a, q.iy, t)) return false;
     return q.cst || nz.fx_locate(xc, nz.dx, nz.inv_dx, nz.kx, nz.nx, q.e, q.fx);
 }
@@ -425,7 +424,7 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
     auto votes = [&](bool b) { return (__ballot_sync(gmask, b) >> shift) & all; };
     RkFast F;
     const int im = (i == 0) ? n - 1 : i - 1, ip = (i + 1 == n) ? 0 : i + 1;
-    const double xl = (double)(im + i) * 0.5 * L.dx, xr = (double)(i + ip) * 0.5 * L.dx;
+    const EdgeX xl{im + i, L.dx}, xr{i + ip, L.dx};
     F.hl = hl;
     F.hr = hr;
     F.slope0 = (float)(-2.0 * L.c_el);
