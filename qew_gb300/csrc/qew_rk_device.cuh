@@ -516,8 +516,12 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
                     (float)fabs(L.fdx)) +
         400.0f * (float)(L.half_dx * fmax(nz.fx_dv_c, nz.fx_dv_g));
     const double g = (double)(3.0f * eps / smin) + 4.0 * ulp + 4.0e-7 * gap;
-    const long long z0 = __double_as_longlong(z - g), z1 = __double_as_longlong(z + g);
-    if (!(z0 > bl && z1 < bh)) return false;
+    // v > 0 up to z0, v <= 0 from z1 on; the bracket's own ends are known. (A
+    // site within its rounding of the zero, z0 <= bl, is what a line near its
+    // critical force is made of.)
+    if (!(z + g > 0.0)) return false;
+    const long long zl = __double_as_longlong(z - g), zh = __double_as_longlong(z + g);
+    const long long z0 = min(max(zl, bl), bh - 1), z1 = max(min(zh, bh), z0);
     // levels across a binade's end, as the serial loop takes them
     int k0 = 0;
     for (; k0 < 60 && (int)(bh >> 52) != (int)(bl >> 52); ++k0) {
