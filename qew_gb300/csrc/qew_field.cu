@@ -183,7 +183,7 @@ __global__ void k_sample(Noise nz, const double *__restrict__ x, const double *_
 // (|z| < 8.58 from 53-bit uniforms), so it and the taps lose nothing, and a
 // tap pair costs four 32 x 32 + 64-bit multiply-adds (about 5 cycles each) where
 // FP64 takes two 64-cycle instructions: 306 -> 150 us an axis of a 4096 x 1024
-// field at xi = 4 (41 taps). A sample is X = X1 2^30 + X0 in units 2^-F,
+// field at xi = 4 (41 taps), 115 with four outputs a thread. A sample is X = X1 2^30 + X0 in units 2^-F,
 // |X| < 2^59; a tap T = T1 2^30 + T0 in units 2^-q, q such that the taps'
 // sum is at most 2^58.
 constexpr double kNoiseMax = 8.58;  // sqrt(2 ln 2^53) = 8.572
@@ -192,7 +192,7 @@ __global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_
     const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
     const int pairs = (ny + 1) / 2;
     if (tid >= (long)nx * pairs) return;
-    const int i = (int)(tid / pairs), jp = (int)(tid % pairs);
+    const int i = (int)(tid % nx), jp = (int)(tid / nx);
     uint32_t c[4] = {(uint32_t)jp, 0u, (uint32_t)i, 0u};
     philox4x32_10(c, seed);
     const uint64_t a = ((((uint64_t)c[0]) << 32) | c[1]) >> 11;
@@ -201,75 +201,115 @@ __global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_
     int k;
     fx_normal_pair(a + 1, b, g_fx_logs, g_fx_turns, z0, z1, k);  // z 2^k, k <= -F
     const int sh = min(-k - F, 63);
-    w[(size_t)i * ny + 2 * jp] = z0 >> sh;
-    if (2 * jp + 1 < ny) w[(size_t)i * ny + 2 * jp + 1] = z1 >> sh;
+    w[(size_t)(2 * jp) * nx + i] = z0 >> sh;  // [ny][nx]
+    if (2 * jp + 1 < ny) w[(size_t)(2 * jp + 1) * nx + i] = z1 >> sh;
 }
 
-// out[i][j] = sum_k taps[k] * in[(i + k - R) mod nx][j]   (axis 0), or along j
-// (axis 1); symmetric taps, tap[k] for distance k. The partial products of
-// weight 2^60, 2^30 and 1 have sums of their own, the lower two folded every
-// four pairs before they can overflow (2^61 a pair). kLast: FP64 out, times
-// 2^exp; else fixed point again, shifted right by exp.
-template <bool kLast>
+// out[p] = sum_k tap[|k|] in[p + k] along the slow axis of in[len][width] (both
+// periodic, symmetric taps, radius R), lanes along the fast one. kLast: FP64 out
+// in the same layout, times 2^exp; else fixed point, shifted right by exp, as
+// out[width][len], so that the other axis is the slow one next.
+// The partial products of weight 2^60, 2^30 and 1 have sums of their own, the
+// lower two folded every four pairs before they can overflow (2^61 a pair).
+// A thread takes 4 consecutive outputs: a step in k then needs two new samples
+// for the four (they slide through registers, split into their 30-bit halves
+// once) where an output alone loads and splits both ends of every pair; what
+// is left is 4 wide multiply-adds a pair.
+template <bool kLast, int kOut>
 __global__ void __launch_bounds__(256)
-k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int nx, int ny,
-             const int2 *__restrict__ tap, int R, int axis, int exp) {
-    const long tid = blockIdx.x * 256l + threadIdx.x;
-    if (tid >= (long)nx * ny) return;
-    const int i = (int)(tid / ny), j = (int)(tid - (long)i * ny);
-    const int n = axis ? ny : nx, at = axis ? j : i;
-    const long st = axis ? 1 : ny;
-    const long long *line = in + (axis ? (size_t)i * ny : (size_t)j);
-    long long P = 0, M = 0, A = 0;
-    unsigned long long L = 0;
-    auto add = [&](int x1, int x0, int2 t) {
-        P += (long long)x1 * t.x;
-        M += (long long)x1 * t.y;
-        M += (long long)x0 * t.x;  // x0 < 2^31
-        L += (unsigned long long)(unsigned)x0 * (unsigned)t.y;
+k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int len, int width,
+             const int2 *__restrict__ tap, int R, int exp, int lsh) {
+    // a block is 2^lsh lanes wide and 256 / 2^lsh threads along the slow axis,
+    // whose windows overlap in L1
+    const unsigned tiles = ((unsigned)width + (1u << lsh) - 1u) >> lsh;
+    const unsigned row = blockIdx.x / tiles;
+    const int l = (int)((blockIdx.x - row * tiles) << lsh) + (int)(threadIdx.x & ((1u << lsh) - 1u));
+    const long long pl = (((long long)row << (8 - lsh)) + (threadIdx.x >> lsh)) * kOut;
+    if (l >= width || pl >= len) return;
+    const int p0 = (int)pl;
+    constexpr int kLow = (1 << 30) - 1;
+    int a1[kOut], a0[kOut], b1[kOut], b0[kOut];  // samples at p0 + u - k and p0 + u + k
+    auto get = [&](int p, int &x1, int &x0) {
+        const long long x = __ldg(in + (size_t)p * (size_t)width + l);
+        x1 = (int)(x >> 30);
+        x0 = (int)x & kLow;
+    };
+    long long P[kOut], M[kOut], A[kOut];
+    unsigned long long L[kOut];
+    auto add = [&](int u, int x1, int x0, int2 t) {
+        P[u] += (long long)x1 * t.x;
+        M[u] += (long long)x1 * t.y;
+        M[u] += (long long)x0 * t.x;  // x0 < 2^31
+        L[u] += (unsigned long long)(unsigned)x0 * (unsigned)t.y;
     };
     auto fold = [&]() {
-        A += (M >> 14) + (long long)(L >> 44);
-        M = 0;
-        L = 0;
-    };
-    constexpr int kLow = (1 << 30) - 1;
-    {
-        const long long x = line[(long)at * st];
-        add((int)(x >> 30), (int)x & kLow, __ldg(tap));
-    }
-    if (at >= R && at + R < n) {
-        const long long *lo = line + (long)at * st, *hi = lo;
-        for (int k0 = 1; k0 <= R; k0 += 4) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int k = k0 + u;
-                if (k > R) break;
-                lo -= st;
-                hi += st;
-                const long long a = *lo, b = *hi;
-                add((int)(a >> 30) + (int)(b >> 30), ((int)a & kLow) + ((int)b & kLow),
-                    __ldg(tap + k));
+        for (int u = 0; u < kOut; ++u) {
+            A[u] += (M[u] >> 14) + (long long)(L[u] >> 44);
+            M[u] = 0;
+            L[u] = 0;
+        }
+    };
+    {
+        const int2 t = __ldg(tap);
+        int p = p0;
+#pragma unroll
+        for (int u = 0; u < kOut; ++u) {
+            P[u] = M[u] = A[u] = 0;
+            L[u] = 0;
+            get(p, a1[u], a0[u]);
+            b1[u] = a1[u];
+            b0[u] = a0[u];
+            add(u, a1[u], a0[u], t);
+            p = p + 1 == len ? 0 : p + 1;
+        }
+    }
+    int pa = p0, pb = (int)((pl + kOut - 1) % len);
+    for (int k0 = 1; k0 <= R; k0 += 4) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (k0 + q > R) break;
+            pa = pa == 0 ? len - 1 : pa - 1;
+            pb = pb + 1 == len ? 0 : pb + 1;
+#pragma unroll
+            for (int u = kOut - 1; u > 0; --u) {
+                a1[u] = a1[u - 1];
+                a0[u] = a0[u - 1];
             }
-            fold();
+#pragma unroll
+            for (int u = 0; u < kOut - 1; ++u) {
+                b1[u] = b1[u + 1];
+                b0[u] = b0[u + 1];
+            }
+            get(pa, a1[0], a0[0]);
+            get(pb, b1[kOut - 1], b0[kOut - 1]);
+            const int2 t = __ldg(tap + k0 + q);
+#pragma unroll
+            for (int u = 0; u < kOut; ++u) add(u, a1[u] + b1[u], a0[u] + b0[u], t);
         }
-    } else {
-        int kl = at, kh = at;
-        for (int k = 1; k <= R; ++k) {
-            kl = (kl == 0) ? n - 1 : kl - 1;
-            kh = (kh + 1 == n) ? 0 : kh + 1;
-            const long long a = line[(long)kl * st], b = line[(long)kh * st];
-            add((int)(a >> 30) + (int)(b >> 30), ((int)a & kLow) + ((int)b & kLow),
-                __ldg(tap + k));
-            if ((k & 3) == 0) fold();
-        }
+        fold();
     }
     fold();
-    const long long v = (P << 5) + (A >> 11);  // units of 2^55
-    if (kLast)
-        ((double *)out)[tid] = fx_to_double(v, exp);
-    else
-        ((long long *)out)[tid] = v >> exp;
+    long long v[kOut];
+#pragma unroll
+    for (int u = 0; u < kOut; ++u) v[u] = (P[u] << 5) + (A[u] >> 11);  // units of 2^55
+    const int cnt = min(kOut, len - p0);
+    if (kLast) {
+        double *o = (double *)out + (size_t)p0 * (size_t)width + l;
+#pragma unroll
+        for (int u = 0; u < kOut; ++u)
+            if (u < cnt) o[(size_t)u * (size_t)width] = fx_to_double(v[u], exp);
+    } else {
+        long long *o = (long long *)out + (size_t)l * (size_t)len + p0;
+        if (kOut == 4 && cnt == kOut && (len & 1) == 0) {  // 16-byte aligned: p0 is a multiple of 4
+            ((longlong2 *)o)[0] = make_longlong2(v[0] >> exp, v[1 % kOut] >> exp);
+            ((longlong2 *)o)[1] = make_longlong2(v[2 % kOut] >> exp, v[3 % kOut] >> exp);
+        } else {
+#pragma unroll
+            for (int u = 0; u < kOut; ++u)
+                if (u < cnt) o[u] = v[u] >> exp;
+        }
+    }
 }
 
 // Population mean and std of n values in two passes (the second about the
@@ -534,10 +574,31 @@ qew_status qew_field_create_generated(qew_ctx *ctx, int nx, int ny, double Lx, d
     if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
     const long pairs = (long)nx * ((ny + 1) / 2);
     k_white_noise<<<(unsigned)((pairs + 255) / 256), 256, 0, ctx->stream>>>(w, nx, ny, seed, F1);
-    const unsigned blocks = (unsigned)((N + 255) / 256);
-    // a filtered sum is in units of 2^(55 - F - q) (k_gauss_conv)
-    k_gauss_conv<false><<<blocks, 256, 0, ctx->stream>>>(w, t, nx, ny, tapy, Ry, 1, F1 + qy - 55 - F2);
-    k_gauss_conv<true><<<blocks, 256, 0, ctx->stream>>>(t, w, nx, ny, tapx, Rx, 0, 55 - F2 - qx);
+    // a filtered sum is in units of 2^(55 - F - q) (k_gauss_conv); w [ny][nx] ->
+    // t [nx][ny] -> w [nx][ny]
+    // one output a thread where four would idle threads (len < 4) or scatter
+    // the lanes' loads (a field of few columns): 2^20 x 1 at xi = 3 386 us so,
+    // 488 with four; 2^18 x 8 314 with four, 341 so
+    auto conv = [&](auto last, auto outs, const long long *in, void *out, int len, int width,
+                    const int2 *tap, int R, int exp) {
+        constexpr int kOut = decltype(outs)::value;
+        int lsh = 0;  // 32 lanes along the fast axis, fewer only on a narrower field
+        while (lsh < 5 && (1 << lsh) < width) ++lsh;
+        const long long tiles = ((long long)width + (1 << lsh) - 1) >> lsh;
+        const long long per = (long long)kOut << (8 - lsh);
+        k_gauss_conv<decltype(last)::value, kOut>
+            <<<(unsigned)(tiles * ((len + per - 1) / per)), 256, 0, ctx->stream>>>(
+                in, out, len, width, tap, R, exp, lsh);
+    };
+    using One = std::integral_constant<int, 1>;
+    using Four = std::integral_constant<int, 4>;
+    if (ny >= 4 && nx >= 4) {
+        conv(std::false_type{}, Four{}, w, t, ny, nx, tapy, Ry, F1 + qy - 55 - F2);
+        conv(std::true_type{}, Four{}, t, w, nx, ny, tapx, Rx, 55 - F2 - qx);
+    } else {
+        conv(std::false_type{}, One{}, w, t, ny, nx, tapy, Ry, F1 + qy - 55 - F2);
+        conv(std::true_type{}, One{}, t, w, nx, ny, tapx, Rx, 55 - F2 - qx);
+    }
     qew_status st = qew_launch_check(ctx, "field_generate", 3);
     if (st != QEW_OK) return cleanup(st);
     st = field_moments(ctx, (const double *)w, N, amplitude, stat);
