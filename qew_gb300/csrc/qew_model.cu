@@ -69,24 +69,6 @@ const void *mapped_host_address(const void *ptr) {
 
 }  // namespace
 
-// Host-buffer gradients without copies: when both host buffers are mapped
-// (pinned) host memory, the kernels read the heights and write the
-// gradients through the host link themselves (NVLink-C2C on Grace-based
-// systems), so the transfer and the gather overlap inside one launch.
-// QEW_ERR_UNSUPPORTED (nothing done) when either buffer is pageable or not
-// 8-byte aligned.
-static qew_status gradient_mapped(qew_ctx *ctx, const qew_field *field, int count,
-                                  const double *h_h, int n, const qew_params *p, int precision,
-                                  double *h_grad) {
-    if (((uintptr_t)h_h | (uintptr_t)h_grad) & 7u) return QEW_ERR_UNSUPPORTED;
-    const double *dh = (const double *)mapped_host_address(h_h);
-    double *dg = (double *)mapped_host_address(h_grad);
-    if (!dh || !dg) return QEW_ERR_UNSUPPORTED;
-    QEW_TRY(qew_gradient_batch(ctx, field, count, dh, n, p, precision, dg));
-    QEW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return QEW_OK;
-}
-
 // Lines k = 0..count-1, n apart, on the FP64 gathers: one launch for up to
 // 65535 of them.
 static qew_status gradient_fp64(qew_ctx *ctx, const qew_field *field, int count, const double *d_h,
@@ -109,7 +91,7 @@ static qew_status gradient_fp64(qew_ctx *ctx, const qew_field *field, int count,
 
 static qew_status gradient_enqueue(qew_ctx *ctx, const qew_field *field, int count,
                                    const double *d_h, int n, const qew_params *p, int precision,
-                                   double *d_grad) {
+                                   double *d_grad, bool host_grad = false) {
     if (precision == QEW_PREC_FP32_SPLIT) {
         if (field->kind != QEW_FIELD_BSPLINE || !field->coef32)
             return qew_fail(ctx, QEW_ERR_INVALID,
@@ -122,10 +104,29 @@ static qew_status gradient_enqueue(qew_ctx *ctx, const qew_field *field, int cou
     if (precision != QEW_PREC_FP64 && precision != QEW_PREC_FP64_REFERENCE)
         return qew_fail(ctx, QEW_ERR_INVALID, "gradient: unknown precision %d", precision);
     if (precision == QEW_PREC_FP64) {  // the cell-polynomial store, when it serves this line
-        const qew_status s = qew_gradient_poly_enqueue(ctx, field, count, d_h, n, p, d_grad);
+        const qew_status s = qew_gradient_poly_enqueue(ctx, field, count, d_h, n, p, d_grad, host_grad);
         if (s != QEW_ERR_UNSUPPORTED) return s;
     }
     return gradient_fp64(ctx, field, count, d_h, n, p, precision, d_grad);
+}
+
+// Host-buffer gradients without copies: when both host buffers are mapped
+// (pinned) host memory, the kernels read the heights and write the
+// gradients through the host link themselves (NVLink-C2C on Grace-based
+// systems), so the transfer and the gather overlap inside one launch.
+// QEW_ERR_UNSUPPORTED (nothing done) when either buffer is pageable or not
+// 8-byte aligned.
+static qew_status gradient_mapped(qew_ctx *ctx, const qew_field *field, int count,
+                                  const double *h_h, int n, const qew_params *p, int precision,
+                                  double *h_grad) {
+    if (((uintptr_t)h_h | (uintptr_t)h_grad) & 7u) return QEW_ERR_UNSUPPORTED;
+    if (!field || !p) return qew_fail(ctx, QEW_ERR_INVALID, "gradient_host: bad arguments");
+    const double *dh = (const double *)mapped_host_address(h_h);
+    double *dg = (double *)mapped_host_address(h_grad);
+    if (!dh || !dg) return QEW_ERR_UNSUPPORTED;
+    QEW_TRY(gradient_enqueue(ctx, field, count, dh, n, p, precision, dg, true));
+    QEW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    return QEW_OK;
 }
 
 qew_status qew_gradient_enqueue(qew_ctx *ctx, const qew_field *field, const double *d_h, int n,

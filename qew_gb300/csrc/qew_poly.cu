@@ -181,39 +181,33 @@ __device__ __forceinline__ long long lane_next(long long v, long long wrap, int 
 }
 
 // Gradient of site i from FP64 sums and edges.
-__device__ __noinline__ void walk_site_rare(const PolyGeom &g, const double *hl, double *out, int i) {
+__device__ __noinline__ double walk_site_rare(const PolyGeom &g, const double *hl, int i) {
     const int n = g.n;
     const int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
     const double hm = __ldg(hl + im), h0 = __ldg(hl + i), hp = __ldg(hl + ip);
     const double dvl = walk_edge_rare(g, im, hm + h0), dvr = walk_edge_rare(g, i, h0 + hp);
-    __stcs(out + i, site_gradient<NoiseBSpline64>(hm, h0, hp, dvl, dvr, 0.0, 0.0, g.L, g.lt, 0.0,
-                                                  false));
+    return site_gradient<NoiseBSpline64>(hm, h0, hp, dvl, dvr, 0.0, 0.0, g.L, g.lt, 0.0, false);
 }
 
-template <int kMin, bool kPow2>
-__global__ void __launch_bounds__(kBS, kMin)
-k_gradient_poly_walk(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
-                     double *__restrict__ grad, int chunks, long long units) {
+// The chunk's gradients to out[0 ..] (out: of site s0). hs: its heights from
+// site s0 - 1 on in shared memory, or null.
+template <bool kPow2, bool kStage>
+__device__ __forceinline__ void walk_chunk(const double *__restrict__ hl, const PolyGeom &g,
+                                           double *__restrict__ out, int s0, int lane,
+                                           const double *hs = nullptr) {
     const int n = g.n;
-    const int lane = threadIdx.x & 31;
-    const long long u = (long long)blockIdx.x * (kBS / 32) + (threadIdx.x >> 5);
-    if (u >= units) return;
-    const int line = (int)(u / chunks);
-    const int s0 = (int)(u - (long long)line * chunks) * kWalkSites;
-    const double *hl = h + (size_t)line * (size_t)n;
-    double *out = grad + (size_t)line * (size_t)n;
     // step k's edges are s0 - 1 + 32 k + lane, each with the site at its
     // right end; the two sites of the wrap edge are done apart
-    if (s0 == 0 && lane == 0) walk_site_rare(g, hl, out, 0);
-    if (s0 + kWalkSites >= n && lane == 1) walk_site_rare(g, hl, out, n - 1);
+    if (s0 == 0 && lane == 0) out[0] = walk_site_rare(g, hl, 0);
+    if (s0 + kWalkSites >= n && lane == 1) out[n - 1 - s0] = walk_site_rare(g, hl, n - 1);
     double x[kWalkSteps];
 #pragma unroll
     for (int k = 0; k < kWalkSteps; ++k) {
         const int i = s0 - 1 + 32 * k + lane;
-        x[k] = __ldg(hl + (i < 0 ? n - 1 : i < n ? i : 0));
+        x[k] = kStage && hs ? hs[32 * k + lane] : __ldg(hl + (i < 0 ? n - 1 : i < n ? i : 0));
     }
-    const int il = s0 - 1 + kWalkEdges;
-    const double last = __ldg(hl + (il < n ? il : 0));  // right end of the last edge
+    const int il = s0 - 1 + kWalkEdges;  // right end of the last edge
+    const double last = kStage && hs ? hs[kWalkEdges] : __ldg(hl + (il < n ? il : 0));
     // the largest exponent of the chunk
     unsigned mx = (unsigned)__double2hiint(last) << 1;
 #pragma unroll
@@ -223,7 +217,7 @@ k_gradient_poly_walk(const double *__restrict__ h, const __grid_constant__ PolyG
     const int sh = 1075 + kWalkGuard - (int)mx - g.ky;
     if (!(mx < 2047u && mx > 200u && sh >= 40 && sh <= 63)) {
         for (int j = lane; j < kWalkSites; j += 32)
-            if (s0 + j > 0 && s0 + j + 1 < n) walk_site_rare(g, hl, out, s0 + j);
+            if (s0 + j > 0 && s0 + j + 1 < n) out[j] = walk_site_rare(g, hl, s0 + j);
         return;
     }
     auto fix = [&](double v) {
@@ -252,13 +246,90 @@ k_gradient_poly_walk(const double *__restrict__ h, const __grid_constant__ PolyG
             const int i = s0 + 32 * (k - 1) + lane;
             const long long S = Rb + lane_next(Rb, R, lane);
             const long long D = lane_next(sb, sl, lane) - sb;
-            if (i > 0 && i + 1 < n && (k < kWalkSteps || lane < 31))
-                __stcs(out + i, fma(g.L.c_el, fx_to_double(D, ek),
-                                    fma(g.half_unit, fx_to_double(S), -g.L.fdx)));
+            if (i > 0 && i + 1 < n && (k < kWalkSteps || lane < 31)) {
+                const double v = fma(g.L.c_el, fx_to_double(D, ek),
+                                     fma(g.half_unit, fx_to_double(S), -g.L.fdx));
+                if (kStage) out[i - s0] = v;
+                else __stcs(out + (i - s0), v);
+            }
         }
         Rb = R;
         sb = sl;
     }
+}
+
+template <int kMin, bool kPow2>
+__global__ void __launch_bounds__(kBS, kMin)
+k_gradient_poly_walk(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
+                     double *__restrict__ grad, int chunks, long long units) {
+    const long long u = (long long)blockIdx.x * (kBS / 32) + (threadIdx.x >> 5);
+    if (u >= units) return;
+    const int line = (int)(u / chunks);
+    const int s0 = (int)(u - (long long)line * chunks) * kWalkSites;
+    const size_t off = (size_t)line * (size_t)g.n;
+    walk_chunk<kPow2, false>(h + off, g, grad + off + s0, s0, threadIdx.x & 31);
+}
+
+// The same for lines in host memory (the same chunks, so the same bits): a
+// persistent block takes runs of 8 chunks, whose heights come into shared
+// memory in aligned 128-byte pieces while the run before is computed, and
+// whose gradients leave the same way. 255-site runs of a warp touch a third
+// line for every two, and the host link pays for each: 8 lines of 2^20 in
+// pinned memory 14.5 G points/s with them, 17.9 so. Two blocks an SM: the link
+// gives less when more is in flight (17.4 with three, 16.7 with four).
+template <bool kPow2>
+__global__ void __launch_bounds__(kBS, 4)
+k_gradient_poly_walk_host(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
+                          double *__restrict__ grad, int chunks, long long units) {
+    constexpr int kWarps = kBS / 32, kRun = kWarps * kWalkSites;
+    __shared__ double s_h[2][kRun + 2], s_out[kRun];
+    const int n = g.n, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const long long runs = (units + kWarps - 1) / kWarps;
+    // line and first site of a run; whole: all its chunks lie inside the line
+    auto place = [&](long long r, size_t &off, int &first) {
+        const long long u = r * kWarps;
+        const int line = (int)(u / chunks);
+        first = (int)(u - (long long)line * chunks) * kWalkSites;
+        off = (size_t)line * (size_t)n;
+        return r < runs && first > 0 && first < n - kRun;
+    };
+    auto fetch = [&](long long r, int buf) {
+        size_t off;
+        int first;
+        if (place(r, off, first)) {
+            const double *p = h + off + first - 1;
+            for (int j = (int)threadIdx.x - ((int)((uintptr_t)p >> 3) & 15); j < kRun + 2; j += kBS)
+                if (j >= 0) cp_async8(&s_h[buf][j], p + j);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    fetch(blockIdx.x, 0);
+    int buf = 0;
+    for (long long r = blockIdx.x; r < runs; r += gridDim.x, buf ^= 1) {
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();  // heights in place; the run before has left s_out and the other buffer
+        fetch(r + gridDim.x, buf ^ 1);
+        size_t off;
+        int first;
+        const bool whole = place(r, off, first);
+        const long long u = r * kWarps + w;
+        const int line = (int)(u / chunks);
+        const int s0 = (int)(u - (long long)line * chunks) * kWalkSites;
+        const size_t mine = (size_t)line * (size_t)n;
+        if (u < units)
+            walk_chunk<kPow2, true>(h + mine, g, s_out + w * kWalkSites, s0, lane,
+                                    whole ? s_h[buf] + w * kWalkSites : nullptr);
+        __syncthreads();
+        if (whole) {
+            double *o = grad + off + first;
+            for (int j = (int)threadIdx.x - ((int)((uintptr_t)o >> 3) & 15); j < kRun; j += kBS)
+                if (j >= 0) __stcs(o + j, s_out[j]);
+        } else if (u < units) {
+            for (int j = lane; j < min(kWalkSites, n - s0); j += 32)
+                __stcs(grad + mine + s0 + j, s_out[w * kWalkSites + j]);
+        }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
 // FxCubic of every (row cell j, column e) from the FP64 coefficients c
@@ -320,7 +391,7 @@ qew_status qew_poly_store_build(qew_ctx *ctx, const double *c, int nx, int ny,
 
 qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count,
                                      const double *d_h, int n, const qew_params *p,
-                                     double *d_grad) {
+                                     double *d_grad, bool host_grad) {
     if (!f || f->kind != QEW_FIELD_BSPLINE || !f->coef64 || !f->poly) return QEW_ERR_UNSUPPORTED;
     PolyGeom g{};
     g.nz = make_bspline64(f, n, p->physical_size);
@@ -362,6 +433,14 @@ qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count
             const long long blocks = (units + kBS / 32 - 1) / (kBS / 32);
             if (blocks > INT_MAX)
                 return qew_fail(ctx, QEW_ERR_INVALID, "gradient: more than 2^31 tiles");
+            if (host_grad) {
+                const int grid = (int)std::min<long long>(blocks, 2ll * ctx->num_sms);
+                if (pow2)
+                    k_gradient_poly_walk_host<true><<<grid, kBS, 0, ctx->stream>>>(d_h, g, d_grad, chunks, units);
+                else
+                    k_gradient_poly_walk_host<false><<<grid, kBS, 0, ctx->stream>>>(d_h, g, d_grad, chunks, units);
+                return qew_launch_check(ctx, "gradient_poly");
+            }
 #define QEW_WALK_LAUNCH(M) \
     (pow2 ? k_gradient_poly_walk<M, true><<<(unsigned)blocks, kBS, 0, ctx->stream>>>(              \
                 d_h, g, d_grad, chunks, units)                                                     \
@@ -386,6 +465,7 @@ qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count
         return qew_launch_check(ctx, "gradient_poly");
     };
     int cand = walk ? 1 : 5;
+    if (walk && host_grad) return launch(cand);  // bound by the host link
     QEW_TRY(qew_tune_pick(ctx, kTuneGradientPoly,
                           qew_tune_class((long long)n * count, (arc ? 1 : 0) + (walk ? 2 : 0) + (pow2 ? 4 : 0)),
                           walk ? 3 : 9, cand, walk ? walk_names : tile_names, launch, &cand));

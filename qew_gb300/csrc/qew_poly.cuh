@@ -27,4 +27,5 @@ qew_status qew_poly_store_build(qew_ctx *ctx, const double *c, int nx, int ny,
 // have one point per field column.
 qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count,
                                      const double *d_h, int n, const qew_params *p,
-                                     double *d_grad);
+                                     double *d_grad,
+                                     bool host_grad = false);
