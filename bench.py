@@ -839,9 +839,9 @@ def fp64_peak(Q, ctx):
 # smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum of one
 # launch divided by its points. For k_gradient these counters leave out its
 # FP64 floor, conversions and compares, so its fraction reads low.
-# k_gradient_poly: 7 on the headline's lines (f = 0, dx = 1: the zero-force
-# form, 4 DFMA + 3 DADD); 8 at f != 0.
-FP64_INST_PER_POINT = {"k_gradient_poly": 7.0, "k_gradient": 49.15}
+# k_gradient_poly: the linear model's walk, 2 DFMA; k_gradient: 3 DADD, 3 DFMA
+# and 1 DMUL (the gathers run in 64-bit integers).
+FP64_INST_PER_POINT = {"k_gradient_poly": 2.0, "k_gradient": 7.01}
 
 
 def run_sections_only(args, Q, torch, rank):
@@ -913,12 +913,13 @@ def run_ours(args):
     # The three forms of the gather on the same lines, each one step = the
     # gradients of all n_inst lines:
     #   fp64            FP64 drop-in: the cell-polynomial store, one batched
-    #                   persistent launch (k_gradient_poly)
+    #                   launch (k_gradient_poly: its walk for the linear model)
     #   fp64_reference  FP64 with the reference's arithmetic bit for bit (its
     #                   16-tap order, true divisions, no fused multiply-adds),
-    #                   one launch per line (k_gradient)
+    #                   one launch (k_gradient)
     #   fp32split       FP32 split-index gather on the x-filtered FP32 store,
-    #                   one batched persistent launch (k_gradient_split_persist)
+    #                   one batched launch (k_gradient_split_walk,
+    #                   reported as k_gradient_split_persist)
     def step_fp64():
         Q.gradient_batch(H, p, noise, G)
 
@@ -998,15 +999,15 @@ def run_ours(args):
     # DRAM bytes (read + write) per line point of each kernel from one ncu
     # capture of the bench's batched launch (8 lines of 2^20 points) on the
     # small field (each point touches the same number of rows whatever the
-    # field height), scaled to the points of one launch. k_gradient_poly: a
-    # warm launch inside the timed loop (--cache-control none); the others
-    # cold (ncu's cache flush, which leaves out the previous launch's
-    # write-back).
+    # field height), scaled to the points of one launch. k_gradient_poly,
+    # k_gradient and k_gradient_split_persist: a warm launch inside the timed
+    # loop (--cache-control none); k_gradient_split: cold (ncu's cache flush,
+    # which leaves out the previous launch's write-back).
     dram_per_point = {
-        "k_gradient_poly": (342.719232e6 + 69.857280e6) / (8 * L_FULL),
-        "k_gradient_split_persist": (237.686784e6 + 22.566656e6) / (8 * L_FULL),
+        "k_gradient_poly": (359.998976e6 + 61.611776e6) / (8 * L_FULL),
+        "k_gradient_split_persist": (222.557440e6 + 24.007936e6) / (8 * L_FULL),
         "k_gradient_split": (241.858816e6 + 20.879104e6) / (8 * L_FULL),
-        "k_gradient": (43.320832e6 + 0.039936e6) / L_FULL,
+        "k_gradient": (340.568320e6 + 55.892736e6) / (8 * L_FULL),
     }
     results = {}
     for name, (fn, bpp, kern, dt) in list(forms.items()) + list(forms_extra.items()):

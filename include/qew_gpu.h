@@ -171,8 +171,8 @@ qew_status qew_ctx_set_stream(qew_ctx *ctx, void *cuda_stream);
 qew_status qew_ctx_synchronize(qew_ctx *ctx);
 /* Limits of the grid barriers in this context's later persistent cooperative
  * launches (Langevin run, Rosso-Krauth sweeps; no reference counterpart): a
- * wait gives up after max_polls polls of about 64 ns (<= 0: the default
- * 2^26) and the launch returns QEW_ERR_TIMEOUT. skip_block >= 0 makes that
+ * wait gives up after max_polls polls, each a round trip to L2 (a third of a
+ * microsecond or more; <= 0: the default 2^26) and the launch returns QEW_ERR_TIMEOUT. skip_block >= 0 makes that
  * CTA leave at its first barrier without arriving, so the others' waits run
  * out: a fault for tests of the timeout path (-1: none). */
 qew_status qew_ctx_set_barrier_limits(qew_ctx *ctx, long long max_polls,

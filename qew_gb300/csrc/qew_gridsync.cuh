@@ -13,7 +13,7 @@
 
 #include "qew_internal.cuh"
 
-constexpr long long kGridBarrierPolls = 1LL << 26;  // ~4 s of 64 ns polls
+constexpr long long kGridBarrierPolls = 1LL << 26;  // some 20 s of round trips to L2
 
 struct GridSync {
     unsigned int count;   // arrivals so far (wraps)
