@@ -10,9 +10,10 @@
 //            c_el = -Gamma/dx)
 //          = Gamma (s_{i-1} - s_i) + (dx/2)(dv_{i-1} + dv_i) - dx f  (arclength).
 //
-// Two kernels:
+// Three kernels:
 //   k_gradient_poly_walk  the linear model: every step up to the last two
 //     multiply-adds in integers (below);
+//   k_gradient_poly_walk_host  the same for lines in host memory;
 //   k_gradient_poly       arclength: FP64 heights and combine, the cell and
 //     the slope's root in fixed point.
 #include <algorithm>
