@@ -501,9 +501,7 @@ qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int 
     if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "field build: %s", cudaGetErrorString(e)));
     qew_free_async(d_max, ctx->stream);
     d_max = nullptr;
-    const int max_exp = (int)(max_bits >> 52);
-    // (1023 for the zero field; outside the range no fixed point and no store)
-    f->fixb = max_bits == 0 ? 1023 : (max_exp >= 256 && max_exp <= 1792) ? max_exp : -1;
+    f->fixb = qew_fix_bound(max_bits);  // < 0: no fixed point and no store
     if (f->fixb < 0 && f->poly) {
         qew_free_async(f->poly, ctx->stream);
         f->poly = nullptr;

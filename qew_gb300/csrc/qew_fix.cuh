@@ -3,17 +3,22 @@
 // GB300 issues one FP64 instruction of a warp every 64 cycles per scheduler
 // (measured: DADD, DMUL, DFMA, compares and conversions alike, with one warp
 // already saturating it), an integer instruction every 1-2. The 16-tap
-// gather's sums are all of one scale -- the field's largest coefficient
-// bounds every partial sum -- so they lose nothing in fixed point with the
-// unit 2^-57 of that bound: about 2^-4 of an FP64 ulp at the bound, where the
-// FP64 sum rounds some twenty times at its terms' own ulps. Measured, with
+// gather's sums are of the scale of their own taps -- the stencil's largest
+// bounds every partial sum -- so each stencil takes its own unit, 2^-57 of that
+// bound: about 2^-4 of an FP64 ulp there, where the FP64 sum rounds some twenty
+// times at its terms' own ulps. (One unit for the whole field loses what a weak
+// region has beside a strong one: with coefficients 4e6 apart the weak region's
+// dV/dy was wrong by 5e-11 of its own scale. The stencil's unit costs some 40
+// integer instructions an edge.) Measured, with
 // the shorter combine of qew_model_kernels.cuh: the gradient of a
 // 262144-point arclength line 43.5 -> 14.0 us, of a 100003-point line off the
 // field's grid 28.0 -> 11.2 us, a step of the FP64 Langevin run 22.9 -> 16.1 us.
 //
-// Formats. A tap is an int64 X with c = X 2^(K-57) (|c| < 2^K for the whole
-// field, K from a maximum taken when the field is built). A fraction t in
-// [0, 1) is T = T1 2^31 + T0 in units of 2^-62, two 31-bit limbs; its product
+// Formats. A tap is an int64 X with c = X 2^(K-57), |c| < 2^K for its row of the
+// stencil; the four rows' sums are then shifted to the stencil's largest K,
+// which is d binary orders below the field's (taken when the field is built):
+// 0 <= d <= kFxOrders, weaker stencils keep the unit of the last.
+// A fraction t in [0, 1) is T = T1 2^31 + T0 in units of 2^-62, two 31-bit limbs; its product
 // with an int64 w, |w| < 2^62, is three 32 x 32 + 64-bit multiply-adds
 // (fx_mul, truncated below the unit of w).
 #pragma once
@@ -56,6 +61,15 @@ __host__ __device__ __forceinline__ unsigned long long fx_shl(unsigned long long
     return s < 64 ? u << s : 0ull;
 #endif
 }
+__host__ __device__ __forceinline__ long long fx_sar(long long u, int s) {  // s >= 0
+#ifdef __CUDA_ARCH__
+    long long r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(u), "r"(s));
+    return r;
+#else
+    return u >> (s < 63 ? s : 63);
+#endif
+}
 // Leading zeros (64 for 0).
 __host__ __device__ __forceinline__ int fx_clz(unsigned long long u) {
 #ifdef __CUDA_ARCH__
@@ -67,6 +81,24 @@ __host__ __device__ __forceinline__ int fx_clz(unsigned long long u) {
 // The limbs of a signed number v * 2^-62, |v| < 2^62.
 __host__ __device__ __forceinline__ FxFrac fx_limbs(long long v) {
     return FxFrac{(int)(v >> 31), (int)((unsigned)v & 0x7fffffffu)};
+}
+
+// Orders of magnitude below the field's largest coefficient that a stencil's
+// unit follows (8 bits in the store's cells; a factor 2^255).
+constexpr int kFxOrders = 255;
+
+// The field's biased exponent from the bits of its largest |coefficient|: 1023
+// for the zero field, -1 for one that fixed point does not serve (a stencil's
+// unit has to stay among the normal numbers, and zero and subnormal taps below it).
+__host__ __device__ __forceinline__ int qew_fix_bound(unsigned long long max_bits) {
+    const int ex = (int)(max_bits >> 52);
+    return max_bits == 0 ? 1023 : (ex >= kFxOrders + 65 && ex <= 1792) ? ex : -1;
+}
+
+// Biased exponent of the largest of four numbers, at least low.
+__device__ __forceinline__ int fx_row_exp(double a, double b, double c, double d, int low) {
+    auto ex = [](double v) { return (int)(((unsigned)__double2hiint(v) >> 20) & 0x7FFu); };
+    return max(max(max(ex(a), ex(b)), max(ex(c), ex(d))), low);
 }
 
 // An FP64 number c, |c| < 2^K with K = kb - 1022, in units of
@@ -166,10 +198,18 @@ __device__ __forceinline__ float fx_frac_to_float(unsigned long long f) {
 // E, so it stays below 12 max|E| < 2^62 (fx_mul's range).
 struct FxCubic {
     long long v, p, u2, w;  // u2 = 2u
+    int d;                  // the unit's orders below the field's
 };
-__device__ __forceinline__ FxCubic fx_cubic(const long long E[4]) {
+// Er: the rows' sums, each in the unit of its own exponent kr (K = kr - 1022);
+// kb: the field's.
+__device__ __forceinline__ FxCubic fx_cubic(const long long Er[4], const int kr[4], int kb) {
+    const int kc = max(max(kr[0], kr[1]), max(kr[2], kr[3]));
+    long long E[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) E[b] = fx_sar(Er[b], kc - kr[b]);
     const long long s = E[0] + E[2];
-    return FxCubic{s + 4 * E[1], E[2] - E[0], 2 * s - 4 * E[1], (E[3] - E[0]) - 3 * (E[2] - E[1])};
+    return FxCubic{s + 4 * E[1], E[2] - E[0], 2 * s - 4 * E[1], (E[3] - E[0]) - 3 * (E[2] - E[1]),
+                   kb - kc};
 }
 __device__ __forceinline__ long long fx_dt2(const FxCubic &c, FxFrac t) {
     return c.p + fx_mul(c.u2 + fx_mul(c.w, t), t);
@@ -177,13 +217,33 @@ __device__ __forceinline__ long long fx_dt2(const FxCubic &c, FxFrac t) {
 __device__ __forceinline__ long long fx_6v(const FxCubic &c, FxFrac t) {
     return c.v + fx_mul(3 * c.p + fx_mul(c.u2 + (c.u2 >> 1) + fx_mul(c.w, t), t), t);
 }
-// One cell of the cell-polynomial store: 32 bytes, 32-byte aligned.
+// One cell of the cell-polynomial store: 32 bytes, 32-byte aligned. d lies in
+// the bits that the three numbers leave free: |p| <= 2 max|E| < 2^59, |u2| and
+// |w| <= 8 max|E| < 2^61.
+__device__ __forceinline__ long long fx_low_bits(long long v, int free) {  // sign-extended
+    const int hi = (int)((unsigned)(v >> 32) << free) >> free;
+    return ((long long)hi << 32) | (long long)(unsigned)v;
+}
 __device__ __forceinline__ FxCubic fx_load_cell(const long long *p) {
     FxCubic c;
+    long long rp, ru, rw;
     asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
-        : "=l"(c.v), "=l"(c.p), "=l"(c.u2), "=l"(c.w)
+        : "=l"(c.v), "=l"(rp), "=l"(ru), "=l"(rw)
         : "l"(p));
+    c.p = fx_low_bits(rp, 4);
+    c.u2 = fx_low_bits(ru, 2);
+    c.w = fx_low_bits(rw, 2);
+    c.d = (int)((((unsigned)(rp >> 32) >> 28) << 4) | (((unsigned)(ru >> 32) >> 30) << 2) |
+                ((unsigned)(rw >> 32) >> 30));
     return c;
+}
+__device__ __forceinline__ void fx_store_cell(long long *p, const FxCubic &c) {
+    const long long m60 = (1ll << 60) - 1, m62 = (1ll << 62) - 1;
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(c.v),
+                 "l"((c.p & m60) | ((long long)(c.d >> 4) << 60)),
+                 "l"((c.u2 & m62) | ((long long)((c.d >> 2) & 3) << 62)),
+                 "l"((c.w & m62) | ((long long)(c.d & 3) << 62))
+                 : "memory");
 }
 
 // The cubic B-spline weights (filtered_noise.h:33-44) at fraction t, in units
@@ -201,6 +261,23 @@ __device__ __forceinline__ void fx_weights(FxFrac t, FxFrac w[4]) {
     w[1] = fx_limbs(w1);
     w[2] = fx_limbs(one - w0 - w1 - w3);
     w[3] = fx_limbs(w3);
+}
+
+// A stencil row's sum in the unit of its own exponent kr (at least kb -
+// kFxOrders, kb the field's): with the weights w(1/2) times 48, in units of
+// 2^(kr - 1074) / 48; with the weights w, in units of 2^(kr - 1079).
+__device__ __forceinline__ long long fx_row_const(const double x[4], int kb, int &kr) {
+    kr = fx_row_exp(x[0], x[1], x[2], x[3], kb - kFxOrders);
+    return ((fx_tap<4>(x[0], kr) + fx_tap<4>(x[3], kr)) +
+            23 * (fx_tap<4>(x[1], kr) + fx_tap<4>(x[2], kr))) >>
+           5;
+}
+__device__ __forceinline__ long long fx_row_sum(const double x[4], const FxFrac w[4], int kb, int &kr) {
+    kr = fx_row_exp(x[0], x[1], x[2], x[3], kb - kFxOrders);
+    long long s = 0;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) s += fx_mul(fx_tap<8>(x[a], kr), w[a]);
+    return s >> 4;
 }
 
 // 1 / sqrt(1 + dh^2). As FP64 instructions the root takes 7 of 64 cycles each;

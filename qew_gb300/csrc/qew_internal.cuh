@@ -289,52 +289,52 @@ struct NoiseBSpline64 {
         if (ef - 523u > 1000u && x != 0.0) return false;  // |x| outside [2^-500, 2^500]
         return fx_cell(div_by(x, d, inv_d), 0, n, ix, t);
     }
-    // The stencil's row sums at cell (ix, iy): x weights w(1/2) times 48 in
-    // exact integers, E in units of 2^(K-52) / 48 ...
-    __device__ __forceinline__ void fx_rows_const(int e, int iy, long long E[4]) const {
+    // The stencil's cubic at cell (ix, iy) from its row sums: x weights w(1/2)
+    // times 48 in exact integers, E in units of 2^(K-52) / 48 ...
+    __device__ __forceinline__ FxCubic fx_rows_const(int e, int iy) const {
         const bool inner = e >= 1 && e + 2 < nx && iy >= 1 && iy + 2 < ny;
         const double *p = coef + ((size_t)iy * (size_t)nx + (size_t)e);
-        int xs[4], ys[4];
+        int xs[4], ys[4], kr[4];
         if (!inner) {
             wrap4(e, nx, xs);
             wrap4(iy, ny, ys);
         }
+        long long E[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            long long X[4];
+            double x[4];
             const double *row = p + (ptrdiff_t)(b - 1) * (ptrdiff_t)nx;
 #pragma unroll
             for (int a = 0; a < 4; ++a)
-                X[a] = fx_tap<4>(inner ? QEW_LDGP(row + (a - 1), coef, (size_t)nx * (size_t)ny, oob)
-                                       : c(xs[a], ys[b]),
-                                 kb);
-            E[b] = ((X[0] + X[3]) + 23 * (X[1] + X[2])) >> 5;
+                x[a] = inner ? QEW_LDGP(row + (a - 1), coef, (size_t)nx * (size_t)ny, oob)
+                             : c(xs[a], ys[b]);
+            E[b] = fx_row_const(x, kb, kr[b]);
         }
+        return fx_cubic(E, kr, kb);
     }
     // ... or general x weights, E in units of 2^(K-57).
-    __device__ __forceinline__ void fx_rows(int ix, FxFrac fx, int iy, long long E[4]) const {
+    __device__ __forceinline__ FxCubic fx_rows(int ix, FxFrac fx, int iy) const {
         const bool inner = ix >= 1 && ix + 2 < nx && iy >= 1 && iy + 2 < ny;
         const double *p = coef + ((size_t)iy * (size_t)nx + (size_t)ix);
-        int xs[4], ys[4];
+        int xs[4], ys[4], kr[4];
         if (!inner) {
             wrap4(ix, nx, xs);
             wrap4(iy, ny, ys);
         }
         FxFrac wx[4];
         fx_weights(fx, wx);
+        long long E[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
+            double x[4];
             const double *row = p + (ptrdiff_t)(b - 1) * (ptrdiff_t)nx;
-            long long s = 0;
 #pragma unroll
             for (int a = 0; a < 4; ++a)
-                s += fx_mul(fx_tap<8>(inner ? QEW_LDGP(row + (a - 1), coef,
-                                                       (size_t)nx * (size_t)ny, oob)
-                                            : c(xs[a], ys[b]),
-                                      kb),
-                            wx[a]);
-            E[b] = s >> 4;
+                x[a] = inner ? QEW_LDGP(row + (a - 1), coef, (size_t)nx * (size_t)ny, oob)
+                             : c(xs[a], ys[b]);
+            E[b] = fx_row_sum(x, wx, kb, kr[b]);
         }
+        return fx_cubic(E, kr, kb);
     }
 
     __device__ __forceinline__ double c(int ix, int iy) const {
@@ -405,9 +405,15 @@ struct NoiseBSpline64 {
             e = QEW_IDX(e, nx, oob);
             return fx_load_cell(poly + ((size_t)iy * (size_t)nx + (size_t)e) * 4);
         }
-        long long E[4];
-        fx_rows_const(e, iy, E);
-        return fx_cubic(E);
+        return fx_rows_const(e, iy);
+    }
+    // The sums 2 dV/dt and 6 V of cell q at fraction t, in FP64 units of fx_dv_*
+    // and fx_v_*.
+    static __device__ __forceinline__ double fx_dv(const FxCubic &q, FxFrac t) {
+        return fx_to_double(fx_dt2(q, t), -q.d);
+    }
+    static __device__ __forceinline__ double fx_v(const FxCubic &q, FxFrac t) {
+        return fx_to_double(fx_6v(q, t), -q.d);
     }
     // Row cell and fraction of the edge midpoint at height a / 2.
     // (On the store of a spacing that is no power of two by one product, within
@@ -426,7 +432,7 @@ struct NoiseBSpline64 {
             if (!(t >= 0.0)) return a - a;  // NaN
             fy = fx_frac((unsigned long long)(fmin(t, 1.0 - 0x1p-53) * 0x1p64));
         }
-        return __dmul_rn(fx_to_double(fx_dt2(fx_const_cell(e, iy), fy)), fx_dv_c);
+        return __dmul_rn(fx_dv(fx_const_cell(e, iy), fy), fx_dv_c);
     }
     // dV/dy / V at the midpoint of edge e (xc its physical x, a the sum of its
     // two heights) in fixed point; what its locate declines (negative or huge
@@ -438,11 +444,9 @@ struct NoiseBSpline64 {
             FxFrac fx, fy;
             if (fx_row(a, iy, fy)) {
                 if (fx_const(e))
-                    return __dmul_rn(fx_to_double(fx_dt2(fx_const_cell(e, iy), fy)), fx_dv_c);
+                    return __dmul_rn(fx_dv(fx_const_cell(e, iy), fy), fx_dv_c);
                 if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
-                    long long E[4];
-                    fx_rows(ix, fx, iy, E);
-                    return __dmul_rn(fx_to_double(fx_dt2(fx_cubic(E), fy)), fx_dv_g);
+                    return __dmul_rn(fx_dv(fx_rows(ix, fx, iy), fy), fx_dv_g);
                 }
             }
         }
@@ -454,11 +458,9 @@ struct NoiseBSpline64 {
             FxFrac fx, fy;
             if (fx_row(a, iy, fy)) {
                 if (fx_const(e))
-                    return __dmul_rn(fx_to_double(fx_6v(fx_const_cell(e, iy), fy)), fx_v_c);
+                    return __dmul_rn(fx_v(fx_const_cell(e, iy), fy), fx_v_c);
                 if (fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
-                    long long E[4];
-                    fx_rows(ix, fx, iy, E);
-                    return __dmul_rn(fx_to_double(fx_6v(fx_cubic(E), fy)), fx_v_g);
+                    return __dmul_rn(fx_v(fx_rows(ix, fx, iy), fy), fx_v_g);
                 }
             }
         }
@@ -473,16 +475,9 @@ struct NoiseBSpline64 {
             if (fx_row(a, iy, fy)) {
                 const bool cst = fx_const(e);
                 if (cst || fx_locate(xc, dx, inv_dx, kx, nx, ix, fx)) {
-                    FxCubic q;
-                    if (cst) {
-                        q = fx_const_cell(e, iy);
-                    } else {
-                        long long E[4];
-                        fx_rows(ix, fx, iy, E);
-                        q = fx_cubic(E);
-                    }
-                    v = __dmul_rn(fx_to_double(fx_6v(q, fy)), cst ? fx_v_c : fx_v_g);
-                    dv = __dmul_rn(fx_to_double(fx_dt2(q, fy)), cst ? fx_dv_c : fx_dv_g);
+                    const FxCubic q = cst ? fx_const_cell(e, iy) : fx_rows(ix, fx, iy);
+                    v = __dmul_rn(fx_v(q, fy), cst ? fx_v_c : fx_v_g);
+                    dv = __dmul_rn(fx_dv(q, fy), cst ? fx_dv_c : fx_dv_g);
                     return;
                 }
             }

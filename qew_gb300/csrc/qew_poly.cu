@@ -157,12 +157,13 @@ constexpr int kWalkEdges = 32 * kWalkSteps;
 constexpr int kWalkSites = kWalkEdges - 1;
 constexpr int kWalkGuard = 8;
 
-// R = dV/dy of edge e < n - 1 in the store's unit from the integer sum a of
-// its heights, whose midpoint in row cells is a 2^-sh, |a 2^-sh| < 2^22.
+// R = dV/dy of edge e < n - 1 in the unit of its cell, d orders below the
+// store's, from the integer sum a of its heights, whose midpoint in row cells is a 2^-sh, |a 2^-sh| < 2^22.
 // kPow2: a power-of-two row spacing; else a is first multiplied by the
 // spacing's reciprocal mantissa (62 bits).
 template <bool kPow2>
-__device__ __forceinline__ long long walk_edge(const PolyGeom &g, int e, long long a, int sh) {
+__device__ __forceinline__ long long walk_edge(const PolyGeom &g, int e, long long a, int sh,
+                                               int &d) {
     if (!kPow2) a = fx_mul(a, g.recip);
     int c = (int)(a >> sh);  // floor
     const FxFrac t = fx_frac((unsigned long long)a << (64 - sh));
@@ -173,7 +174,9 @@ __device__ __forceinline__ long long walk_edge(const PolyGeom &g, int e, long lo
     }
     c = QEW_IDX(c, g.nz.ny, g.nz.oob);
     e = QEW_IDX(e, g.nz.nx, g.nz.oob);
-    return fx_dt2(fx_load_cell(g.nz.poly + ((size_t)c * (size_t)g.nz.nx + (size_t)e) * 4), t);
+    const FxCubic q = fx_load_cell(g.nz.poly + ((size_t)c * (size_t)g.nz.nx + (size_t)e) * 4);
+    d = q.d;
+    return fx_dt2(q, t);
 }
 
 // v of the next lane; the last lane gets `wrap` of the first one.
@@ -231,30 +234,36 @@ __device__ __forceinline__ void walk_chunk(const double *__restrict__ hl, const 
         return ((long long)fx_shr(w, (int)(mx - ((hi >> 20) & 0x7FFu))) ^ sg) - sg;
     };
     const int ek = (int)mx - 1075 - kWalkGuard;
-    long long H = fix(x[0]), Rb = 0, sb = 0;  // Rb, sb: edge and slope of the step before
+    long long H = fix(x[0]), Rb = 0, sb = 0;  // Rb (db), sb: edge and slope of the step before
+    int db = 0;
 #pragma unroll
     for (int k = 0; k <= kWalkSteps; ++k) {
         long long R = 0, sl = 0;
+        int d = 0;
         if (k < kWalkSteps) {
             const long long Hn = fix(k + 1 < kWalkSteps ? x[k + 1 < kWalkSteps ? k + 1 : 0] : last);
             const long long Hp = lane_next(H, Hn, lane);
             const int e = s0 - 1 + 32 * k + lane;
-            R = walk_edge<kPow2>(g, e >= 0 && e + 1 < n ? e : 0, H + Hp, sh);
+            R = walk_edge<kPow2>(g, e >= 0 && e + 1 < n ? e : 0, H + Hp, sh, d);
             sl = Hp - H;
             H = Hn;
         }
         if (k > 0) {  // the sites of the step before
             const int i = s0 + 32 * (k - 1) + lane;
-            const long long S = Rb + lane_next(Rb, R, lane);
+            const long long Rn = lane_next(Rb, R, lane);
+            const int dn = __shfl_sync(0xffffffffu, lane == 0 ? d : db, (lane + 1) & 31);
+            const int ds = min(db, dn);  // both edges in the unit of the larger
+            const long long S = fx_sar(Rb, db - ds) + fx_sar(Rn, dn - ds);
             const long long D = lane_next(sb, sl, lane) - sb;
             if (i > 0 && i + 1 < n && (k < kWalkSteps || lane < 31)) {
                 const double v = fma(g.L.c_el, fx_to_double(D, ek),
-                                     fma(g.half_unit, fx_to_double(S), -g.L.fdx));
+                                     fma(g.half_unit, fx_to_double(S, -ds), -g.L.fdx));
                 if (kStage) out[i - s0] = v;
                 else __stcs(out + (i - s0), v);
             }
         }
         Rb = R;
+        db = d;
         sb = sl;
     }
 }
@@ -348,33 +357,33 @@ __global__ void __launch_bounds__(kStoreBS) k_poly_store(const double *__restric
     const int e = blockIdx.x * kStoreBS + threadIdx.x;
     if (e >= nx) return;
     const unsigned long long mb = *max_bits;
-    const int kb = mb == 0 ? 1023 : (int)(mb >> 52);
+    const int kb = qew_fix_bound(mb);
+    if (kb < 0) return;  // no fixed point for this field: the store is dropped
     const int j0 = blockIdx.y * kStoreRows;
     const int j1 = min(ny, j0 + kStoreRows);
     int xs[4];
     wrap4(e, nx, xs);
     int r = (j0 == 0) ? ny - 1 : j0 - 1;  // row j0-1, periodic
-    auto next_row = [&]() {
+    long long E[4];
+    int kr[4];
+    auto next_row = [&](int b) {
         const double *row = c + (size_t)r * nx;
         r = (r + 1 == ny) ? 0 : r + 1;
-        return ((fx_tap<4>(__ldg(row + xs[0]), kb) + fx_tap<4>(__ldg(row + xs[3]), kb)) +
-                23 * (fx_tap<4>(__ldg(row + xs[1]), kb) + fx_tap<4>(__ldg(row + xs[2]), kb))) >>
-               5;
+        const double x[4] = {__ldg(row + xs[0]), __ldg(row + xs[1]), __ldg(row + xs[2]),
+                             __ldg(row + xs[3])};
+        E[b] = fx_row_const(x, kb, kr[b]);
     };
-    long long E[4];
-    E[0] = next_row();
-    E[1] = next_row();
-    E[2] = next_row();
+    next_row(0);
+    next_row(1);
+    next_row(2);
     for (int j = j0; j < j1; ++j) {
-        E[3] = next_row();
-        const FxCubic q = fx_cubic(E);
-        long long *o = out + ((size_t)j * (size_t)nx + (size_t)e) * 4;  // 32-byte aligned
-        asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(o), "l"(q.v), "l"(q.p),
-                     "l"(q.u2), "l"(q.w)
-                     : "memory");
-        E[0] = E[1];
-        E[1] = E[2];
-        E[2] = E[3];
+        next_row(3);
+        fx_store_cell(out + ((size_t)j * (size_t)nx + (size_t)e) * 4, fx_cubic(E, kr, kb));
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            E[b] = E[b + 1];
+            kr[b] = kr[b + 1];
+        }
     }
 }
 

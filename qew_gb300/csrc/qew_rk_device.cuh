@@ -294,6 +294,7 @@ __device__ __forceinline__ double rk_forward_zero_pair(const Noise &nz, int i, i
 // a 2048-point line (16 taps): 39.0 -> 5.8 ms, of 16384 points 8.1 ms.
 struct RkEdge {     // one edge's cubics in row cells iy and iy + 1
     long long p[2], u2[2], w[2];
+    int d[2];  // the cells' units' orders below the field's (FxCubic)
     int iy;
     double unit;
 };
@@ -310,8 +311,15 @@ __device__ __forceinline__ int rk_cell(const NoiseBSpline64 &nz, const RkEdge &e
 struct RkFast {
     RkEdge l, r;
     double hl, hr;
-    float slope0, bl, br;  // -dv/dh = slope0 + bl q_l + br q_r, q = d(2 dV/dt)/dt
+    // -dv/dh = slope0 + bl q_l + br q_r, q = d(2 dV/dt)/dt in units of 2^32 of the
+    // cell's unit, b by window cell
+    float slope0, bl[2], br[2];
 };
+
+// b 2^-d (0 where a float may not hold it).
+__device__ __forceinline__ float rk_scale(float b, int d) {
+    return d < 126 ? b * __int_as_float((127 - d) << 23) : 0.0f;
+}
 
 // v(h) as rk_site_velocity gives it; s: -dv/dh; cl, cr: the window cells (-1:
 // outside, v unset).
@@ -327,17 +335,17 @@ __device__ __forceinline__ double rk_fast_velocity(const NoiseBSpline64 &nz, con
     const long long twl = fx_mul(wl, tl), twr = fx_mul(wr, tr);
     const long long Rl = (l1 ? F.l.p[1] : F.l.p[0]) + fx_mul(ul + twl, tl);
     const long long Rr = (r1 ? F.r.p[1] : F.r.p[0]) + fx_mul(ur + twr, tr);
-    s = fmaf(F.bl, (float)(int)((ul + 2 * twl) >> 32), fmaf(F.br, (float)(int)((ur + 2 * twr) >> 32),
-                                                            F.slope0));
-    const double dvl = __dmul_rn(fx_to_double(Rl), F.l.unit);
-    const double dvr = __dmul_rn(fx_to_double(Rr), F.r.unit);
+    s = fmaf(l1 ? F.bl[1] : F.bl[0], (float)(int)((ul + 2 * twl) >> 32),
+             fmaf(r1 ? F.br[1] : F.br[0], (float)(int)((ur + 2 * twr) >> 32), F.slope0));
+    const double dvl = __dmul_rn(fx_to_double(Rl, -(l1 ? F.l.d[1] : F.l.d[0])), F.l.unit);
+    const double dvr = __dmul_rn(fx_to_double(Rr, -(r1 ? F.r.d[1] : F.r.d[0])), F.r.unit);
     return rk_velocity_of<NoiseBSpline64>(dvl, dvr, L, 0.0, 0.0, QEW_MODEL_LINEAR, h, F.hl, F.hr);
 }
 
-// The smaller q of window cell k, in units of 2^32.
-__device__ __forceinline__ float rk_qmin(const RkEdge &ed, int k) {
+// The smaller b q of window cell k.
+__device__ __forceinline__ float rk_qmin(const RkEdge &ed, const float b[2], int k) {
     const long long u = k ? ed.u2[1] : ed.u2[0], w = k ? ed.w[1] : ed.w[0];
-    return fminf((float)(int)(u >> 32), (float)(int)((u + 2 * w) >> 32));
+    return (k ? b[1] : b[0]) * fminf((float)(int)(u >> 32), (float)(int)((u + 2 * w) >> 32));
 }
 
 // One edge's place: its column, and general x weights where it needs them.
@@ -367,15 +375,16 @@ __device__ __forceinline__ void rk_window(const NoiseBSpline64 &nz, RkFast &F, c
         const int l1 = ql.iy + 1 == nz.ny ? 0 : ql.iy + 1, r1 = qr.iy + 1 == nz.ny ? 0 : qr.iy + 1;
         const FxCubic a = nz.fx_const_cell(ql.e, ql.iy), b = nz.fx_const_cell(ql.e, l1);
         const FxCubic c = nz.fx_const_cell(qr.e, qr.iy), d = nz.fx_const_cell(qr.e, r1);
-        F.l.p[0] = a.p, F.l.u2[0] = a.u2, F.l.w[0] = a.w;
-        F.l.p[1] = b.p, F.l.u2[1] = b.u2, F.l.w[1] = b.w;
-        F.r.p[0] = c.p, F.r.u2[0] = c.u2, F.r.w[0] = c.w;
-        F.r.p[1] = d.p, F.r.u2[1] = d.u2, F.r.w[1] = d.w;
+        F.l.p[0] = a.p, F.l.u2[0] = a.u2, F.l.w[0] = a.w, F.l.d[0] = a.d;
+        F.l.p[1] = b.p, F.l.u2[1] = b.u2, F.l.w[1] = b.w, F.l.d[1] = b.d;
+        F.r.p[0] = c.p, F.r.u2[0] = c.u2, F.r.w[0] = c.w, F.r.d[0] = c.d;
+        F.r.p[1] = d.p, F.r.u2[1] = d.u2, F.r.w[1] = d.w, F.r.d[1] = d.d;
         return;
     }
     // row sums 0..4 of the left edge's rows iy - 1 .. iy + 3, 5..9 of the right's
     constexpr int kPass = (10 + G - 1) / G;
     long long mine[kPass];
+    int kmine[kPass];
 #pragma unroll
     for (int p = 0; p < kPass; ++p) {
         const int k = min(p * G + lane, 9);
@@ -386,27 +395,27 @@ __device__ __forceinline__ void rk_window(const NoiseBSpline64 &nz, RkFast &F, c
         while (y >= nz.ny) y -= nz.ny;  // at most 3 times
         int xs[4];
         wrap4(e, nz.nx, xs);
+        const double x[4] = {nz.c(xs[0], y), nz.c(xs[1], y), nz.c(xs[2], y), nz.c(xs[3], y)};
         if (right ? qr.cst : ql.cst) {
-            mine[p] = ((fx_tap<4>(nz.c(xs[0], y), nz.kb) + fx_tap<4>(nz.c(xs[3], y), nz.kb)) +
-                       23 * (fx_tap<4>(nz.c(xs[1], y), nz.kb) + fx_tap<4>(nz.c(xs[2], y), nz.kb))) >>
-                      5;
+            mine[p] = fx_row_const(x, nz.kb, kmine[p]);
         } else {
             FxFrac wx[4];
             fx_weights(right ? qr.fx : ql.fx, wx);
-            long long t = 0;
-#pragma unroll
-            for (int a = 0; a < 4; ++a) t += fx_mul(fx_tap<8>(nz.c(xs[a], y), nz.kb), wx[a]);
-            mine[p] = t >> 4;
+            mine[p] = fx_row_sum(x, wx, nz.kb, kmine[p]);
         }
     }
     long long E[10];
+    int kr[10];
 #pragma unroll
-    for (int k = 0; k < 10; ++k) E[k] = __shfl_sync(gmask, mine[k / G], k % G, G);
+    for (int k = 0; k < 10; ++k) {
+        E[k] = __shfl_sync(gmask, mine[k / G], k % G, G);
+        kr[k] = __shfl_sync(gmask, kmine[k / G], k % G, G);
+    }
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const FxCubic a = fx_cubic(E + k), b = fx_cubic(E + 5 + k);
-        F.l.p[k] = a.p, F.l.u2[k] = a.u2, F.l.w[k] = a.w;
-        F.r.p[k] = b.p, F.r.u2[k] = b.u2, F.r.w[k] = b.w;
+        const FxCubic a = fx_cubic(E + k, kr + k, nz.kb), b = fx_cubic(E + 5 + k, kr + 5 + k, nz.kb);
+        F.l.p[k] = a.p, F.l.u2[k] = a.u2, F.l.w[k] = a.w, F.l.d[k] = a.d;
+        F.r.p[k] = b.p, F.r.u2[k] = b.u2, F.r.w[k] = b.w, F.r.d[k] = b.d;
     }
 }
 
@@ -438,8 +447,13 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
         if (!rk_place(nz, ql, im, xl, __dadd_rn(hl, a)) || !rk_place(nz, qr, i, xr, __dadd_rn(a, hr)))
             return false;
         rk_window<G>(nz, F, ql, qr, lane, gmask);
-        F.bl = (float)(0.5 * L.half_dx * F.l.unit * nz.inv_dy * 0x1p32);
-        F.br = (float)(0.5 * L.half_dx * F.r.unit * nz.inv_dy * 0x1p32);
+        const float bl = (float)(0.5 * L.half_dx * F.l.unit * nz.inv_dy * 0x1p32);
+        const float br = (float)(0.5 * L.half_dx * F.r.unit * nz.inv_dy * 0x1p32);
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            F.bl[k] = rk_scale(bl, F.l.d[k]);
+            F.br[k] = rk_scale(br, F.r.d[k]);
+        }
         double b = a, adv = advanced;
         bool valid = true;
         if (advanced + 1.001 * G * rp.dstep < rp.max_advance) {
@@ -472,9 +486,8 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
             vhc = __shfl_sync(gmask, v, j, G);
             const int l0 = __shfl_sync(gmask, cl, j - 1, G), l1 = __shfl_sync(gmask, cl, j, G);
             const int r0 = __shfl_sync(gmask, cr, j - 1, G), r1 = __shfl_sync(gmask, cr, j, G);
-            const float ml = fminf(rk_qmin(F.l, l0), rk_qmin(F.l, l1));
-            const float mr = fminf(rk_qmin(F.r, r0), rk_qmin(F.r, r1));
-            smin = fmaf(F.bl, ml, fmaf(F.br, mr, F.slope0));
+            smin = F.slope0 + fminf(rk_qmin(F.l, F.bl, l0), rk_qmin(F.l, F.bl, l1)) +
+                   fminf(rk_qmin(F.r, F.br, r0), rk_qmin(F.r, F.br, r1));
             // a step as long as a period of the field could skip cells
             if (!(l0 <= l1 && r0 <= r1 && rp.dstep < 2.0 * nz.dy && smin > 0.25f * F.slope0))
                 return false;
