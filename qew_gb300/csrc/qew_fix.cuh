@@ -283,12 +283,15 @@ __device__ __forceinline__ long long fx_row_sum(const double x[4], const FxFrac 
 // 1 / sqrt(1 + dh^2). As FP64 instructions the root takes 7 of 64 cycles each;
 // here it is in units of 2^-62 from the single precision root w0 and its
 // exact error r = 1 - w0^2 - (w0 dh)^2 to second order (the third is below
-// 2^-62), about 100 cycles of integer instructions. |dh| outside [2^-30, 2^8)
-// takes FP64's rsqrt (the small ones: 1 to rounding).
+// 2^-62), about 100 cycles of integer instructions, and rounds once, into the
+// result: 0.29 ulp rms without bias, where the FP64 instructions round some
+// four times (0.63). Below 2^-30 the root is 1 to rounding; from 2^8 on FP64's
+// rsqrt takes it.
 __device__ __forceinline__ double fx_invroot(double dh) {
     const unsigned hi = (unsigned)__double2hiint(dh), lo = (unsigned)__double2loint(dh);
     const int x = (int)((hi >> 20) & 0x7FFu) - 1023;  // |dh| in [2^x, 2^(x+1))
-    if (x < -30 || x > 7) return rsqrt(fma(dh, dh, 1.0));
+    if (x < -30) return 1.0;
+    if (x > 7) return rsqrt(fma(dh, dh, 1.0));
     const unsigned mh = (hi & 0x000FFFFFu) | 0x00100000u;
     // |dh| = M 2^(x - 61), M in [2^61, 2^62)
     const unsigned long long M = ((unsigned long long)__funnelshift_l(lo, mh, 9) << 32) |
@@ -297,15 +300,20 @@ __device__ __forceinline__ double fx_invroot(double dh) {
     const float w0f = rsqrtf(fmaf(f, f, 1.0f));
     const unsigned w0 = (unsigned)(w0f * 2147483648.0f);  // 2^-31, at most 2^31
     // t = w0 |dh| in units of 2^-62 (below 2^62: w0 |dh| < 1 by more than r)
-    const unsigned long long p = (M >> 31) * w0 + (((M & 0x7fffffffull) * w0) >> 31);  // 2^(x-61)
-    const unsigned long long t = x < 0 ? fx_shr(p, -1 - x) : fx_shl(p, x + 1);
+    const unsigned long long ph = (M >> 31) * w0, pl = (M & 0x7fffffffull) * w0;
+    const unsigned long long t =
+        x < 0 ? fx_shr(ph + (pl >> 31), -1 - x) : fx_shl(ph, x + 1) + fx_shr(pl, 30 - x);
     const long long ww = (long long)((unsigned long long)w0 * w0);  // w0^2, 2^-62
     const long long r = (1ll << 62) - ww - fx_mul((long long)t, fx_limbs((long long)t));  // |r| < 2^42
     const long long r1 = r >> 20;
     const long long c = (r >> 1) + ((3 * ((r1 * r1) >> 22)) >> 3);
-    // w = w0 (1 + c)
-    const long long w = ((long long)w0 << 31) + (((c >> 10) * (long long)w0) >> 21);
-    return fx_to_double(w, -62);
+    // w = w0 (1 + c) with every bit of the product, in units of 2^-62, of
+    // 2^-(62 + x) where the root is that small (cut at 2^-52 it made every
+    // slope too small, by 0.7 to 1 ulp)
+    const int sh = max(x, 0);
+    const long long cw = (c >> 20) * (long long)w0 + (((c & 0xFFFFFll) * (long long)w0) >> 20);
+    const long long w = ((long long)w0 << (31 + sh)) + (cw >> (11 - sh));
+    return fx_to_double(w, -62 - sh);
 }
 // dh / sqrt(1 + dh^2)
 __device__ __forceinline__ double fx_slope(double dh) { return __dmul_rn(dh, fx_invroot(dh)); }
