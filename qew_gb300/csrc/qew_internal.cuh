@@ -199,15 +199,39 @@ __host__ __device__ __forceinline__ bool dbl_is_pow2(double d) {
     return d > 0 && (b & 0x000FFFFFFFFFFFFFLL) == 0 && ((b >> 52) & 0x7FF) != 0;
 }
 
+// A spacing that the fixed-point locate may divide by (NoiseBSpline64::div_by):
+// in [2^-500, 2^500], not the one mantissa (all ones) Markstein's theorem
+// leaves out.
+__host__ __device__ __forceinline__ bool qew_fixed_div_ok(double d) {
+#ifdef __CUDA_ARCH__
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+#else
+    unsigned long long b;
+    memcpy(&b, &d, sizeof(b));
+#endif
+    const int ef = (int)(b >> 52);
+    return ef >= 523 && ef <= 1523 && (b & 0x000FFFFFFFFFFFFFull) != 0x000FFFFFFFFFFFFFull;
+}
+
 // Line spacing dx = physical_size / n with exact shortcuts for its divisions.
 // With the line's tension and force, the folded factors of the per-site
 // combine as well (site_gradient, qew_model_kernels.cuh).
 struct LineDx {
     double dx, inv_dx, inv_dx2;
-    bool pow2;
+    bool pow2, fixed;  // fixed: a spacing that slope() may divide by
     double half_dx, c_el, fdx;  // dx / 2, -Gamma / dx, dx f
     __host__ __device__ __forceinline__ double div(double v) const {
         return pow2 ? v * inv_dx : v / dx;
+    }
+    // v / dx to rounding, as div, for finite v of ordinary size by three FP64
+    // instructions where the division takes nine (NoiseBSpline64::div_by).
+    // The product with 1 / dx alone would scale every slope of a line by the
+    // same rounding error.
+    __device__ __forceinline__ double slope(double v) const {
+        const double q = v * inv_dx;
+        if (pow2) return q;
+        if (!fixed || ((unsigned)__double2hiint(q) & 0x7FF00000u) > (1500u << 20)) return __ddiv_rn(v, dx);
+        return fma(fma(-q, dx, v), inv_dx, q);
     }
     __host__ __device__ __forceinline__ double div2(double v) const {  // v / (dx*dx)
         return pow2 ? v * inv_dx2 : v / (dx * dx);
@@ -220,6 +244,7 @@ __host__ __device__ __forceinline__ LineDx make_line_dx(double physical_size, in
     L.inv_dx = 1.0 / L.dx;
     L.inv_dx2 = 1.0 / (L.dx * L.dx);
     L.pow2 = dbl_is_pow2(L.dx);
+    L.fixed = qew_fixed_div_ok(L.dx);
     L.half_dx = 0.5 * L.dx;
     L.c_el = -lt / L.dx;
     L.fdx = L.dx * f;
@@ -756,15 +781,6 @@ static inline bool qew_is_pow2(double d) {
     int e;
     const double m = frexp(d, &e);
     return d > 0 && m == 0.5;
-}
-// A spacing that the fixed-point locate may divide by (NoiseBSpline64::div_by):
-// in [2^-500, 2^500], not the one mantissa (all ones) Markstein's theorem
-// leaves out.
-static inline bool qew_fixed_div_ok(double d) {
-    uint64_t b;
-    memcpy(&b, &d, sizeof(b));
-    const int ef = (int)(b >> 52);
-    return ef >= 523 && ef <= 1523 && (b & 0x000FFFFFFFFFFFFFull) != 0x000FFFFFFFFFFFFFull;
 }
 static inline NoiseBSpline64 make_bspline64(const qew_field *f, int n = 0,
                                             double physical_size = 0) {

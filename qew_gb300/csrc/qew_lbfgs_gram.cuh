@@ -434,7 +434,7 @@ __device__ qew_lbfgs_result lbfgs_gram(Team &T, const Noise &nz, double *__restr
             const int e = p0 + k, ep = e + 1 == n ? 0 : e + 1;
             double v, dv;
             noise_both_edge(nz, e, EdgeX{e + ep, L.dx}, x0 + x1, v, dv);
-            const double dh = (x1 - x0) * L.inv_dx;
+            const double dh = L.slope(x1 - x0);
             double el;
             if (arc) {
                 const double w = fx_invroot(dh);

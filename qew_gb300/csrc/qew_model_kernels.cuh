@@ -23,7 +23,7 @@ __device__ __forceinline__ double edge_energy(const Noise &nz, int i, int ip, do
                                               int model) {
     // Unfused where a contraction would change the rounding (1 + s^2, the
     // f*h term), so the reference-exact functor reproduces its operations.
-    const double dh_dx = noise_is_ref<Noise>::value ? L.div(hip - hi) : (hip - hi) * L.inv_dx;
+    const double dh_dx = noise_is_ref<Noise>::value ? L.div(hip - hi) : L.slope(hip - hi);
     double line_energy;
     if (model == QEW_MODEL_LINEAR)
         line_energy = lt * dh_dx * dh_dx * 0.5;
@@ -53,7 +53,7 @@ __device__ __forceinline__ void edge_gradient(const Noise &nz, int e, int n, dou
             const double dh = L.div(hep - he);
             sl = dh / sqrt(__dadd_rn(1.0, __dmul_rn(dh, dh)));
         } else {
-            sl = fx_slope((hep - he) * L.inv_dx);
+            sl = fx_slope(L.slope(hep - he));
         }
     }
 }

@@ -113,7 +113,7 @@ k_gradient_poly(const double *__restrict__ h, const __grid_constant__ PolyGeom g
             slot = QEW_IDX(slot, kTile + 1, g.nz.oob);
             const double he = sh[slot], hep = sh[slot + 1];
             s_dv[slot] = e + 1 < n ? g.nz.dvdy_edge_store(e, hep + he) : walk_edge_rare(g, e, hep + he);
-            s_sl[slot] = fx_slope((hep - he) * g.L.inv_dx);
+            s_sl[slot] = fx_slope(g.L.slope(hep - he));
         };
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {

@@ -43,8 +43,8 @@ __device__ __forceinline__ double rk_velocity_of(double dvl, double dvr, const L
     } else {
         const double rest = fma(L.half_dx, __dadd_rn(dvl, dvr), -L.fdx);
         if (model == QEW_MODEL_LINEAR) return -fma(L.c_el, fma(-2.0, hi, __dadd_rn(hl, hr)), rest);
-        const double sll = fx_slope(__dmul_rn(__dsub_rn(hi, hl), L.inv_dx));
-        const double slr = fx_slope(__dmul_rn(__dsub_rn(hr, hi), L.inv_dx));
+        const double sll = fx_slope(L.slope(__dsub_rn(hi, hl)));
+        const double slr = fx_slope(L.slope(__dsub_rn(hr, hi)));
         return -fma(lt, __dsub_rn(sll, slr), rest);
     }
 }

@@ -15,13 +15,19 @@ spread between 1/2 and 2: 0.29 sqrt(1 + 4/3) = 0.44 for a uniform logarithm);
 one-sided where the root is within a few ulps of 1 (slopes about 2^-26), so the
 bias is measured against the correctly rounded root times s: the two differ for
 one slope in a thousand, by an ulp either way, and the difference's mean over
-2^17 slopes scatters by 1e-4; 0.005 is a fiftieth of rounding's own spread."""
+2^17 slopes scatters by 1e-4; 0.005 is a fiftieth of rounding's own spread.
+
+With a spacing that is no power of two the difference of heights is divided by
+it and rounded once more (a quarter of an ulp more in the square of the rms);
+its reciprocal's own rounding must not appear, which would move every slope of
+the line the same way by up to an ulp."""
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+LD = np.longdouble
 
 
 @pytest.mark.parametrize("lo,hi", [(-34, -29), (-28, -20), (-10, -4), (-4, -1), (-1, 1), (1, 6), (6, 8)])
@@ -51,3 +57,26 @@ def test_slope_rounds_to_nearest(Q, lo, hi):
     assert np.sqrt(np.mean(err ** 2)) <= 0.55, stat
     assert np.abs(err).max() <= 1.51, stat
 
+
+def test_slope_with_a_spacing_whose_reciprocal_rounds_far(Q):
+    """dx with 1 / dx almost half an ulp from a number: the slopes stay unbiased."""
+    import torch
+    rng = np.random.default_rng(4)
+    m = 1 << 15
+    n = 2 * (m + 1)
+    cand = rng.uniform(1.0, 2.0, 20000)
+    off = np.abs((1 / cand.astype(LD) - (1 / cand).astype(LD)) / np.spacing(1 / cand))
+    dx = float(cand[np.argmax(off)])
+    assert off.max() > 0.45
+    k = rng.integers(1 << 20, 1 << 21, m).astype(np.float64) * rng.choice([-1.0, 1.0], m)
+    dh = np.ldexp(2 * k + 1, -25)
+    line = np.repeat(np.concatenate([[0.0], np.cumsum(dh)]), 2)
+    length = float(n) * dx
+    x = dh.astype(LD) / (length / n)  # the spacing as the model forms it
+    got = -Q.gradient(torch.as_tensor(line, device="cuda"),
+                      Q.Params(length, 1.0, 0.0, Q.Model.Arclength), Q.ZeroNoise()).cpu().numpy()[1:-1:2]
+    want = x / np.sqrt(1 + x * x)
+    err = ((got - want) / np.spacing(np.abs(got))).astype(np.float64) * np.sign(dh)
+    # three roundings of at most a third of an ulp rms each, as seen in the
+    # slope's ulps; the mean of 2^15 of them scatters by 0.003
+    assert abs(err.mean()) <= 0.01 and np.sqrt(np.mean(err ** 2)) <= 0.6
