@@ -280,18 +280,21 @@ __device__ __forceinline__ double rk_forward_zero_pair(const Noise &nz, int i, i
 //   * March: lane j evaluates the point j serial steps ahead (lane 0 the
 //     start, so the first round holds v(h_i) too); the first v <= 0 brackets
 //     the zero between it and the point before.
-//   * Within a cell v is a quadratic, so the smaller end of its slope there
-//     follows from the cell's cubic. Where the bound over the bracket's cells
+//   * Within a cell v is a quadratic, so both ends of its slope there follow
+//     from the cell's cubic. Where the bound over the bracket's cells
 //     is positive (-dv/dh >= s > 0: the elastic slope 2 Gamma / dx outweighs
 //     the field's curvature), v falls all along and has one zero. A secant and
 //     a Newton step find it to about 1e-8, two evaluations either side bracket
-//     it, and a line between them gives it to rounding.
+//     it, and a line between them gives it up to the slope's change there and
+//     the rounding of v, which grows with each edge's own slope (the edges' may
+//     cancel in s) times the rounding of its height sum.
 //   * Bisection then only asks on which side of the zero its midpoints lie. In
 //     integers of the bracket's binade the midpoints are a grid where the width
 //     halves without a remainder (else the levels are replayed); a midpoint
 //     nearer to the zero than v's rounding errors over s is evaluated.
-// Anything else (a steep field, a bracket out of the two cells) takes the generic search. 200 sweeps of
-// a 2048-point line (16 taps): 39.0 -> 5.8 ms, of 16384 points 8.1 ms.
+// Anything else (a steep field, a bracket out of the two cells) takes the generic
+// search. 200 sweeps of
+// a 2048-point line (16 taps): 39.0 -> 6.1 ms.
 struct RkEdge {     // one edge's cubics in row cells iy and iy + 1
     long long p[2], u2[2], w[2];
     int d[2];  // the cells' units' orders below the field's (FxCubic)
@@ -316,9 +319,31 @@ struct RkFast {
     float slope0, bl[2], br[2];
 };
 
-// b 2^-d (0 where a float may not hold it).
+// b 2^-d for a cell's d (from 252 orders on it is far below any slope that counts).
 __device__ __forceinline__ float rk_scale(float b, int d) {
-    return d < 126 ? b * __int_as_float((127 - d) << 23) : 0.0f;
+    d = min(d, 252);
+    const int half = d >> 1;
+    return b * __int_as_float((127 - half) << 23) * __int_as_float((127 - d + half) << 23);
+}
+
+// An edge's b q over the window cells from k0 to k1: its smallest value, the
+// largest of its magnitude and of its change along a cell.
+struct RkSlope {
+    float lo, mag, bend;
+};
+__device__ __forceinline__ RkSlope rk_slope(const RkEdge &ed, const float b[2], int k0, int k1) {
+    RkSlope r{0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float q0 = (float)(int)(ed.u2[k] >> 32), q1 = (float)(int)((ed.u2[k] + 2 * ed.w[k]) >> 32);
+        const float s0 = b[k] * q0, s1 = b[k] * q1;
+        const bool first = k == k0, used = first || k == k1;
+        const float lo = fminf(s0, s1);
+        r.lo = used ? (first ? lo : fminf(r.lo, lo)) : r.lo;
+        r.mag = used ? fmaxf(r.mag, fmaxf(fabsf(s0), fabsf(s1))) : r.mag;
+        r.bend = used ? fmaxf(r.bend, fabsf(s1 - s0)) : r.bend;
+    }
+    return r;
 }
 
 // v(h) as rk_site_velocity gives it; s: -dv/dh; cl, cr: the window cells (-1:
@@ -340,12 +365,6 @@ __device__ __forceinline__ double rk_fast_velocity(const NoiseBSpline64 &nz, con
     const double dvl = __dmul_rn(fx_to_double(Rl, -(l1 ? F.l.d[1] : F.l.d[0])), F.l.unit);
     const double dvr = __dmul_rn(fx_to_double(Rr, -(r1 ? F.r.d[1] : F.r.d[0])), F.r.unit);
     return rk_velocity_of<NoiseBSpline64>(dvl, dvr, L, 0.0, 0.0, QEW_MODEL_LINEAR, h, F.hl, F.hr);
-}
-
-// The smaller b q of window cell k.
-__device__ __forceinline__ float rk_qmin(const RkEdge &ed, const float b[2], int k) {
-    const long long u = k ? ed.u2[1] : ed.u2[0], w = k ? ed.w[1] : ed.w[0];
-    return (k ? b[1] : b[0]) * fminf((float)(int)(u >> 32), (float)(int)((u + 2 * w) >> 32));
 }
 
 // One edge's place: its column, and general x weights where it needs them.
@@ -437,8 +456,10 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
     F.hl = hl;
     F.hr = hr;
     F.slope0 = (float)(-2.0 * L.c_el);
+    // the slopes are compared as floats, far from their range's ends
+    if (!(F.slope0 >= 1e-20f && F.slope0 <= 1e20f)) return false;
     double a = hi, advanced = 0.0, lo = 0.0, hc = 0.0, vlo = 0.0, vhc = 0.0;
-    float s, smin;
+    float s, smin, bend, mag_l, mag_r;
     int cl, cr;
     // The march takes at most ceil(max_advance / dstep) steps (validated on
     // the host), at least one a round.
@@ -486,10 +507,17 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
             vhc = __shfl_sync(gmask, v, j, G);
             const int l0 = __shfl_sync(gmask, cl, j - 1, G), l1 = __shfl_sync(gmask, cl, j, G);
             const int r0 = __shfl_sync(gmask, cr, j - 1, G), r1 = __shfl_sync(gmask, cr, j, G);
-            smin = F.slope0 + fminf(rk_qmin(F.l, F.bl, l0), rk_qmin(F.l, F.bl, l1)) +
-                   fminf(rk_qmin(F.r, F.br, r0), rk_qmin(F.r, F.br, r1));
+            const RkSlope sl = rk_slope(F.l, F.bl, l0, l1), sr = rk_slope(F.r, F.br, r0, r1);
+            mag_l = sl.mag;
+            mag_r = sr.mag;
+            bend = sl.bend + sr.bend;
+            // less what the floats round and the integers' upper halves leave out
+            smin = F.slope0 + sl.lo + sr.lo -
+                   (1.0e-6f * (F.slope0 + mag_l + mag_r) +
+                    2.0f * (fmaxf(F.bl[0], F.bl[1]) + fmaxf(F.br[0], F.br[1])));
             // a step as long as a period of the field could skip cells
-            if (!(l0 <= l1 && r0 <= r1 && rp.dstep < 2.0 * nz.dy && smin > 0.25f * F.slope0))
+            if (!(l0 <= l1 && r0 <= r1 && rp.dstep < 2.0 * nz.dy && smin > 0.25f * F.slope0 &&
+                  smin < 1e25f))
                 return false;
             break;
         }
@@ -521,14 +549,26 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
     const double v0 = __shfl_sync(gmask, vs, 0, G), v1 = __shfl_sync(gmask, vs, 1, G);
     const double x0 = __shfl_sync(gmask, side, 0, G);
     const double z = fma((double)((float)v0 / (float)(v0 - v1)), 2.0 * gap, x0);
-    // v's rounding errors, at most: the two sums of heights (the midpoints'
-    // through the field's slope, below 3/4 of the elastic one on each edge),
-    // the integers' conversion, the combine; and the line's own error
-    const float eps =
-        1.7e-16f * ((float)fabs(L.c_el) * (float)(fabs(hl) + fabs(hr) + 2.0 * fabs(hc)) +
-                    (float)fabs(L.fdx)) +
-        400.0f * (float)(L.half_dx * fmax(nz.fx_dv_c, nz.fx_dv_g));
-    const double g = (double)(3.0f * eps / smin) + 4.0 * ulp + 4.0e-7 * gap;
+    // v's rounding errors, at most, each within 2^-53 of its number (1.7e-16: and
+    // a half more): the sums of heights in the elastic part; each edge's
+    // midpoint (the sum, its quotient by the spacing, the fold of a negative one
+    // into the period) times that edge's own slope, the field's weight of which
+    // s knows only the sum; the force; and the integers' units and the
+    // conversions and products of dV/dy (R below 2^60: 700 units in all).
+    const float ah = (float)fabs(hc), al = (float)fabs(hl), ar = (float)fabs(hr);
+    const float period = 2.0f * (float)nz.ny * (float)nz.dy;
+    const float unit = (float)(2.0 * nz.dy * 0x1p-32) *
+                       fmaxf(fmaxf(F.bl[0], F.bl[1]), fmaxf(F.br[0], F.br[1]));
+    const float eps = 1.7e-16f * (2.0f * (float)fabs(L.c_el) * (al + ar + ah) + (float)fabs(L.fdx) +
+                                  mag_l * (2.0f * (al + ah) + period) +
+                                  mag_r * (2.0f * (ar + ah) + period)) +
+                      700.0f * unit;
+    // The line's zero is off by v's errors at its two points over s, by the
+    // change of the slope between them (bend / 2 dy a unit of height: half of
+    // that times gap^2 over s) and by the floats' quotient.
+    const float gf = (float)gap;
+    const double g = (double)((3.0f * eps + bend * (float)(0.25 * nz.inv_dy) * gf * gf) / smin) +
+                     4.0 * ulp + 4.0e-7 * gap;
     // v > 0 up to z0, v <= 0 from z1 on; the bracket's own ends are known. (A
     // site within its rounding of the zero, z0 <= bl, is what a line near its
     // critical force is made of.)
