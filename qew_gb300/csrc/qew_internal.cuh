@@ -447,17 +447,26 @@ struct NoiseBSpline64 {
         if (poly && ky == kPolyNotPow2) return fx_cell(a * (0.5 * inv_dy), 0, ny, iy, t);
         return fx_locate(a, 2.0 * dy, 0.5 * inv_dy, ky == kPolyNotPow2 ? ky : ky - 1, ny, iy, t);
     }
-    // dV/dy of an edge e < nx - 1 on the store.
-    __device__ __forceinline__ double dvdy_edge_store(int e, double a) const {
+    // dV/dy of an edge e < nx - 1 on the store as R 2^-d in units of fx_dv_c;
+    // false for a NaN.
+    __device__ __forceinline__ bool dvdy_edge_store(int e, double a, long long &R, int &d) const {
         int iy;
         FxFrac fy;
         if (!fx_row(a, iy, fy)) {
             double t;
             grid_locate(a * 0.5, dy, inv_dy, dy_pow2, ny, iy, t);
-            if (!(t >= 0.0)) return a - a;  // NaN
+            if (!(t >= 0.0)) return false;
             fy = fx_frac((unsigned long long)(fmin(t, 1.0 - 0x1p-53) * 0x1p64));
         }
-        return __dmul_rn(fx_dv(fx_const_cell(e, iy), fy), fx_dv_c);
+        const FxCubic q = fx_const_cell(e, iy);
+        R = fx_dt2(q, fy);
+        d = q.d;
+        return true;
+    }
+    __device__ __forceinline__ double dvdy_edge_store(int e, double a) const {
+        long long R;
+        int d;
+        return dvdy_edge_store(e, a, R, d) ? __dmul_rn(fx_to_double(R, -d), fx_dv_c) : a - a;
     }
     // dV/dy / V at the midpoint of edge e (xc its physical x, a the sum of its
     // two heights) in fixed point; what its locate declines (negative or huge

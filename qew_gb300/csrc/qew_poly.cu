@@ -20,6 +20,8 @@
 #include <climits>
 #include <cmath>
 
+#include <math_constants.h>
+
 #include "qew_internal.cuh"
 #include "qew_model_kernels.cuh"
 #include "qew_poly.cuh"
@@ -41,9 +43,8 @@ struct PolyGeom {
     float inv_ny;
 };
 
-// dV/dy of an edge that the integers do not cover (the wrap edge, a chunk of
-// FP64 sums): out of line, so that its general path takes no registers of
-// the kernels' loops.
+// dV/dy of an edge that the store does not cover (the wrap edge): out of line,
+// so that its general path takes no registers of the kernels' loops.
 __device__ __noinline__ double walk_edge_rare(const PolyGeom &g, int e, double sum) {
     const int ep = (e + 1 == g.n) ? 0 : e + 1;
     return g.nz.dvdy_edge_sum(e, EdgeX{e + ep, g.L.dx}, sum);
@@ -141,15 +142,16 @@ k_gradient_poly(const double *__restrict__ h, const __grid_constant__ PolyGeom g
 // The linear gradient with the heights themselves as integers. A warp takes
 // chunks of 255 consecutive sites, the 256 edges about them in 8 steps of 32;
 // the chunk's 257 heights become signed integers in the unit 2^-8 of the ulp
-// of the largest one: exactly, but for bits of heights more than 2^8
-// below it, cut at 2^-8 of the ulp that FP64 sums beside the largest round
-// at. The midpoint sum, its row cell (folded into the field's period) and
+// of the largest one: exactly down to 2^-8 of it, smaller ones cut at that
+// unit, which FP64's sum with a neighbour rounds coarser as long as one of the
+// two is above 2^-7 of the largest. The midpoint sum, its row cell (folded into the field's period) and
 // fraction, dV/dy and the second difference of the heights are then integer
 // sums and products, and a site takes two FP64 instructions (the combine)
 // for seven before:
 //   grad = c_el d2h + (half_unit (R_l + R_r) - dx f).
-// A chunk with a non-finite height, or heights too small or too large beside
-// the row spacing, takes the FP64 sums of k_gradient_poly. Chunks start at
+// A chunk with two neighbours below that, a non-finite height, or heights too
+// small or too large beside the row spacing (a flat line at 0) takes FP64 sums
+// (walk_chunk_fp64). Chunks start at
 // multiples of 255 of their line, whatever the launch, so every launch shape
 // and batch gives the same bits.
 constexpr int kWalkSteps = 8;
@@ -180,11 +182,59 @@ __device__ __forceinline__ long long walk_edge(const PolyGeom &g, int e, long lo
 }
 
 // v of the next lane; the last lane gets `wrap` of the first one.
-__device__ __forceinline__ long long lane_next(long long v, long long wrap, int lane) {
+template <class T>
+__device__ __forceinline__ T lane_next(T v, T wrap, int lane) {
     return __shfl_sync(0xffffffffu, lane == 0 ? wrap : v, (lane + 1) & 31);
 }
 
-// Gradient of site i from FP64 sums and edges.
+// Both edges' dV/dy, each in its cell's unit, as an integer in the unit of the
+// larger, ds orders below the field's.
+__device__ __forceinline__ long long walk_pair(long long Rl, int dl, long long Rr, int dr, int &ds) {
+    ds = min(dl, dr);
+    return fx_sar(Rl, dl - ds) + fx_sar(Rr, dr - ds);
+}
+
+// The chunk's gradients from FP64 sums of heights, a lane an edge as in
+// walk_chunk: 5 FP64 instructions a site. Out of line, as walk_edge_rare.
+__device__ __noinline__ void walk_chunk_fp64(const PolyGeom &g, const double *hl, double *out, int s0,
+                                             int lane, const double *hs) {
+    const int n = g.n;
+    auto height = [&](int j) {  // of site s0 - 1 + j
+        const int i = s0 - 1 + j;
+        return hs ? hs[j] : __ldg(hl + (i < 0 ? n - 1 : i < n ? i : 0));
+    };
+    double h = height(lane), hb = 0.0, hpb = 0.0;  // b: of the step before
+    long long Rb = 0;
+    int db = 0;  // -1: a NaN
+    for (int k = 0; k <= kWalkSteps; ++k) {
+        double hp = 0.0, hn = 0.0;
+        long long R = 0;
+        int d = 0;
+        if (k < kWalkSteps) {
+            hn = k + 1 < kWalkSteps ? height(32 * (k + 1) + lane) : height(kWalkEdges);
+            hp = lane_next(h, hn, lane);
+            const int e = s0 - 1 + 32 * k + lane;
+            if (e >= 0 && e + 1 < n && !g.nz.dvdy_edge_store(e, hp + h, R, d)) d = -1;
+        }
+        if (k > 0) {  // the sites of the step before
+            const int i = s0 + 32 * (k - 1) + lane;
+            const double hr = lane_next(hpb, hp, lane);
+            const int dr = lane_next(db, d, lane);
+            int ds;
+            const long long S = walk_pair(Rb, db, lane_next(Rb, R, lane), dr, ds);
+            const double dv = ds < 0 ? CUDART_NAN : fx_to_double(S, -ds);
+            if (i > 0 && i + 1 < n && (k < kWalkSteps || lane < 31))
+                out[i - s0] = fma(g.L.c_el, fma(-2.0, hpb, hb + hr), fma(g.half_unit, dv, -g.L.fdx));
+        }
+        hb = h;
+        hpb = hp;
+        Rb = R;
+        db = d;
+        h = hn;
+    }
+}
+
+// Gradient of site i (a wrap site) from FP64 sums and edges.
 __device__ __noinline__ double walk_site_rare(const PolyGeom &g, const double *hl, int i) {
     const int n = g.n;
     const int im = i == 0 ? n - 1 : i - 1, ip = i + 1 == n ? 0 : i + 1;
@@ -212,16 +262,33 @@ __device__ __forceinline__ void walk_chunk(const double *__restrict__ hl, const 
     }
     const int il = s0 - 1 + kWalkEdges;  // right end of the last edge
     const double last = kStage && hs ? hs[kWalkEdges] : __ldg(hl + (il < n ? il : 0));
-    // the largest exponent of the chunk
-    unsigned mx = (unsigned)__double2hiint(last) << 1;
+    // the largest and the smallest exponent of the chunk
+    unsigned mx = (unsigned)__double2hiint(last) << 1, mn = mx;
 #pragma unroll
-    for (int k = 0; k < kWalkSteps; ++k) mx = max(mx, (unsigned)__double2hiint(x[k]) << 1);
+    for (int k = 0; k < kWalkSteps; ++k) {
+        const unsigned b = (unsigned)__double2hiint(x[k]) << 1;
+        mx = max(mx, b);
+        mn = min(mn, b);
+    }
     mx = __reduce_max_sync(0xffffffffu, mx) >> 21;
+    mn = __reduce_min_sync(0xffffffffu, mn) >> 21;
     // midpoint in cells = a 2^-sh for a in units of 2^(mx - 1075 - guard)
     const int sh = 1075 + kWalkGuard - (int)mx - g.ky;
-    if (!(mx < 2047u && mx > 200u && sh >= 40 && sh <= 63)) {
-        for (int j = lane; j < kWalkSites; j += 32)
-            if (s0 + j > 0 && s0 + j + 1 < n) out[j] = walk_site_rare(g, hl, s0 + j);
+    bool whole = mx < 2047u && mx > 200u && sh >= 40 && sh <= 63;
+    if (whole && mn + 7 < mx) {  // two neighbours that small: the integers would cut their sum
+        auto large = [&](double v) {
+            return __ballot_sync(0xffffffffu, (((unsigned)__double2hiint(v) << 1) >> 21) + 7 >= mx);
+        };
+        unsigned b = large(x[0]);
+#pragma unroll
+        for (int k = 0; k < kWalkSteps; ++k) {
+            const unsigned nb = large(k + 1 < kWalkSteps ? x[k + 1 < kWalkSteps ? k + 1 : 0] : last);
+            whole = whole && (b | __funnelshift_r(b, nb, 1)) == 0xffffffffu;
+            b = nb;
+        }
+    }
+    if (!whole) {
+        walk_chunk_fp64(g, hl, out, s0, lane, kStage ? hs : nullptr);
         return;
     }
     auto fix = [&](double v) {
@@ -250,10 +317,8 @@ __device__ __forceinline__ void walk_chunk(const double *__restrict__ hl, const 
         }
         if (k > 0) {  // the sites of the step before
             const int i = s0 + 32 * (k - 1) + lane;
-            const long long Rn = lane_next(Rb, R, lane);
-            const int dn = __shfl_sync(0xffffffffu, lane == 0 ? d : db, (lane + 1) & 31);
-            const int ds = min(db, dn);  // both edges in the unit of the larger
-            const long long S = fx_sar(Rb, db - ds) + fx_sar(Rn, dn - ds);
+            int ds;
+            const long long S = walk_pair(Rb, db, lane_next(Rb, R, lane), lane_next(db, d, lane), ds);
             const long long D = lane_next(sb, sl, lane) - sb;
             if (i > 0 && i + 1 < n && (k < kWalkSteps || lane < 31)) {
                 const double v = fma(g.L.c_el, fx_to_double(D, ek),
