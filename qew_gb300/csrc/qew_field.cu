@@ -31,17 +31,19 @@ namespace {
 //   c[k] = g (y[k] + z w[k+1]),  g = -6 z / (1 - z^2) = sqrt(3),
 // which equals the cascade c = -6 z anticausal(causal(s)). A chunk starts
 // each recursion kWarm samples away from zero, reading the periodic
-// neighbours: the neglected tail is z^kWarm = 5e-19 of the signal, so every
-// output equals the exact periodic solve up to rounding, for any N (the
-// warm-up wraps for short N). Lines are m = 0..M-1 at stride `lst`; samples
+// neighbours: the neglected tail is z^kWarm = 2.5e-37 of a sample that far away,
+// so every output equals the exact periodic solve up to its own rounding, for
+// any N (the warm-up wraps for short N), beside samples 1e20 times larger too. Lines are m = 0..M-1 at stride `lst`; samples
 // at stride `st`; consecutive threads take consecutive lines so each step's
 // accesses coalesce when lst == 1. FP64-bound: 4 instructions a sample (5
 // with the gain, which the last axis applies for both, times the field's
-// scale where one is given) and a half for the warm-ups. 4096 x 1024, both
-// axes: 284 -> 109 us (the cascade's four passes before).
+// scale where one is given) and as much again for the warm-ups. 4096 x 1024, both
+// axes: 284 -> 127 us (the cascade's four passes before; 109 with warm-ups of
+// 32, whose tail of 5e-19 is no longer below rounding where a weak region lies
+// beside strong samples).
 constexpr double kPole = -0.26794919243112270;  // sqrt(3) - 2
 constexpr int kChunk = 64;
-constexpr int kWarm = 32;
+constexpr int kWarm = 64;
 constexpr int kPreBS = 128;
 
 __device__ __forceinline__ int pmod(long k, int N) {
