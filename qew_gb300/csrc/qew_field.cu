@@ -181,13 +181,13 @@ __global__ void k_sample(Noise nz, const double *__restrict__ x, const double *_
 // (the real-space form of exp(-(2 pi xi f)^2 / 2) in Fourier space; taps to
 // |k| <= ceil(5 xi), normalised so the sum of squared taps is 1), in the
 // reference's host layout [nx][ny].
-// The filter runs in 64-bit fixed point (qew_fix.cuh): the noise is bounded
-// (|z| < 8.58 from 53-bit uniforms), so it and the taps lose nothing, and a
-// tap pair costs four 32 x 32 + 64-bit multiply-adds (about 5 cycles each) where
+// The filter runs in 64-bit fixed point (qew_fix.cuh): the noise and the filtered
+// sums are bounded (ConvUnits), samples are rounded at 2^-55 and 2^-53 and the taps
+// at 2^-59 of unity, so the field's error stays below 4e-16 of its deviation at
+// any xi, where FP64 sums of 41000 terms (xi = 4096) come to 8e-15; a tap pair costs four 32 x 32 + 64-bit multiply-adds (about 5 cycles each) where
 // FP64 takes two 64-cycle instructions: 306 -> 150 us an axis of a 4096 x 1024
 // field at xi = 4 (41 taps), 115 with four outputs a thread. A sample is X = X1 2^30 + X0 in units 2^-F,
-// |X| < 2^59; a tap T = T1 2^30 + T0 in units 2^-q, q such that the taps'
-// sum is at most 2^58.
+// |X| < 2^59; a tap T = T1 2^30 + T0 <= 2^58 in units 2^-q.
 constexpr double kNoiseMax = 8.58;  // sqrt(2 ln 2^53) = 8.572
 
 __global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_t seed, int F) {
@@ -203,8 +203,9 @@ __global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_
     int k;
     fx_normal_pair(a + 1, b, g_fx_logs, g_fx_turns, z0, z1, k);  // z 2^k, k <= -F
     const int sh = min(-k - F, 63);
-    w[(size_t)(2 * jp) * nx + i] = z0 >> sh;  // [ny][nx]
-    if (2 * jp + 1 < ny) w[(size_t)(2 * jp + 1) * nx + i] = z1 >> sh;
+    const long long half = sh > 0 ? 1ll << (sh - 1) : 0;
+    w[(size_t)(2 * jp) * nx + i] = (z0 + half) >> sh;  // [ny][nx]
+    if (2 * jp + 1 < ny) w[(size_t)(2 * jp + 1) * nx + i] = (z1 + half) >> sh;
 }
 
 // out[p] = sum_k tap[|k|] in[p + k] along the slow axis of in[len][width] (both
@@ -212,7 +213,8 @@ __global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_
 // in the same layout, times 2^exp; else fixed point, shifted right by exp, as
 // out[width][len], so that the other axis is the slow one next.
 // The partial products of weight 2^60, 2^30 and 1 have sums of their own, the
-// lower two folded every four pairs before they can overflow (2^61 a pair).
+// lower two folded, rounded to 2^44, every four pairs before they can overflow
+// (2^61 a pair); the whole is in units of 2^(60 - up).
 // A thread takes 4 consecutive outputs: a step in k then needs two new samples
 // for the four (they slide through registers, split into their 30-bit halves
 // once) where an output alone loads and splits both ends of every pair; what
@@ -220,7 +222,7 @@ __global__ void k_white_noise(long long *__restrict__ w, int nx, int ny, uint64_
 template <bool kLast, int kOut>
 __global__ void __launch_bounds__(256)
 k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int len, int width,
-             const int2 *__restrict__ tap, int R, int exp, int lsh) {
+             const int2 *__restrict__ tap, int R, int exp, int up, int lsh) {
     // a block is 2^lsh lanes wide and 256 / 2^lsh threads along the slow axis,
     // whose windows overlap in L1
     const unsigned tiles = ((unsigned)width + (1u << lsh) - 1u) >> lsh;
@@ -230,6 +232,8 @@ k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int len, 
     if (l >= width || pl >= len) return;
     const int p0 = (int)pl;
     constexpr int kLow = (1 << 30) - 1;
+    constexpr long long kHalfM = 1ll << 13;  // of the folds' rounding
+    constexpr unsigned long long kHalfL = 1ull << 43;
     int a1[kOut], a0[kOut], b1[kOut], b0[kOut];  // samples at p0 + u - k and p0 + u + k
     auto get = [&](int p, int &x1, int &x0) {
         const long long x = __ldg(in + (size_t)p * (size_t)width + l);
@@ -248,8 +252,8 @@ k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int len, 
 #pragma unroll
         for (int u = 0; u < kOut; ++u) {
             A[u] += (M[u] >> 14) + (long long)(L[u] >> 44);
-            M[u] = 0;
-            L[u] = 0;
+            M[u] = kHalfM;
+            L[u] = kHalfL;
         }
     };
     {
@@ -257,8 +261,9 @@ k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int len, 
         int p = p0;
 #pragma unroll
         for (int u = 0; u < kOut; ++u) {
-            P[u] = M[u] = A[u] = 0;
-            L[u] = 0;
+            P[u] = A[u] = 0;
+            M[u] = kHalfM;
+            L[u] = kHalfL;
             get(p, a1[u], a0[u]);
             b1[u] = a1[u];
             b0[u] = a0[u];
@@ -294,7 +299,12 @@ k_gauss_conv(const long long *__restrict__ in, void *__restrict__ out, int len, 
     fold();
     long long v[kOut];
 #pragma unroll
-    for (int u = 0; u < kOut; ++u) v[u] = (P[u] << 5) + (A[u] >> 11);  // units of 2^55
+    for (int u = 0; u < kOut; ++u) v[u] = (P[u] << up) + (A[u] >> (16 - up));
+    if (!kLast) {
+        const long long half = (1ll << exp) >> 1;
+#pragma unroll
+        for (int u = 0; u < kOut; ++u) v[u] += half;
+    }
     const int cnt = min(kOut, len - p0);
     if (kLast) {
         double *o = (double *)out + (size_t)p0 * (size_t)width + l;
@@ -386,14 +396,14 @@ double fft_freq(int k, int n) {
     return (double)ks / (double)n;
 }
 
-// Taps 0..R of the normalised symmetric filter in fixed point (units 2^-q),
-// and the bound on the filter's gain (the taps' sum).
-std::vector<int2> gauss_taps(double xi, int &R, int &q, double &gain) {
+// Taps 0..R of the normalised symmetric filter; its gain (the taps' sum), and its
+// norm on len periodic samples (1, more where the filter wraps onto itself).
+std::vector<double> gauss_taps(double xi, int len, int &R, double &gain, double &norm) {
     R = (xi > 0) ? (int)ceil(5.0 * xi) : 0;
     std::vector<double> t(R + 1);
     double s2 = 0.0;
     for (int k = -R; k <= R; ++k) {
-        const double v = (xi > 0) ? exp(-0.5 * (double)k * k / (xi * xi)) : 1.0;
+        const double v = (xi * xi > 0) ? exp(-0.5 * (double)k * k / (xi * xi)) : (k == 0 ? 1.0 : 0.0);
         if (k >= 0) t[k] = v;
         s2 += v * v;
     }
@@ -402,14 +412,33 @@ std::vector<int2> gauss_taps(double xi, int &R, int &q, double &gain) {
         t[k] /= sqrt(s2);
         gain += (k ? 2.0 : 1.0) * t[k];
     }
-    q = 58 - std::max(0, (int)ceil(log2(gain)));
-    std::vector<int2> T(R + 1);
-    for (int k = 0; k <= R; ++k) {
-        const long long v = llrint(ldexp(t[k], q));
-        T[k] = make_int2((int)(v >> 30), (int)(v & ((1 << 30) - 1)));
-    }
-    return T;
+    const int period = std::min(len, 2 * R + 1);
+    std::vector<double> folded(period, 0.0);
+    for (int k = 0; k <= 2 * R; ++k) folded[k % period] += t[k < R ? R - k : k - R];
+    norm = 0.0;
+    for (double v : folded) norm += v * v;
+    norm = sqrt(norm);
+    return t;
 }
+
+// One filter pass's fixed point. Its sums are bounded by `bound`: |z| < 8.58 for
+// the noise (53-bit uniforms) times the gain, or 40 standard deviations (a
+// normal number exceeds that once in 10^350), whichever is less, as every sum of
+// a part of the taps is. With b = ceil(log2 bound), samples in units 2^-F and
+// taps in 2^-q, q <= 58, the sum of the upper products stays below 2^62, and the
+// whole in units of 2^U, U = F + q + b - 62, as well.
+struct ConvUnits {
+    int q, b, up;  // up = 60 - U
+    std::vector<int2> tap;
+    ConvUnits(const std::vector<double> &t, int F, double bound) : b((int)ceil(log2(bound))) {
+        q = std::min(58, 122 - F - b);
+        up = 60 - (F + q + b - 62);
+        for (double v : t) {
+            const long long T = llrint(ldexp(v, q));
+            tap.push_back(make_int2((int)(T >> 30), (int)(T & ((1 << 30) - 1))));
+        }
+    }
+};
 
 // scale (a device number, or null) multiplies the field.
 qew_status field_build(qew_ctx *ctx, const double *src, bool src_on_device, int nx,
@@ -545,13 +574,17 @@ qew_status qew_field_create_generated(qew_ctx *ctx, int nx, int ny, double Lx, d
         return qew_fail(ctx, QEW_ERR_INVALID, "field_create_generated: bad arguments");
     QEW_CUDA(ctx, cudaSetDevice(ctx->device));
     const size_t N = (size_t)nx * ny;
-    int Rx, Ry, qx, qy;
-    double gx, gy;
-    const std::vector<int2> tx = gauss_taps(xi_x_cells, Rx, qx, gx);
-    const std::vector<int2> ty = gauss_taps(xi_y_cells, Ry, qy, gy);
+    int Rx, Ry;
+    double gx, gy, sx, sy;
+    const std::vector<double> wx = gauss_taps(xi_x_cells, nx, Rx, gx, sx);
+    const std::vector<double> wy = gauss_taps(xi_y_cells, ny, Ry, gy, sy);
     // samples in [-2^59, 2^59): 2^-F1 for the noise, 2^-F2 after the y filter
+    const double by = std::min(kNoiseMax * gy, 40.0 * sy), bx = std::min(by * gx, 40.0 * sx * sy);
     const int F1 = 59 - (int)ceil(log2(kNoiseMax));
-    const int F2 = 59 - std::max(0, (int)ceil(log2(kNoiseMax * gy)));
+    const ConvUnits uy(wy, F1, by);
+    const int F2 = 59 - uy.b;
+    const ConvUnits ux(wx, F2, bx);
+    const std::vector<int2> &tx = ux.tap, &ty = uy.tap;
     long long *w = nullptr, *t = nullptr;
     double *stat = nullptr;
     auto cleanup = [&](qew_status s) {
@@ -574,13 +607,13 @@ qew_status qew_field_create_generated(qew_ctx *ctx, int nx, int ny, double Lx, d
     if (e != cudaSuccess) return cleanup(qew_fail(ctx, QEW_ERR_CUDA, "%s", cudaGetErrorString(e)));
     const long pairs = (long)nx * ((ny + 1) / 2);
     k_white_noise<<<(unsigned)((pairs + 255) / 256), 256, 0, ctx->stream>>>(w, nx, ny, seed, F1);
-    // a filtered sum is in units of 2^(55 - F - q) (k_gauss_conv); w [ny][nx] ->
-    // t [nx][ny] -> w [nx][ny]
+    // a filtered sum is in units of 2^(U - F - q) = 2^(b - 62); the first one's
+    // samples of 2^-F2 are 3 bits coarser. w [ny][nx] -> t [nx][ny] -> w [nx][ny]
     // one output a thread where four would idle threads (len < 4) or scatter
     // the lanes' loads (a field of few columns): 2^20 x 1 at xi = 3 386 us so,
     // 488 with four; 2^18 x 8 314 with four, 341 so
     auto conv = [&](auto last, auto outs, const long long *in, void *out, int len, int width,
-                    const int2 *tap, int R, int exp) {
+                    const int2 *tap, int R, int exp, int up) {
         constexpr int kOut = decltype(outs)::value;
         int lsh = 0;  // 32 lanes along the fast axis, fewer only on a narrower field
         while (lsh < 5 && (1 << lsh) < width) ++lsh;
@@ -588,16 +621,16 @@ qew_status qew_field_create_generated(qew_ctx *ctx, int nx, int ny, double Lx, d
         const long long per = (long long)kOut << (8 - lsh);
         k_gauss_conv<decltype(last)::value, kOut>
             <<<(unsigned)(tiles * ((len + per - 1) / per)), 256, 0, ctx->stream>>>(
-                in, out, len, width, tap, R, exp, lsh);
+                in, out, len, width, tap, R, exp, up, lsh);
     };
     using One = std::integral_constant<int, 1>;
     using Four = std::integral_constant<int, 4>;
     if (ny >= 4 && nx >= 4) {
-        conv(std::false_type{}, Four{}, w, t, ny, nx, tapy, Ry, F1 + qy - 55 - F2);
-        conv(std::true_type{}, Four{}, t, w, nx, ny, tapx, Rx, 55 - F2 - qx);
+        conv(std::false_type{}, Four{}, w, t, ny, nx, tapy, Ry, 3, uy.up);
+        conv(std::true_type{}, Four{}, t, w, nx, ny, tapx, Rx, ux.b - 62, ux.up);
     } else {
-        conv(std::false_type{}, One{}, w, t, ny, nx, tapy, Ry, F1 + qy - 55 - F2);
-        conv(std::true_type{}, One{}, t, w, nx, ny, tapx, Rx, 55 - F2 - qx);
+        conv(std::false_type{}, One{}, w, t, ny, nx, tapy, Ry, 3, uy.up);
+        conv(std::true_type{}, One{}, t, w, nx, ny, tapx, Rx, ux.b - 62, ux.up);
     }
     qew_status st = qew_launch_check(ctx, "field_generate", 3);
     if (st != QEW_OK) return cleanup(st);
