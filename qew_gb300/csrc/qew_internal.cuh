@@ -816,11 +816,13 @@ static inline NoiseBSpline64 make_bspline64(const qew_field *f, int n = 0,
     nz.fx_dv_c = nz.fx_v_c = nz.fx_dv_g = nz.fx_v_g = 0.0;
     if (f->fixb >= 0 && qew_fixed_div_ok(f->dx) && qew_fixed_div_ok(f->dy)) {
         const int K = f->fixb - 1022;  // |coefficient| < 2^K
-        nz.kb = f->fixb;
         nz.fx_dv_c = ldexp(1.0, K - 53) / (48.0 * f->dy);
         nz.fx_v_c = ldexp(1.0, K - 52) / 288.0;
         nz.fx_dv_g = ldexp(1.0, K - 58) / f->dy;
         nz.fx_v_g = ldexp(1.0, K - 57) / 6.0;
+        // the units and R times them stay normal numbers, else FP64 sums
+        if (fmin(nz.fx_dv_g, nz.fx_v_g) > 0x1p-700 && fmax(nz.fx_dv_c, nz.fx_v_c) < 0x1p+900)
+            nz.kb = f->fixb;
     }
 #ifdef QEW_BOUNDS_CHECK
     nz.oob = qew_bounds_words();

@@ -487,7 +487,9 @@ qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count
     g.half_unit = g.L.half_dx * g.nz.fx_dv_c;
     g.inv_ny = 1.0f / (float)f->ny;
     const bool arc = (p->model == QEW_MODEL_ARCLENGTH);
-    const bool walk = !arc && std::isfinite(g.half_unit);
+    const bool walk = !arc;  // k_gradient_poly is for arclength
+    // (dx / 2 times the unit leaves FP64's range: FP64 sums and combine)
+    if (walk && !(g.half_unit > 0x1p-700 && g.half_unit < 0x1p+900)) return QEW_ERR_UNSUPPORTED;
     // Candidates; every one computes the same numbers (the per-site
     // arithmetic does not depend on the launch): sites per thread {1, 2, 4} x
     // resident CTAs per SM {2, 3, 4}, default 2 sites, 4 CTAs; for the walk
