@@ -25,6 +25,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 // Fraction limbs: t = (t1 * 2^31 + t0) * 2^-62.
 struct FxFrac {
     int t1, t0;
@@ -130,17 +132,30 @@ __device__ __forceinline__ double fx_to_double(long long r, int k = 0) {
     return __longlong_as_double((long long)fx_double_bits(r, k));
 }
 
+__host__ __device__ __forceinline__ unsigned long long fx_bits(double a) {
+#ifdef __CUDA_ARCH__
+    return (unsigned long long)__double_as_longlong(a);
+#else
+    unsigned long long b;
+    memcpy(&b, &a, sizeof(b));
+    return b;
+#endif
+}
+
 // Row cell and fraction of g = a * 2^k in a period of n cells, from the bits
 // of a: the numbers that the reference's fold gives (filtered_noise.h:80-92),
 // which rounds a negative g's sum with the period to FP64. False for what the
-// FP64 code has to decide: non-finite or subnormal a, |g| >= 2^30, and the
-// last cell of a period other than the first two about zero, where the
-// reference's division by the period may round up.
-__device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &iy, unsigned long long &f) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+// FP64 code has to decide: non-finite or subnormal a, |g| >= 2^50, and, outside
+// the first two periods about zero, the last two FP64 numbers of a period,
+// where the reference's division by the period may round up. (Declining the
+// whole last cell, and |g| >= 2^30, made 8 lines of 2^20 points there 1530 us on 16
+// taps where FP64 alone took 1166; now 244 and 263.)
+__host__ __device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &iy,
+                                                   unsigned long long &f) {
+    const unsigned long long b = fx_bits(a);
     const int ef = (int)(b >> 52) & 0x7FF;
     const int e = ef + k - 1023;
-    if (ef == 0 || ef == 2047 || e > 29) {
+    if (ef == 0 || ef == 2047 || e > 49) {
         iy = 0;
         f = 0ull;
         return (b << 1) == 0ull;
@@ -149,28 +164,38 @@ __device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &iy, unsig
     const int up = 12 + e;  // fraction bits to the top of 64 (the integer part leaves)
     f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
     iy = e >= 0 ? (int)fx_shr(m, 52 - e) : 0;
-    bool ok = true;
-    if ((long long)b < 0) {
-        if (n == 1) return false;
-        ok = iy < n;
-        iy = f ? -iy - 1 : -iy;
-        f = 0ull - f;
-        iy %= n;
-        if (iy < 0) iy += n;
-        ok = ok || iy + 1 < n;
-        if (iy > 0) {  // round g + period to FP64 (to nearest even)
-            const int drop = 43 - __clz(iy);  // 12 + floor(log2(iy))
-            const unsigned long long add = ((1ull << (drop - 1)) - 1ull) + ((f >> drop) & 1ull);
-            const bool carry = f + add < f;
-            f = ((f + add) >> drop) << drop;
-            if (carry) {
-                f = 0ull;
-                iy = (iy + 1 == n) ? 0 : iy + 1;
-            }
-        }
+    bool later = false;  // than the two periods about zero
+    if (e > 29) {        // up to 50 bits: whole periods taken out in 64-bit arithmetic
+        const unsigned long long whole = fx_shr(m, 52 - e);
+        later = whole >= (unsigned long long)n;
+        iy = (int)(whole % (unsigned long long)n);
     } else if (iy >= n) {
+        later = true;
         iy %= n;
-        ok = iy + 1 < n;
+    }
+    // the fraction after a fold, two units of a's last bit or more before the end
+    const auto inside = [&]() { return f < 0ull - fx_shl(2ull, up); };
+    if ((long long)b >= 0) return !later || iy + 1 < n || inside();
+    if (n == 1) return false;
+    // bits below 2^-64 leave a mark in the lowest one, for the sums with the
+    // period that lie next to halfway between two numbers
+    const bool cut = up < 0 && fx_shl(f, -up) != m;
+    iy = (f || cut) ? n - 1 - iy : (iy ? n - iy : 0);
+    f = cut ? ~f | 1ull : 0ull - f;
+    const bool ok = !later || iy + 1 < n || inside();
+    if (iy > 0) {  // round g + period to FP64 (to nearest even)
+#ifdef __CUDA_ARCH__
+        const int drop = 43 - __clz(iy);  // 12 + floor(log2(iy))
+#else
+        const int drop = 43 - __builtin_clz((unsigned)iy);
+#endif
+        const unsigned long long add = ((1ull << (drop - 1)) - 1ull) + ((f >> drop) & 1ull);
+        const bool carry = f + add < f;
+        f = ((f + add) >> drop) << drop;
+        if (carry) {
+            f = 0ull;
+            iy = (iy + 1 == n) ? 0 : iy + 1;
+        }
     }
     return ok;
 }

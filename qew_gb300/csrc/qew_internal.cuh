@@ -268,7 +268,8 @@ struct NoiseBSpline64;
 // NoiseBSpline64::dvdy (deriv) / value out of line: the FP64 16-tap sum, for
 // the few edges that the fixed-point gather declines.
 static __device__ __noinline__ double bspline_slow_call(const double *coef, int nx, int ny, double dx,
-                                                        double dy, double x, double y,
+                                                        double dy, double inv_dx, double inv_dy,
+                                                        double x, double y,
                                                         bool deriv QEW_OOB_WORDS);
 __device__ __forceinline__ double bspline_slow(const NoiseBSpline64 &nz, bool deriv, double x,
                                                double y);
@@ -469,7 +470,7 @@ struct NoiseBSpline64 {
         return dvdy_edge_store(e, a, R, d) ? __dmul_rn(fx_to_double(R, -d), fx_dv_c) : a - a;
     }
     // dV/dy / V at the midpoint of edge e (xc its physical x, a the sum of its
-    // two heights) in fixed point; what its locate declines (negative or huge
+    // two heights) in fixed point; what its locate declines (a rounded period end, huge
     // heights, non-finite ones) is summed in FP64. The last product is never
     // contracted, so every kernel gets the same bits.
     __device__ __forceinline__ double dvdy_edge_sum(int e, EdgeX xc, double a) const {
@@ -551,7 +552,8 @@ struct NoiseBSpline64 {
 };
 
 static __device__ __noinline__ double bspline_slow_call(const double *coef, int nx, int ny, double dx,
-                                                        double dy, double x, double y,
+                                                        double dy, double inv_dx, double inv_dy,
+                                                        double x, double y,
                                                         bool deriv QEW_OOB_WORDS) {
     NoiseBSpline64 nz;
     nz.coef = coef;
@@ -559,8 +561,8 @@ static __device__ __noinline__ double bspline_slow_call(const double *coef, int 
     nz.ny = ny;
     nz.dx = dx;
     nz.dy = dy;
-    nz.inv_dx = 1.0 / dx;
-    nz.inv_dy = 1.0 / dy;
+    nz.inv_dx = inv_dx;
+    nz.inv_dy = inv_dy;
     nz.dx_pow2 = dbl_is_pow2(dx);
     nz.dy_pow2 = dbl_is_pow2(dy);
 #ifdef QEW_BOUNDS_CHECK
@@ -571,9 +573,9 @@ static __device__ __noinline__ double bspline_slow_call(const double *coef, int 
 __device__ __forceinline__ double bspline_slow(const NoiseBSpline64 &nz, bool deriv, double x,
                                                double y) {
 #ifdef QEW_BOUNDS_CHECK
-    return bspline_slow_call(nz.coef, nz.nx, nz.ny, nz.dx, nz.dy, x, y, deriv, nz.oob);
+    return bspline_slow_call(nz.coef, nz.nx, nz.ny, nz.dx, nz.dy, nz.inv_dx, nz.inv_dy, x, y, deriv, nz.oob);
 #else
-    return bspline_slow_call(nz.coef, nz.nx, nz.ny, nz.dx, nz.dy, x, y, deriv);
+    return bspline_slow_call(nz.coef, nz.nx, nz.ny, nz.dx, nz.dy, nz.inv_dx, nz.inv_dy, x, y, deriv);
 #endif
 }
 
