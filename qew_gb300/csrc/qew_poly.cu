@@ -350,10 +350,13 @@ k_gradient_poly_walk(const double *__restrict__ h, const __grid_constant__ PolyG
 // memory in aligned 128-byte pieces while the run before is computed, and
 // whose gradients leave the same way. 255-site runs of a warp touch a third
 // line for every two, and the host link pays for each: 8 lines of 2^20 in
-// pinned memory 14.5 G points/s with them, 17.9 so. Two blocks an SM: the link
-// gives less when more is in flight (17.4 with three, 16.7 with four).
+// pinned memory 14.5 G points/s with them, 19.3 so. Fewer blocks than SMs: the
+// link gives less when more is in flight (two blocks an SM 17.8, one 18.0, four
+// for five SMs 19.0, seven for ten 19.3, one for two 14.7; the kernel of
+// 256-site tiles on FP64 sums that was here before the walk 19.65). So there are
+// registers to spare, and a warp's eight gathers are in flight together.
 template <bool kPow2>
-__global__ void __launch_bounds__(kBS, 4)
+__global__ void __launch_bounds__(kBS, 2)
 k_gradient_poly_walk_host(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
                           double *__restrict__ grad, int chunks, long long units) {
     constexpr int kWarps = kBS / 32, kRun = kWarps * kWalkSites;
@@ -511,7 +514,7 @@ qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count
             if (blocks > INT_MAX)
                 return qew_fail(ctx, QEW_ERR_INVALID, "gradient: more than 2^31 tiles");
             if (host_grad) {
-                const int grid = (int)std::min<long long>(blocks, 2ll * ctx->num_sms);
+                const int grid = (int)std::min<long long>(blocks, std::max(1, ctx->num_sms * 7 / 10));
                 if (pow2)
                     k_gradient_poly_walk_host<true><<<grid, kBS, 0, ctx->stream>>>(d_h, g, d_grad, chunks, units);
                 else
