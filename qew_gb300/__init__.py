@@ -660,9 +660,11 @@ class LangevinDynamics:
 
     def __del__(self):
         try:
-            if self.h:
+            # (the collector may finalise a cycle's context first: its stream,
+            # on which the buffer is freed, is gone with it)
+            if self.h and self.ctx.h:
                 self.ctx.lib.qew_langevin_destroy(self.h)
-                self.h = None
+            self.h = None
         except Exception:
             pass
 
