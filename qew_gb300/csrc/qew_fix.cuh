@@ -149,21 +149,21 @@ __host__ __device__ __forceinline__ unsigned long long fx_bits(double a) {
 // the first two periods about zero, the last two FP64 numbers of a period,
 // where the reference's division by the period may round up. (Declining the
 // whole last cell, and |g| >= 2^30, made 8 lines of 2^20 points there 1530 us on 16
-// taps where FP64 alone took 1166; now 244 and 263.)
-__host__ __device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &iy,
-                                                   unsigned long long &f) {
-    const unsigned long long b = fx_bits(a);
-    const int ef = (int)(b >> 52) & 0x7FF;
-    const int e = ef + k - 1023;
-    if (ef == 0 || ef == 2047 || e > 49) {
-        iy = 0;
-        f = 0ull;
-        return (b << 1) == 0ull;
-    }
+// taps where FP64 alone took 1166; now 251 and 269.)
+//
+// fx_fold: g outside the field's first period (b: the bits of a, e: g's binary
+// exponent), out of line: with its code in every gather the Rosso-Krauth search
+// outgrew the instruction cache (200 sweeps of 2048 sites 6.76 ms, 5.87 so; a
+// line outside the first period pays 3 % for the call).
+struct FxFold {
+    unsigned long long f;
+    int iy, ok;
+};
+static __host__ __device__ __noinline__ FxFold fx_fold(unsigned long long b, int e, int n) {
     const unsigned long long m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
-    const int up = 12 + e;  // fraction bits to the top of 64 (the integer part leaves)
-    f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
-    iy = e >= 0 ? (int)fx_shr(m, 52 - e) : 0;
+    const int up = 12 + e;
+    unsigned long long f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
+    int iy = e >= 0 ? (int)fx_shr(m, 52 - e) : 0;
     bool later = false;  // than the two periods about zero
     if (e > 29) {        // up to 50 bits: whole periods taken out in 64-bit arithmetic
         const unsigned long long whole = fx_shr(m, 52 - e);
@@ -173,10 +173,10 @@ __host__ __device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &
         later = true;
         iy %= n;
     }
-    // the fraction after a fold, two units of a's last bit or more before the end
+    // the fraction lies two units of a's last bit or more before the end
     const auto inside = [&]() { return f < 0ull - fx_shl(2ull, up); };
-    if ((long long)b >= 0) return !later || iy + 1 < n || inside();
-    if (n == 1) return false;
+    if ((long long)b >= 0) return FxFold{f, iy, !later || iy + 1 < n || inside()};
+    if (n == 1) return FxFold{f, 0, 0};
     // bits below 2^-64 leave a mark in the lowest one, for the sums with the
     // period that lie next to halfway between two numbers
     const bool cut = up < 0 && fx_shl(f, -up) != m;
@@ -196,6 +196,30 @@ __host__ __device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &
             f = 0ull;
             iy = (iy + 1 == n) ? 0 : iy + 1;
         }
+    }
+    return FxFold{f, iy, ok};
+}
+
+__host__ __device__ __forceinline__ bool fx_cell64(double a, int k, int n, int &iy,
+                                                   unsigned long long &f) {
+    const unsigned long long b = fx_bits(a);
+    const int ef = (int)(b >> 52) & 0x7FF;
+    const int e = ef + k - 1023;
+    if (ef == 0 || ef == 2047 || e > 49) {
+        iy = 0;
+        f = 0ull;
+        return (b << 1) == 0ull;
+    }
+    const unsigned long long m = (b & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull;
+    const int up = 12 + e;  // fraction bits to the top of 64 (the integer part leaves)
+    f = up >= 0 ? fx_shl(m, up) : fx_shr(m, -up);
+    iy = e >= 0 ? (int)fx_shr(m, 52 - e) : 0;
+    bool ok = true;
+    if ((long long)b < 0 || iy >= n || e > 29) {
+        const FxFold r = fx_fold(b, e, n);
+        iy = r.iy;
+        f = r.f;
+        ok = r.ok;
     }
     return ok;
 }

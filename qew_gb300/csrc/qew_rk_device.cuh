@@ -294,7 +294,7 @@ __device__ __forceinline__ double rk_forward_zero_pair(const Noise &nz, int i, i
 //     nearer to the zero than v's rounding errors over s is evaluated.
 // Anything else (a steep field, a bracket out of the two cells) takes the generic
 // search. 200 sweeps of
-// a 2048-point line (16 taps): 39.0 -> 6.1 ms.
+// a 2048-point line (16 taps): 39.0 -> 5.9 ms.
 struct RkEdge {     // one edge's cubics in row cells iy and iy + 1
     long long p[2], u2[2], w[2];
     int d[2];  // the cells' units' orders below the field's (FxCubic)
