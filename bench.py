@@ -839,9 +839,9 @@ def fp64_peak(Q, ctx):
 # smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}_pred_on.sum of one
 # launch divided by its points. For k_gradient these counters leave out its
 # FP64 floor, conversions and compares, so its fraction reads low.
-# k_gradient_poly: the linear model's walk, 2 DFMA; k_gradient: 3 DADD, 3 DFMA
+# k_gradient_poly_walk (the linear model): 2 DFMA; k_gradient: 3 DADD, 3 DFMA
 # and 1 DMUL (the gathers run in 64-bit integers).
-FP64_INST_PER_POINT = {"k_gradient_poly": 2.0, "k_gradient": 7.01}
+FP64_INST_PER_POINT = {"k_gradient_poly_walk": 2.0, "k_gradient": 7.01}
 
 
 def run_sections_only(args, Q, torch, rank):
@@ -913,13 +913,12 @@ def run_ours(args):
     # The three forms of the gather on the same lines, each one step = the
     # gradients of all n_inst lines:
     #   fp64            FP64 drop-in: the cell-polynomial store, one batched
-    #                   launch (k_gradient_poly: its walk for the linear model)
+    #                   launch (k_gradient_poly_walk for the linear model)
     #   fp64_reference  FP64 with the reference's arithmetic bit for bit (its
     #                   16-tap order, true divisions, no fused multiply-adds),
     #                   one launch (k_gradient)
     #   fp32split       FP32 split-index gather on the x-filtered FP32 store,
-    #                   one batched launch (k_gradient_split_walk,
-    #                   reported as k_gradient_split_persist)
+    #                   one batched launch (k_gradient_split_walk)
     def step_fp64():
         Q.gradient_batch(H, p, noise, G)
 
@@ -929,13 +928,13 @@ def run_ours(args):
     def step_split():
         Q.gradient_split_batch(cells, fracs, p, noise, g32)
 
-    poly_kernel = "k_gradient" if args.no_poly_store else "k_gradient_poly"
+    poly_kernel = "k_gradient" if args.no_poly_store else "k_gradient_poly_walk"
     forms = {
         "fp64": (step_fp64, 48.0, poly_kernel, "f64"),
         "fp64_reference": (step_fp64_ref, 48.0, "k_gradient (reference-exact arithmetic)",
                            "f64"),
         "fp32split": (step_split, 28.0,
-                      "k_gradient_split" if args.no_edge_store else "k_gradient_split_persist",
+                      "k_gradient_split" if args.no_edge_store else "k_gradient_split_walk",
                       "f32"),
     }
     # The energy of the same lines, objective() once per line (each call
@@ -999,15 +998,15 @@ def run_ours(args):
     # DRAM bytes (read + write) per line point of each kernel from one ncu
     # capture of the bench's batched launch (8 lines of 2^20 points) on the
     # small field (each point touches the same number of rows whatever the
-    # field height), scaled to the points of one launch. k_gradient_poly,
-    # k_gradient and k_gradient_split_persist: a warm launch inside the timed
+    # field height), scaled to the points of one launch. k_gradient_poly_walk,
+    # k_gradient and k_gradient_split_walk: a warm launch inside the timed
     # loop (--cache-control none); k_gradient_split: cold (ncu's cache flush,
     # which leaves out the previous launch's write-back).
     dram_per_point = {
-        "k_gradient_poly": (359.998976e6 + 61.611776e6) / (8 * L_FULL),
-        "k_gradient_split_persist": (222.557440e6 + 24.007936e6) / (8 * L_FULL),
+        "k_gradient_poly_walk": (359.828480e6 + 62.031872e6) / (8 * L_FULL),
+        "k_gradient_split_walk": (222.557440e6 + 24.007936e6) / (8 * L_FULL),
         "k_gradient_split": (241.858816e6 + 20.879104e6) / (8 * L_FULL),
-        "k_gradient": (340.568320e6 + 55.892736e6) / (8 * L_FULL),
+        "k_gradient": (354.030336e6 + 56.268544e6) / (8 * L_FULL),
     }
     results = {}
     for name, (fn, bpp, kern, dt) in list(forms.items()) + list(forms_extra.items()):

@@ -89,6 +89,10 @@ enum { QEW_STORE_FP64 = 1, QEW_STORE_FP32 = 2, QEW_STORE_FP32_EDGE = 4,
  * when the field is built (4x the FP64 coefficient memory, 32 bytes per
  * cell). The FP64 gradient on such a line then reads one 32-byte cell per
  * edge and evaluates two integer products instead of the 16-tap tensor sum.
+ * Each cell has a unit of its own, so a weak region beside coefficients many
+ * orders larger keeps the accuracy of FP64 sums there. A field whose largest
+ * |coefficient| is no finite number between 2^-702 and 2^770 holds no store and
+ * takes FP64 sums.
  * Results stay within 1e-15 of the gradient scale of the reference's order;
  * they are not bitwise equal to it (QEW_PREC_FP64_REFERENCE keeps that
  * order). */

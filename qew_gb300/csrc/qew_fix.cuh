@@ -11,8 +11,8 @@
 // dV/dy was wrong by 5e-11 of its own scale. The stencil's unit costs some 40
 // integer instructions an edge.) Measured, with
 // the shorter combine of qew_model_kernels.cuh: the gradient of a
-// 262144-point arclength line 43.5 -> 14.0 us, of a 100003-point line off the
-// field's grid 28.0 -> 11.2 us, a step of the FP64 Langevin run 22.9 -> 16.1 us.
+// 262144-point arclength line 45.1 -> 12.3 us, of three 100003-point lines off the
+// field's grid 92.2 -> 20.5 us (in one launch), 8 lines of 2^20 points 1002 -> 218 us.
 //
 // Formats. A tap is an int64 X with c = X 2^(K-57), |c| < 2^K for its row of the
 // stencil; the four rows' sums are then shifted to the stencil's largest K,

@@ -168,7 +168,7 @@ k_langevin_run(Noise nz, double *h, double *tmp, int n, LineDx L, double lt, dou
 // idles; from the last thread down, so that on a short region the increments
 // and the edges fall to different warps: 4096 sites 4.5 -> 3.7 us a step in
 // FP64, 2.7 -> 2.4 in FP32, with the wrap edge's general weights gone from the
-// chain 2.3 and 1.6; 65536 sites 6.3 -> 4.9 and 4.2 -> 3.05).
+// chain 2.4 and 1.7; 65536 sites 6.3 -> 5.0 and 4.2 -> 3.1).
 //
 // Shared memory, in doubles of the region R = seg + 2K: heights (two
 // buffers), edge values, arclength slopes, increments.
@@ -476,8 +476,8 @@ qew_status qew_langevin_run(qew_langevin *l, const qew_field *field, double *d_h
         const int cls = qew_tune_class(n, (kN32 ? 1 : 0) + (model == QEW_MODEL_ARCLENGTH ? 2 : 0) +
                                               (reads_poly_store(nz) ? 4 : 0));
         // Default from measurement at L = 65536 (us a step): K = 16 steps per
-        // barrier at 2 CTAs per SM, FP64 4.9 against 10.9 with one barrier per
-        // step, FP32 3.05 against 7.9. A tuned shape must be 5 % faster than the
+        // barrier at 2 CTAs per SM, FP64 5.0 against 10.8 with one barrier per
+        // step, FP32 3.1 against 7.7. A tuned shape must be 5 % faster than the
         // default on the probe.
         const int dflt = 5;
         int cand = dflt;

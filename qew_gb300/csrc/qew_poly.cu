@@ -60,7 +60,7 @@ __device__ __forceinline__ void cp_async8(void *smem, const void *gmem) {
 // CTA walks tiles of kTile sites gridDim.x apart and copies the next tile's
 // heights into its spare shared buffer with cp.async while the current
 // tile's gathers are in flight. Bound about equally by 10 FP64 instructions a
-// point and by issue: 8 lines of 2^20 points 262 -> 178 us.
+// point and by issue: 8 lines of 2^20 points 269 -> 181 us.
 template <int kItems>
 __global__ void __launch_bounds__(kBS, kMinCtas)
 k_gradient_poly(const double *__restrict__ h, const __grid_constant__ PolyGeom g,
@@ -497,7 +497,7 @@ qew_status qew_gradient_poly_enqueue(qew_ctx *ctx, const qew_field *f, int count
     // arithmetic does not depend on the launch): sites per thread {1, 2, 4} x
     // resident CTAs per SM {2, 3, 4}, default 2 sites, 4 CTAs; for the walk
     // (a chunk per warp) registers for {4, 5, 6} resident CTAs per SM, default
-    // 5: 86.3, 84.8 and 87.5 us on 8 lines of 2^20 points.
+    // 5: 92.6, 86.6 and 88.2 us on 8 lines of 2^20 points of a 1024-row field.
     static const char *const tile_names[9] = {"1 site x 2 CTA/SM", "1 site x 3 CTA/SM",
                                               "1 site x 4 CTA/SM", "2 sites x 2 CTA/SM",
                                               "2 sites x 3 CTA/SM", "2 sites x 4 CTA/SM",

@@ -7,12 +7,14 @@
 // j the interpolant is a cubic in the fraction t (filtered_noise.h:33-62) of
 // the x-filtered coefficients E_b of rows j-1 .. j+2. The store keeps, per
 // (row cell j, column e), that cubic as four 64-bit fixed-point numbers
-// (FxCubic, qew_fix.cuh), taken once when the field is built from the same
-// integers that the 16-tap gather forms at each call: a field with the store
-// and one without give the same gradient bit for bit on such a line where
-// its spacing makes the column midpoints exact. A gradient edge then reads
-// one aligned 32-byte cell and evaluates two integer products, where the
-// reference's order (filtered_noise.h:159-176) reads 16 taps.
+// (FxCubic, qew_fix.cuh) in a unit of the cell's own, taken once when the field
+// is built from the same integers that the 16-tap gather forms at each call:
+// where dx and dy are powers of two, an edge's dV/dy and V are the same bits with
+// the store and without. (The linear gradient's walk adds heights and both edges
+// in integers before it rounds, and a dy that is no power of two locates a row
+// on the store by one product, so gradients agree to rounding.) A gradient edge
+// then reads one aligned 32-byte cell and evaluates two integer products, where
+// the reference's order (filtered_noise.h:159-176) reads 16 taps.
 #pragma once
 
 #include "qew_internal.cuh"

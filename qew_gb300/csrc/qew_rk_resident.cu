@@ -7,8 +7,8 @@
 // or bisection levels per round in rk_forward_zero_group) with the serial
 // search's result exactly, so both forms produce bit-identical lines.
 //
-// The grid barrier spins on a generation word with a bounded number of polls;
-// if it gives up it raises an error flag, every CTA leaves the sweep loop, and
+// The grid barrier polls its count of arrivals (qew_gridsync.cuh) a bounded
+// number of times; if it gives up it raises an error flag, every CTA leaves the sweep loop, and
 // the host returns QEW_ERR_TIMEOUT. A cooperative launch guarantees that all
 // CTAs are resident, so the barrier completes unless the device is stalled.
 #include <cooperative_groups.h>
@@ -141,8 +141,8 @@ qew_status qew_rk_block_resident(qew_ctx *ctx, const qew_field *field, double *d
         // warps-per-SM budget (and the resident slots, or the context's share
         // of them); the serial form takes what is left.
         // Measured for 200 sweeps (bitwise-equal results): n = 2048 8-lane
-        // groups 5.8 ms, lane pairs 6.7, one lane 64; n = 4096 5.8 and 6.7;
-        // n = 16384 13.5 and 8.1: 8-lane groups while they stay within about
+        // groups 5.9 ms, lane pairs 6.6, one lane 38; n = 4096 6.0 and 6.8;
+        // n = 16384 13.3 and 7.3: 8-lane groups while they stay within about
         // 4 warps per SM, lane pairs up to 8, the serial search beyond.
         const void *forms[3] = {(const void *)k_rk_resident<N, 8>, (const void *)k_rk_resident<N, 2>,
                                 (const void *)k_rk_resident<N, 1>};

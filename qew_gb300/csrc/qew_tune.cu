@@ -16,7 +16,8 @@ struct Entry {
 std::mutex g_mu;
 std::map<std::tuple<int, int, int>, Entry> g_cache;
 
-const char *kKernelNames[kTuneKernels] = {"k_gradient_poly", "k_gradient_split_persist",
+const char *kKernelNames[kTuneKernels] = {"k_gradient_poly",
+                                          "k_gradient_split_walk (k_gradient_split_persist)",
                                           "k_rk_resident", "k_langevin_run"};
 
 }  // namespace

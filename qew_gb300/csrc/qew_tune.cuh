@@ -17,8 +17,8 @@
 #include "qew_internal.cuh"
 
 enum {
-    kTuneGradientPoly = 0,   // k_gradient_poly: sites per thread x resident CTAs per SM
-    kTuneGradientSplit = 1,  // reported as k_gradient_split_persist: steps a chunk x resident CTAs per SM
+    kTuneGradientPoly = 0,   // k_gradient_poly: sites per thread x resident CTAs per SM; its walk: CTAs per SM
+    kTuneGradientSplit = 1,  // k_gradient_split_walk: steps a chunk x resident CTAs per SM
     kTuneRkSearch = 2,       // k_rk_resident: lanes per site's forward-zero search
     kTuneLangevinRun = 3,    // k_langevin_run / k_langevin_run_tb: steps per grid barrier x CTAs per SM
     kTuneKernels = 4
