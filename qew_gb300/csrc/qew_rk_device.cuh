@@ -548,7 +548,10 @@ __device__ __forceinline__ bool rk_forward_zero_fast(const NoiseBSpline64 &nz, i
     if (votes(!(cl >= 0 && cr >= 0 && ((lane & 1) ? vs <= 0 : vs > 0)))) return false;
     const double v0 = __shfl_sync(gmask, vs, 0, G), v1 = __shfl_sync(gmask, vs, 1, G);
     const double x0 = __shfl_sync(gmask, side, 0, G);
-    const double z = fma((double)((float)v0 / (float)(v0 - v1)), 2.0 * gap, x0);
+    // what follows is in floats, far from their range's ends
+    const float fall = (float)(v0 - v1);
+    if (!(fall >= 1e-28f && fall <= 1e28f && width >= 1e-30f)) return false;
+    const double z = fma((double)((float)v0 / fall), 2.0 * gap, x0);
     // v's rounding errors, at most, each within 2^-53 of its number (1.7e-16: and
     // a half more): the sums of heights in the elastic part; each edge's
     // midpoint (the sum, its quotient by the spacing, the fold of a negative one

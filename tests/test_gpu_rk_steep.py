@@ -12,10 +12,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def forms_agree(Q, f, h0, p, dstep, tol, sweeps):
+def forms_agree(Q, f, h0, p, dstep, tol, sweeps, scale=1.0):
     import torch
-    rp = Q.RkParams(dstep=dstep, max_advance=1000.0 * dstep, root_tol=tol, sweep_tol=1e-30,
-                    runaway=1e9, max_sweeps=sweeps)
+    rp = Q.RkParams(dstep=dstep, max_advance=1000.0 * dstep, root_tol=tol, sweep_tol=1e-30 * scale,
+                    runaway=1e9 * scale, max_sweeps=sweeps)
     want = h0.clone()
     rw = Q.rk_block(want, p, f, rp, form=Q.QEW_RK_PLAIN)
     assert bool((want != h0).any())
@@ -29,6 +29,7 @@ def forms_agree(Q, f, h0, p, dstep, tol, sweeps):
             assert (rg.blocked, rg.runaway, rg.sweeps) == (rw.blocked, rw.runaway, rw.sweeps)
     finally:
         f.ctx.force_tune_candidate(Q.QEW_TUNE_RK_SEARCH, -1)
+    return want
 
 
 @pytest.mark.parametrize("spacing,base", [(1.0, 600.25), (1.0, 3.0e7), (0.375, 3.0e7), (0.37, 2.0e7),
@@ -64,3 +65,22 @@ def test_steep_random_fields_bitwise(Q, tension, xi, amplitude, spacing, base, s
     p = Q.Params(float(n), tension, 0.2 * amplitude, Q.Model.Linear)
     for tol, sweeps in ((1e-10 * spacing, 40), (0.0, 12)):
         forms_agree(Q, f, h0, p, 0.5 * spacing, tol, sweeps)
+
+
+@pytest.mark.parametrize("height,force", [(2.0 ** -90, 2.0 ** -34), (2.0 ** -60, 2.0 ** -66), (2.0 ** 60, 2.0 ** 50)])
+def test_scaled_units_bitwise(Q, height, force):
+    """Heights and forces in units whose velocities leave the range of single
+    precision, in which the search compares slopes: a power of two scales the
+    plain form's line exactly, and every form follows it."""
+    import torch
+    n, ny = 1024, 256
+    v = np.random.default_rng(4).standard_normal((n, ny))
+    rng = np.random.default_rng(5)
+    h = torch.as_tensor(100.0 + rng.uniform(0, 5.0, n), device="cuda")
+    lines = []
+    for a, b in ((1.0, 1.0), (height, force)):
+        f = Q.FilteredNoise(v * (a * a * b), float(n), a * ny)
+        p = Q.Params(float(n), 2.0 * b, 0.2 * a * b, Q.Model.Linear)
+        h0 = h * a
+        lines.append(forms_agree(Q, f, h0, p, 0.5 * a, 1e-10 * a, 20, a) / a)
+    assert torch.equal(*lines)
